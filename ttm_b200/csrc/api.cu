@@ -253,6 +253,8 @@ int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t s
         // TMA-fed row mode measured 0.87-0.88 of HBM against 0.65-0.72 at m = 8).
         const int64_t a_bytes = v.outer * v.nq * v.inner * (x.dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= stream_min_bytes && stream_supported(v, x.dtype);
+        if (x.dtype == TLIBTTM_F64 && small_m_takes_gemm_f64(v, tma))
+            return note_launch(launch_simt_gemm(v, x.dtype, s, nullptr, false, false), K_SIMT_GEMM);
         // Few rows (outer * inner <= 8) and a long l range the TMA kernel does not take: the
         // column and row kernels would run a block or two; the l range goes over the GPU instead.
         if (!tma && bvec_small_supported(v)) {
@@ -630,6 +632,7 @@ int launches_of(const Single& sg, int dtype, int precision)
         const View3& v = sg.pl.v;
         const int64_t a_bytes = v.outer * v.nq * v.inner * (dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= kPlanStreamMinBytes && stream_supported(v, dtype);
+        if (dtype == TLIBTTM_F64 && small_m_takes_gemm_f64(v, tma)) return 1;
         return (!tma && bvec_small_supported(v)) ? 2 : 1;
     }
     int pr = precision == TLIBTTM_PREC_DEFAULT ? g_precision.load() : precision;
@@ -970,7 +973,6 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
     P->precision = precision;
     P->dev = dev;
     const size_t es = dtype == TLIBTTM_F32 ? sizeof(float) : sizeof(double);
-    const int64_t tile = dtype == TLIBTTM_F32 ? kGemmTileF32 : kGemmTileF64;
     struct Item { GroupDesc d; double cost; };
     std::vector<Item> items;
     std::vector<View3> tcviews;   // problems of the grouped bf16x3 launch
@@ -1051,15 +1053,15 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
                             d.tiles_n = 1;
                         } else {
                             d.kind = 0;
-                            d.tiles_m = ceil_div(M, tile);
-                            d.tiles_n = ceil_div(v.m, tile);
+                            d.tiles_m = ceil_div(M, kGemmRows);
+                            grouped_columns(v.m, dtype, &d.tiles_n, &d.cols);
                             const bool ak = v.inner == 1;
                             bool vec = (reinterpret_cast<uintptr_t>(v.a) % 16 == 0) && (reinterpret_cast<uintptr_t>(v.c) % 16 == 0);
                             vec = vec && (ak ? (v.nq % rv == 0 && v.m % rv == 0) : (v.inner % rv == 0));
                             d.flags = (ak ? 1 : 0) | (vec ? 2 : 0);
                         }
                         // cost ~ work-item count x work per item, for a largest-first order
-                        const double per_item = d.kind == 0 ? (double)v.nq * tile * tile
+                        const double per_item = d.kind == 0 ? (double)v.nq * kGemmRows * d.cols
                                                             : (double)v.nq * (d.flags & 1 ? kGemvRows : 8 * 32 * (d.flags & 2 ? rv : 1)) * 16;
                         items.push_back(Item{d, (double)(d.tiles_m * d.tiles_n) * per_item});
                     }

@@ -70,7 +70,7 @@ struct GroupDesc {
     int b_cm;
     int kind;          // 0: slice-GEMM tiles, 1: rows of the small-m kernel
     int flags;         // bit 0: fibres contiguous (inner == 1); bit 1: 16-byte vector access
-    int pad;
+    int cols;          // slice-GEMM: columns of a tile
     int64_t tiles_m;   // slice-GEMM: row tiles; small-m: blocks of 256 rows (256 * 16/sizeof(T) when
                        // strided fibres are read with 16-byte loads)
     int64_t tiles_n;   // slice-GEMM: column tiles; small-m: 1
@@ -102,9 +102,13 @@ const char* kernel_name(int id);
 // Launchers (simt_kernels.cu). Return cudaSuccess or the launch error.
 // The slice-GEMM; when its tiles cannot fill the GPU and n_q is long, the K loop is split over
 // more blocks and the parts are added by a second kernel (*launches = 2, else 1).
-// force_split: split the K loop whenever n_q >= 2048 (a schedule of its own for the tuner).
+// force_split: split the K loop whenever n_q >= 2048 (a schedule of its own for the tuner);
+// may_split false: never (one launch).
 cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr,
-                             bool force_split = false);
+                             bool force_split = false, bool may_split = true);
+// Double, m <= kSmallM: whether the matrix-instruction slice-GEMM is the faster choice against the
+// small-m kernels (`tma`: the TMA-fed one would take the problem).
+bool small_m_takes_gemm_f64(const View3& v, bool tma);
 int simt_gemm_launch_count(const View3& v, int dtype);
 // Few output rows (outer * inner <= 8), 16 < m <= 256, n_q >= 4096: a kernel that streams B with
 // the l range split over the GPU, then a fixed-order reduction (*launches = 2).
@@ -128,8 +132,10 @@ cudaError_t launch_grouped(const GroupDesc* d_desc, int count, int64_t total, un
 cudaError_t launch_grouped_small(const GroupDesc* d_desc, int count, int64_t total, unsigned long long* queue,
                                  int dtype, int grid, cudaStream_t s);
 int grouped_small_blocks_per_sm(int dtype);
-// Row / column tile sizes of the slice-GEMM for an element type, and rows per small-m work item.
-constexpr int kGemmTileF32 = 128, kGemmTileF64 = 64, kGemvRows = 256;
+// Rows of a slice-GEMM tile and of a small-m work item, and the column tiles of the grouped
+// slice-GEMM for m columns (their number and width).
+constexpr int kGemmRows = 128, kGemvRows = 256;
+void grouped_columns(int64_t m, int dtype, int64_t* tiles, int* cols);
 // Blocks per SM the grouped kernel is launched with.
 int grouped_blocks_per_sm(int dtype);
 

@@ -1,0 +1,299 @@
+// FP64 slice-GEMM on the double-precision matrix instruction (mma.sync m8n8k4.f64).
+//
+// One tile is BM (128 or 64) rows (flattened (k, i) pairs) x up to 8 * NF columns j; 2 BM threads.
+// Warp w owns rows [16 w, 16 w + 16) and every column of the tile: the widths are whole builds in
+// groups of eight columns, so that no warp multiplies padding (m = 100: two tiles of 56 columns).
+// A and B tiles of 16 l go through a ring of ST shared-memory stages filled with cp.async.
+//
+// What bounds it: the FP64 pipe (37.1 TFLOP/s for a stream of mma on this part, 33.9 for plain
+// DFMA) once m passes about 24; below that, reading A. A k-step of four l costs a warp 1 or 2 A and
+// NF B shared loads for 2 NF mma of 256 multiply-adds each; the DFMA tile of 64 x 64 it replaced
+// needed 8 loads for 16 DFMA of 32. Measured, before -> now: A 256^3, m = 128, middle mode
+// 323 -> 150 us (29 TFLOP/s); (150, 171, 333), m = 100 189 -> 91 us; (200, 180, 160), m = 20
+// 84 -> 21 us; contiguous fibres of 384, 78000 rows, m = 16 (TMA row kernel) 139 -> 54 us.
+// Rows of 64 for at most 16 columns (five blocks of 128 threads per SM, 16-byte copies): 59 us at
+// 128 rows against 53; with 8-byte copies 128 rows are faster (73 against 119 us).
+#pragma once
+
+#include "common.cuh"
+
+namespace tlibttm {
+namespace f64 {
+
+constexpr int BK = 16;
+
+// Row pitches are 4 mod 16 doubles: the 4 l x 4 rows (or columns) that half a warp reads lie in
+// distinct banks.
+template <int BM, int NF, int ST, bool AK, bool BCM>
+struct Smem {
+    static constexpr int BN = NF * 8;
+    static constexpr int AP = AK ? BK + 4 : BM + 4, AR = AK ? BM : BK;
+    static constexpr int BP = BCM ? BN + 4 : BK + 4, BR = BCM ? BK : BN;
+    __align__(16) double a[ST][AR][AP];   // [row][l] for contiguous fibres, else [l][row]
+    __align__(16) double b[ST][BR][BP];   // [l][j] for column-major B, else [j][l]
+};
+
+__device__ __forceinline__ void mma(double (&c)[2], double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Copies 16 or 8 bytes; zeroes the destination where !ok (src is then not read).
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool ok)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy8(void* dst, const void* src, bool ok)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(ok ? 8 : 0)
+                 : "memory");
+}
+
+// row / inner, in 32 bits where both fit
+__device__ __forceinline__ int64_t slice_of(int64_t row, int64_t inner)
+{
+    if ((((uint64_t)row | (uint64_t)inner) >> 32) == 0) return (int64_t)((uint32_t)row / (uint32_t)inner);
+    return row / inner;
+}
+
+// One stage (16 l) of a warp's 16 rows x 8 N columns. At most eight columns: two accumulation
+// chains (even and odd l / 4), added by the caller at the end.
+template <int N, bool AK, bool BCM, int AR, int AP, int BR, int BP, int NA>
+__device__ __forceinline__ void stage(const double (&sa)[AR][AP], const double (&sb)[BR][BP], int warp, int g, int c,
+                                      double (&acc)[2][NA][2])
+{
+    if constexpr (N <= NA) {
+#pragma unroll
+        for (int kk = 0; kk < BK; kk += 4) {
+            // rows of mma r, group g: 2 g + r (strided fibres: one 16-byte load), 8 r + g otherwise
+            double a0, a1;
+            if (AK) {
+                a0 = sa[warp * 16 + g][kk + c];
+                a1 = sa[warp * 16 + 8 + g][kk + c];
+            } else {
+                const double2 t = *reinterpret_cast<const double2*>(&sa[kk + c][warp * 16 + 2 * g]);
+                a0 = t.x;
+                a1 = t.y;
+            }
+#pragma unroll
+            for (int f = 0; f < N; ++f) {
+                const double b = BCM ? sb[kk + c][8 * f + g] : sb[8 * f + g][kk + c];
+                const int to = N == 1 ? (kk >> 2) & 1 : f;
+                mma(acc[0][to], a0, b);
+                mma(acc[1][to], a1, b);
+            }
+        }
+    }
+}
+
+// The column tiles of a problem: `cols` of them per row tile, nf groups of eight columns each.
+// Tile t covers rows [BM (t / cols), ...) and columns [8 nf (t % cols), ...).
+struct Grid {
+    int64_t cols;
+    int nf;
+};
+
+// Tiles first, first + step, ... below `last`, l in [l_begin, l_end) of each; the stages of
+// consecutive tiles follow one another through the ring, so that the next tile's loads are in
+// flight while this one's results are stored. VEC: 16-byte copies of A (alignment checked by the
+// host). The caller synchronises the block between two calls that share `sm`.
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, bool EXACT>
+__device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t step, int64_t last, const Grid& gr,
+                                      Smem<BM, NF, ST, AK, BCM>& sm, int64_t l_begin, int64_t l_end)
+{
+    constexpr int BN = NF * 8, NT = 2 * BM, NA = NF == 1 ? 2 : NF;
+    const double* __restrict__ A = static_cast<const double*>(v.a);
+    const double* __restrict__ B = static_cast<const double*>(v.b);
+    double* __restrict__ C = static_cast<double*>(v.c);
+    const int64_t inner = v.inner, m = v.m, nq = v.nq;
+    const int64_t M = v.outer * inner;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
+
+    // A copies: WA elements each, LA of them per thread and stage. Strided fibres: all of a
+    // thread's copies are of the same rows, l apart; contiguous fibres: same l, rows apart.
+    constexpr int WA = VEC ? 2 : 1, LA = BM * BK / WA / NT;
+    constexpr int AX = (AK ? BK : BM) / WA;          // copies along the contiguous extent
+    constexpr int AY = NT / AX;                      // rows of copies per pass
+    const int ax = (tid % AX) * WA, ay = tid / AX;
+    // B copies: 8 bytes each (any alignment of m and n_q), of the columns below 8 nf only
+    constexpr int BX = !BCM ? BK : NF == 1 ? 8 : NF == 2 ? 16 : NF <= 4 ? 32 : 64, BY = NT / BX;
+    constexpr int LB = ((BCM ? BK : BN) + BY - 1) / BY;
+    const int bx = tid % BX, by = tid / BX;
+
+    // the tile being loaded, and where in its l range
+    int64_t lt = first, ll = l_begin, ln0 = 0;
+    int a_rows = 0;          // contiguous fibres: rows of the tile in A; else 1 if this thread's row is
+    const double* ap = A;
+    auto start = [&]() {
+        const int64_t rt = gr.cols == 1 ? lt : slice_of(lt, gr.cols);
+        const int64_t m0 = rt * BM;
+        ln0 = (lt - rt * gr.cols) * gr.nf * 8;
+        if (AK) {
+            a_rows = (int)(M - m0 < BM ? M - m0 : BM);
+            ap = A + (m0 + ay) * nq + ax;
+        } else {
+            const int64_t row = m0 + ax;
+            a_rows = row < M;
+            const int64_t k = a_rows ? slice_of(row, inner) : 0;
+            ap = A + (a_rows ? k * inner * nq + (row - k * inner) : 0) + (int64_t)ay * inner;
+        }
+    };
+    auto issue = [&](int st) {
+#pragma unroll
+        for (int s = 0; s < LA; ++s) {
+            if (AK) {
+                const bool ok = ay + s * AY < a_rows && ll + ax < l_end;
+                const double* src = ok ? ap + (int64_t)s * AY * nq + ll : A;
+                if (VEC) copy16(&sm.a[st][ay + s * AY][ax], src, ok);
+                else copy8(&sm.a[st][ay + s * AY][ax], src, ok);
+            } else {
+                const bool ok = a_rows && ll + ay + s * AY < l_end;
+                const double* src = ok ? ap + (ll + s * AY) * inner : A;
+                if (VEC) copy16(&sm.a[st][ay + s * AY][ax], src, ok);
+                else copy8(&sm.a[st][ay + s * AY][ax], src, ok);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < LB; ++s) {
+            const int jo = BCM ? bx : by + s * BY, lo = BCM ? by + s * BY : bx;
+            if (jo >= (EXACT ? BN : gr.nf * 8) || lo >= BK) continue;
+            const int64_t j = ln0 + jo, l = ll + lo;
+            const bool ok = j < m && l < l_end;
+            const double* src = ok ? (BCM ? B + j + l * m : B + j * nq + l) : B;
+            copy8(BCM ? &sm.b[st][lo][jo] : &sm.b[st][jo][lo], src, ok);
+        }
+    };
+    // loads one stage (none past the last tile) and moves on; one commit group per call, empty
+    // ones too, so that wait_group counts stages
+    auto load_next = [&](int st) {
+        if (lt < last) {
+            issue(st);
+            ll += BK;
+            if (ll >= l_end) {
+                ll = l_begin;
+                lt += step;
+                if (lt < last) start();
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (lt < last) start();
+#pragma unroll
+    for (int st = 0; st < ST - 1; ++st) load_next(st);
+    int rd = 0, wr = ST - 1;
+    const int nk = (int)ceil_div(l_end - l_begin, BK);
+
+    for (int64_t t = first; t < last; t += step) {
+    const int64_t t_row = gr.cols == 1 ? t : slice_of(t, gr.cols);
+    const int64_t m0 = t_row * BM, n0 = (t - t_row * gr.cols) * gr.nf * 8;
+    const int nf = EXACT ? NF : (int)(m - n0 < gr.nf * 8 ? (m - n0 + 7) / 8 : gr.nf);
+
+    double acc[2][NA][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int f = 0; f < NA; ++f) acc[r][f][0] = acc[r][f][1] = 0.0;
+
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();   // stage rd has landed for all, and all have read stage wr's last contents
+        load_next(wr);
+        if constexpr (EXACT) {
+            stage<NF, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc);
+        } else {
+            // one build per width: predicated-off mma would take the pipe as long as executed ones
+            switch (nf) {
+            case 1: stage<1, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 2: stage<2, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 3: stage<3, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 4: stage<4, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 5: stage<5, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 6: stage<6, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 7: stage<7, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            default: stage<NF, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            }
+        }
+        rd = rd + 1 == ST ? 0 : rd + 1;
+        wr = wr + 1 == ST ? 0 : wr + 1;
+    }
+
+    if (nf == 1) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) acc[r][0][e] += acc[r][1][e];
+    }
+
+    // C(row, j) = base(row) + j inner; lane (g, c) holds columns 8 f + 2 c and 8 f + 2 c + 1
+    const bool c16 = (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
+    if (AK) {
+        const bool vec = c16 && (m & 1) == 0;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int64_t row = m0 + warp * 16 + 8 * r + g;
+            if (row >= M) continue;
+            double* cp = C + row * m;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                const int64_t j = n0 + 8 * f + 2 * c;
+                if (f >= nf || j >= m) continue;
+                if (vec) {
+                    *reinterpret_cast<double2*>(cp + j) = make_double2(acc[r][f][0], acc[r][f][1]);
+                } else {
+                    cp[j] = acc[r][f][0];
+                    if (j + 1 < m) cp[j + 1] = acc[r][f][1];
+                }
+            }
+        }
+    } else {
+        const int64_t row = m0 + warp * 16 + 2 * g;
+        if (row >= M) continue;
+        const int64_t k0 = slice_of(row, inner), i0 = row - k0 * inner;
+        double* cp = C + k0 * inner * m + i0;
+        if (c16 && (inner & 1) == 0) {
+            // row + 1 lies in the same slice (and M is even)
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int64_t j = n0 + 8 * f + 2 * c + e;
+                    if (f < nf && j < m)
+                        *reinterpret_cast<double2*>(cp + j * inner) = make_double2(acc[0][f][e], acc[1][f][e]);
+                }
+        } else {
+            const bool two = row + 1 < M;
+            // the next row: i + 1 of this slice, or i = 0 of the next
+            double* cq = i0 + 1 < inner ? cp + 1 : C + (k0 + 1) * inner * m;
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int64_t j = n0 + 8 * f + 2 * c + e;
+                    if (f < nf && j < m) {
+                        cp[j * inner] = acc[0][f][e];
+                        if (two) cq[j * inner] = acc[1][f][e];
+                    }
+                }
+        }
+    }
+    }
+}
+
+// Column tiles of a problem of m columns, and the width of each in groups of eight: as even as
+// possible, at most NF groups.
+__host__ __device__ inline Grid split_columns(int64_t m, int nf_max)
+{
+    const int64_t groups = ceil_div(m, 8);
+    Grid g;
+    g.cols = ceil_div(groups, nf_max);
+    g.nf = (int)ceil_div(groups, g.cols);
+    return g;
+}
+
+}  // namespace f64
+}  // namespace tlibttm

@@ -1,10 +1,11 @@
 // SIMT kernels of the B200 TTM library: the exact-arithmetic ("plain") paths.
 //
-//  simt_gemm  slice-GEMM over the dense view C[k][j][i] = sum_l A[k][l][i] B(j,l),
-//             FP32 FFMA or FP64 DFMA, 128x128 (f32) / 64x64 (f64) CTA tiles,
-//             register-double-buffered shared-memory stages. Rows of the GEMM
-//             are the flattened (k, i) pairs, so one kernel covers every
-//             layout case without transposing anything.
+//  simt_gemm  slice-GEMM over the dense view C[k][j][i] = sum_l A[k][l][i] B(j,l):
+//             FP32 FFMA in 128x128 CTA tiles with register-double-buffered
+//             shared-memory stages; FP64 on the double-precision matrix
+//             instruction (gemm_f64.cuh). Rows of the GEMM are the flattened
+//             (k, i) pairs, so one kernel covers every layout case without
+//             transposing anything.
 //  colvec     bandwidth kernel for small m when A's fibres along mode q are
 //             strided (inner >= 2): each thread owns W consecutive i of one k
 //             and streams 16-byte loads along l; B is staged in shared memory.
@@ -18,6 +19,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_f64.cuh"
 
 namespace tlibttm {
 namespace {
@@ -62,6 +64,7 @@ __device__ __forceinline__ double fma_t(double a, double b, double c) { return _
 
 // ---------------------------------------------------------------------------------------------
 // simt_gemm
+//   (float; the FP64 tile is in gemm_f64.cuh)
 //   AK   : A is K-major (inner == 1, fibres contiguous); otherwise rows (i) are contiguous.
 //   VEC  : 16-byte vector loads of A and vector stores of C (alignment and divisibility checked
 //          by the host).
@@ -327,6 +330,22 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 3 : 2)) simt_gemm_split
     View3 part = v;
     part.c = ws + (size_t)blockIdx.z * (size_t)(v.outer * v.m * v.inner);
     gemm_tile<T, AK, VEC, BCM>(part, (int64_t)blockIdx.x * (32 * RV), (int64_t)blockIdx.y * (32 * RV), sm, l0, l1);
+}
+
+// FP64: tiles of 128 x 8 nf (gemm_f64.cuh), column tiles next to one another so that they share
+// A's rows in L2. gridDim.z parts of the l range write partial results to ws, as above.
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
+__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 5) dmma_gemm_kernel(View3 v, f64::Grid gr, int64_t tiles, int64_t lper, double* ws)
+{
+    extern __shared__ __align__(16) unsigned char dmma_smem[];
+    auto& sm = *reinterpret_cast<f64::Smem<BM, NF, ST, AK, BCM>*>(dmma_smem);
+    int64_t l0 = 0, l1 = v.nq;
+    if (gridDim.z > 1) {
+        l0 = (int64_t)blockIdx.z * lper;
+        l1 = l0 + lper < v.nq ? l0 + lper : v.nq;
+        v.c = ws + (size_t)blockIdx.z * (size_t)(v.outer * v.m * v.inner);
+    }
+    f64::tiles<BM, NF, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr, sm, l0, l1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -901,13 +920,6 @@ __global__ void __launch_bounds__(256) strided_kernel(StridedProblem sp)
 // counter; an item is one slice-GEMM tile of a problem (m > 16) or a block of 256 rows of a
 // small-m problem. Problems are ordered largest first by the host, so the tail is short.
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-union GroupedSmem {
-    GemmSmem<T> gemm;
-    ColvecSmem<T, 16> col;
-    RowdotSmem<T, 16> row;
-};
-
 // ASYNC: unaligned column items take colvec_async (its ring must be part of SM).
 template <typename T, int MB, bool ASYNC, class SM>
 __device__ __forceinline__ void grouped_small(const View3& v, int flags, int64_t local, SM& sm)
@@ -925,15 +937,33 @@ __device__ __forceinline__ void grouped_small(const View3& v, int flags, int64_t
     }
 }
 
+constexpr int kGroupNF = 8, kGroupST = 3;   // the FP64 tile of the grouped launch
+template <typename T>
+constexpr size_t grouped_smem_bytes()
+{
+    if (sizeof(T) == 4) return sizeof(GemmSmem<T>);
+    const size_t rows = sizeof(f64::Smem<kGemmRows, kGroupNF, kGroupST, true, false>),
+                 cols = sizeof(f64::Smem<kGemmRows, kGroupNF, kGroupST, false, true>);
+    return std::max(rows, cols);   // the largest of the four forms: one pitch of A with one of B
+}
+
+#define TLIBTTM_TILES                                                                                \
+    if (ak) {                                                                                        \
+        if (vec) { if (g.b_cm) TLIBTTM_TILE(true, true, true); else TLIBTTM_TILE(true, true, false); } \
+        else     { if (g.b_cm) TLIBTTM_TILE(true, false, true); else TLIBTTM_TILE(true, false, false); } \
+    } else {                                                                                         \
+        if (vec) { if (g.b_cm) TLIBTTM_TILE(false, true, true); else TLIBTTM_TILE(false, true, false); } \
+        else     { if (g.b_cm) TLIBTTM_TILE(false, false, true); else TLIBTTM_TILE(false, false, false); } \
+    }
+
 // Two CTAs per SM (at most 128 registers; a few spill): measured faster on the batched workload
 // than one CTA of 255 registers.
 template <typename T>
 __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __restrict__ desc, int count, int64_t total,
                                                       unsigned long long* queue)
 {
-    constexpr int RV = 16 / sizeof(T);
-    constexpr int BM = 32 * RV, BN = 32 * RV;
-    __shared__ GroupedSmem<T> sm;
+    constexpr int BM = 128, BN = 128;
+    extern __shared__ __align__(16) unsigned char grouped_smem[];
     __shared__ int64_t item_s;
     for (;;) {
         if (threadIdx.x == 0) item_s = (int64_t)atomicAdd(queue, 1ull);
@@ -957,22 +987,21 @@ __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __rest
         v.inner = g.inner;
         v.m = g.m;
         v.b_cm = g.b_cm;
-        if (g.kind == 0) {
-            const int64_t m0 = (local % g.tiles_m) * BM, n0 = (local / g.tiles_m) * BN;
-            const bool ak = g.flags & 1, vec = g.flags & 2;
-            if (ak) {
-                if (vec) { if (g.b_cm) gemm_tile<T, true, true, true>(v, m0, n0, sm.gemm); else gemm_tile<T, true, true, false>(v, m0, n0, sm.gemm); }
-                else     { if (g.b_cm) gemm_tile<T, true, false, true>(v, m0, n0, sm.gemm); else gemm_tile<T, true, false, false>(v, m0, n0, sm.gemm); }
-            } else {
-                if (vec) { if (g.b_cm) gemm_tile<T, false, true, true>(v, m0, n0, sm.gemm); else gemm_tile<T, false, true, false>(v, m0, n0, sm.gemm); }
-                else     { if (g.b_cm) gemm_tile<T, false, false, true>(v, m0, n0, sm.gemm); else gemm_tile<T, false, false, false>(v, m0, n0, sm.gemm); }
-            }
+        const bool ak = g.flags & 1, vec = g.flags & 2;
+        if constexpr (sizeof(T) == 8) {
+            const f64::Grid gr{g.tiles_n, g.cols / 8};
+#define TLIBTTM_TILE(AKv, VECv, BCMv)                                                                        \
+    f64::tiles<kGemmRows, kGroupNF, kGroupST, AKv, VECv, BCMv, false>(v, local, 1, local + 1, gr,                    \
+                                                   *reinterpret_cast<f64::Smem<kGemmRows, kGroupNF, kGroupST, AKv, BCMv>*>(grouped_smem), \
+                                                   0, v.nq)
+            TLIBTTM_TILES
+#undef TLIBTTM_TILE
         } else {
-            if (g.m <= 1) grouped_small<T, 1, false>(v, g.flags, local, sm);
-            else if (g.m <= 2) grouped_small<T, 2, false>(v, g.flags, local, sm);
-            else if (g.m <= 4) grouped_small<T, 4, false>(v, g.flags, local, sm);
-            else if (g.m <= 8) grouped_small<T, 8, false>(v, g.flags, local, sm);
-            else grouped_small<T, 16, false>(v, g.flags, local, sm);
+            auto& gm = *reinterpret_cast<GemmSmem<T>*>(grouped_smem);
+            const int64_t m0 = (local / g.tiles_n) * BM, n0 = (local % g.tiles_n) * BN;
+#define TLIBTTM_TILE(AKv, VECv, BCMv) gemm_tile<T, AKv, VECv, BCMv>(v, m0, n0, gm)
+            TLIBTTM_TILES
+#undef TLIBTTM_TILE
         }
         __syncthreads();
     }
@@ -1025,11 +1054,25 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) grouped_small_ker
     }
 }
 
+int g_sms_simt = 0;
+
+cudaError_t sms_of_device(int& sms)
+{
+    if (!g_sms_simt) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms_simt, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+    }
+    sms = g_sms_simt;
+    return cudaSuccess;
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-template <typename T>
-cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, int64_t lper = 0, T* ws = nullptr)
+cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, int64_t lper = 0, float* ws = nullptr)
 {
+    using T = float;
     constexpr int RV = 16 / sizeof(T);
     constexpr int BM = 32 * RV, BN = 32 * RV;
     const bool ak = v.inner == 1;
@@ -1053,6 +1096,70 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     }
 #undef TLIBTTM_GEMM
     return cudaGetLastError();
+}
+
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
+cudaError_t dmma_launch(const View3& v, cudaStream_t s, const f64::Grid& gr, int sms, int split, int64_t lper, double* ws)
+{
+    constexpr int smem = (int)sizeof(f64::Smem<BM, NF, ST, AK, BCM>);
+    const auto kernel = dmma_gemm_kernel<BM, NF, ST, AK, VEC, BCM>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t tiles = ceil_div(v.outer * v.inner, BM) * gr.cols;
+    // Short l ranges: a fixed set of blocks walks the tiles, so that the ring stays full across
+    // them (n_q = 16, A 256 MB: m = 64 147 -> 114 us, m = 8 94 -> 67 us). Longer ones: a block per
+    // tile, which the scheduler balances better (m = 64, n_q = 48: 97 us against 113).
+    const bool walk = v.nq <= (NF <= 2 ? 8 : 2) * f64::BK;
+    const int64_t slots = (int64_t)sms * (BM == 128 ? 2 : 5);
+    const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
+    kernel<<<grid, 2 * BM, smem, s>>>(v, gr, tiles, lper, ws);
+    return cudaGetLastError();
+}
+
+template <int BM, int NF, int ST>
+cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const f64::Grid& gr, int sms, int split, int64_t lper, double* ws)
+{
+    const bool ak = v.inner == 1;
+    const bool vec = aligned16(v.a) && (ak ? v.nq : v.inner) % 2 == 0;
+#define TLIBTTM_DMMA(AKv, VECv) \
+    (v.b_cm ? dmma_launch<BM, NF, ST, AKv, VECv, true>(v, s, gr, sms, split, lper, ws) \
+            : dmma_launch<BM, NF, ST, AKv, VECv, false>(v, s, gr, sms, split, lper, ws))
+    if (ak) return vec ? TLIBTTM_DMMA(true, true) : TLIBTTM_DMMA(true, false);
+    return vec ? TLIBTTM_DMMA(false, true) : TLIBTTM_DMMA(false, false);
+#undef TLIBTTM_DMMA
+}
+
+// Widest column tile in groups of eight: 64 columns where the tiles fill the GPU, narrower ones
+// (more blocks, A's rows shared through L2) where they do not.
+int dmma_width(const View3& v, int sms)
+{
+    const int64_t rows = ceil_div(v.outer * v.inner, 128), groups = ceil_div(v.m, 8);
+    for (int nf : {8, 4})
+        if (groups > nf / 2 && rows * ceil_div(groups, nf) >= sms) return nf;
+    return 2;
+}
+
+cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, int64_t lper = 0, double* ws = nullptr)
+{
+    int sms = 0;
+    const cudaError_t e = sms_of_device(sms);
+    if (e != cudaSuccess) return e;
+    const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % 2 == 0;
+    const f64::Grid gr = f64::split_columns(v.m, split > 1 ? (v.m > 16 ? 8 : 2) : dmma_width(v, sms));
+    switch (gr.nf) {
+    case 1:
+        return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws)
+                   : dmma_dispatch_nf<128, 1, 4>(v, s, gr, sms, split, lper, ws);
+    case 2:
+        return vec ? dmma_dispatch_nf<64, 2, 4>(v, s, gr, sms, split, lper, ws)
+                   : dmma_dispatch_nf<128, 2, 4>(v, s, gr, sms, split, lper, ws);
+    case 3: return dmma_dispatch_nf<128, 3, 4>(v, s, gr, sms, split, lper, ws);
+    case 4: return dmma_dispatch_nf<128, 4, 4>(v, s, gr, sms, split, lper, ws);
+    case 5: return dmma_dispatch_nf<128, 5, 3>(v, s, gr, sms, split, lper, ws);
+    case 6: return dmma_dispatch_nf<128, 6, 3>(v, s, gr, sms, split, lper, ws);
+    case 7: return dmma_dispatch_nf<128, 7, 3>(v, s, gr, sms, split, lper, ws);
+    default: return dmma_dispatch_nf<128, 8, 3>(v, s, gr, sms, split, lper, ws);
+    }
 }
 
 template <typename T, int W, int LS>
@@ -1423,30 +1530,15 @@ cudaError_t bvec_dispatch(const View3& v, int sms, cudaStream_t s, int* launches
     return e;
 }
 
-int g_sms_simt = 0;
-
-cudaError_t sms_of_device(int& sms)
-{
-    if (!g_sms_simt) {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms_simt, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-    }
-    sms = g_sms_simt;
-    return cudaSuccess;
-}
-
 // Parts of the K loop for a slice-GEMM whose tiles cannot fill the GPU (1 when none is needed).
 // `force` (a tuner's schedule): split whenever n_q >= 2048, into enough parts for two rounds of
 // blocks.
 template <typename T>
 int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
 {
-    constexpr int RV = 16 / sizeof(T);
-    constexpr int64_t BM = 32 * RV, BN = 32 * RV, BK = 8;
+    constexpr int64_t BM = 128, BN = sizeof(T) == 8 ? 64 : 128, BK = 8;
     const int64_t tiles = ceil_div(v.outer * v.inner, BM) * ceil_div(v.m, BN);
-    const int64_t slots = (int64_t)sms * (sizeof(T) == 8 ? 3 : 2);
+    const int64_t slots = (int64_t)sms * 2;
     lper = v.nq;
     if (v.nq < 2048 || (!force && tiles * 2 > slots)) return 1;
     int64_t S = std::min<int64_t>(ceil_div(slots, tiles), v.nq / 1024);
@@ -1461,19 +1553,19 @@ int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
 }
 
 template <typename T>
-cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool force)
+cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool force, bool may_split)
 {
     int sms = 0;
     cudaError_t e = sms_of_device(sms);
     if (e != cudaSuccess) return e;
     int64_t lper = 0;
-    const int S = gemm_split_parts<T>(v, sms, lper, force);
+    const int S = may_split ? gemm_split_parts<T>(v, sms, lper, force) : 1;
     if (launches) *launches = S > 1 ? 2 : 1;
-    if (S <= 1) return simt_gemm_dispatch<T>(v, s);
+    if (S <= 1) return simt_gemm_dispatch(v, s, 1, 0, static_cast<T*>(nullptr));
     const int64_t nc = v.outer * v.m * v.inner;
     T* ws = nullptr;
     if ((e = dev_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess) return e;
-    e = simt_gemm_dispatch<T>(v, s, S, lper, ws);
+    e = simt_gemm_dispatch(v, s, S, lper, ws);
     if (e == cudaSuccess) {
         split_reduce_kernel<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nc, 256), 4096)), 256, 0, s>>>(
             ws, S, nc, static_cast<T*>(v.c));
@@ -1485,10 +1577,28 @@ cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool
 
 }  // namespace
 
-cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches, bool force_split)
+cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches, bool force_split, bool may_split)
 {
-    return dtype == 0 ? simt_gemm_launch<float>(v, s, launches, force_split)
-                      : simt_gemm_launch<double>(v, s, launches, force_split);
+    return dtype == 0 ? simt_gemm_launch<float>(v, s, launches, force_split, may_split)
+                      : simt_gemm_launch<double>(v, s, launches, force_split, may_split);
+}
+
+// Measured over A of 2^14 to 2^26 doubles, n_q 3 to 2001, inner 1 to 1001, as time of the small-m
+// kernel over time of the slice-GEMM tile of 8 or 16 columns:
+//   m 9..16   1.1-2.8 from n_q = 12 on (0.7-1.0 at n_q = 8; fibres of at most 16 keep their kernels); rows of i off 16-byte boundaries
+//             1.3-3.6 from n_q = 64, 0.95-1.07 at 24
+//   m 5..8    1.1-1.6 from n_q = 250, 0.85-1.2 at 64
+//   m <= 4    1.0-1.7 from n_q = 250 where the TMA-fed kernel does not take the problem; where it
+//             does, that kernel reads A at the copy rate already
+// Few row tiles leave the GPU idle: long contiguous fibres then go to the l-split kernels, strided
+// rows to the column kernel's l split.
+bool small_m_takes_gemm_f64(const View3& v, bool tma)
+{
+    const int64_t tiles = ceil_div(v.outer * v.inner, kGemmRows);
+    if (v.inner == 1) return v.nq > (v.m > 8 ? kFlatMaxNq : 127) && (v.nq < 1024 || tiles >= 16) && (v.m > 4 || !tma);
+    const bool vec = aligned16(v.a) && v.inner % 2 == 0;
+    if (v.m > 8) return tiles >= 16 && v.nq >= (vec ? 12 : 32);
+    return tiles >= 128 && v.nq >= 128 && (v.m > 4 || !vec);
 }
 
 int simt_gemm_launch_count(const View3& v, int dtype)
@@ -1547,19 +1657,37 @@ cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s)
     return dtype == 0 ? rowdot_dispatch<float>(v, s) : rowdot_dispatch<double>(v, s);
 }
 
+void grouped_columns(int64_t m, int dtype, int64_t* tiles, int* cols)
+{
+    if (dtype == 0) {
+        *cols = 128;
+        *tiles = ceil_div(m, 128);
+    } else {
+        const f64::Grid g = f64::split_columns(m, kGroupNF);
+        *tiles = g.cols;
+        *cols = g.nf * 8;
+    }
+}
+
 int grouped_blocks_per_sm(int dtype)
 {
     int n = 0;
-    cudaError_t e = dtype == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grouped_kernel<float>, 256, 0)
-                               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grouped_kernel<double>, 256, 0);
+    cudaError_t e = dtype == 0 ? cudaSuccess
+                               : cudaFuncSetAttribute(grouped_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)grouped_smem_bytes<double>());
+    if (e == cudaSuccess)
+        e = dtype == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grouped_kernel<float>, 256,
+                                                                       grouped_smem_bytes<float>())
+                       : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, grouped_kernel<double>, 256,
+                                                                       grouped_smem_bytes<double>());
     return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
 cudaError_t launch_grouped(const GroupDesc* d_desc, int count, int64_t total, unsigned long long* queue, int dtype,
                            int grid, cudaStream_t s)
 {
-    if (dtype == 0) grouped_kernel<float><<<grid, 256, 0, s>>>(d_desc, count, total, queue);
-    else grouped_kernel<double><<<grid, 256, 0, s>>>(d_desc, count, total, queue);
+    if (dtype == 0) grouped_kernel<float><<<grid, 256, grouped_smem_bytes<float>(), s>>>(d_desc, count, total, queue);
+    else grouped_kernel<double><<<grid, 256, grouped_smem_bytes<double>(), s>>>(d_desc, count, total, queue);
     return cudaGetLastError();
 }
 

@@ -19,6 +19,12 @@ static __device__ __forceinline__ unsigned long long pair_dup(float x)
     asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
     return r;
 }
+static __device__ __forceinline__ unsigned long long pair_of(float lo, float hi)
+{
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
 static __device__ __forceinline__ float pair_lo(unsigned long long r) { return __uint_as_float((unsigned)r); }
 static __device__ __forceinline__ float pair_hi(unsigned long long r) { return __uint_as_float((unsigned)(r >> 32)); }
 #endif
@@ -77,6 +83,14 @@ struct GroupDesc {
     int64_t first;     // index of the problem's first work item
 };
 
+// Column tiles of a slice-GEMM: `cols` of them per row tile, of nf groups of columns each (of
+// eight, or four in the narrow FP32 tiles). Tile t covers row tile t / cols and the groups from
+// nf (t % cols) on.
+struct ColumnGrid {
+    int64_t cols;
+    int nf;
+};
+
 // Kernel identifiers (for diagnostics and launch counting).
 enum KernelId : int {
     K_NONE = 0,
@@ -106,9 +120,9 @@ const char* kernel_name(int id);
 // may_split false: never (one launch).
 cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr,
                              bool force_split = false, bool may_split = true);
-// Double, m <= kSmallM: whether the matrix-instruction slice-GEMM is the faster choice against the
-// small-m kernels (`tma`: the TMA-fed one would take the problem).
-bool small_m_takes_gemm_f64(const View3& v, bool tma);
+// m <= kSmallM: whether the slice-GEMM is the faster choice against the small-m kernels (`tma`: the
+// TMA-fed one would take the problem).
+bool small_m_takes_gemm(const View3& v, int dtype, bool tma);
 int simt_gemm_launch_count(const View3& v, int dtype);
 // Few output rows (outer * inner <= 8), 16 < m <= 256, n_q >= 4096: a kernel that streams B with
 // the l range split over the GPU, then a fixed-order reduction (*launches = 2).
@@ -143,6 +157,25 @@ int grouped_blocks_per_sm(int dtype);
 constexpr int64_t kSmallM = 16;
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// The column tiles of m columns, as even as possible, at most nf_max groups wide.
+inline ColumnGrid split_columns(int64_t m, int nf_max, int group = 8)
+{
+    const int64_t groups = ceil_div(m, group);
+    ColumnGrid g;
+    g.cols = ceil_div(groups, nf_max);
+    g.nf = (int)ceil_div(groups, g.cols);
+    return g;
+}
+
+#ifdef __CUDACC__
+// a / b for non-negative a, in 32 bits where both fit
+static __device__ __forceinline__ int64_t slice_of(int64_t a, int64_t b)
+{
+    if ((((uint64_t)a | (uint64_t)b) >> 32) == 0) return (int64_t)((uint32_t)a / (uint32_t)b);
+    return a / b;
+}
+#endif
 
 // Division of 32-bit unsigned n by a divisor d fixed at set-up, by multiplication (Granlund and
 // Montgomery, "Division by invariant integers using multiplication", 1994): with l = ceil(log2 d)

@@ -54,13 +54,6 @@ __device__ __forceinline__ void copy8(void* dst, const void* src, bool ok)
                  : "memory");
 }
 
-// row / inner, in 32 bits where both fit
-__device__ __forceinline__ int64_t slice_of(int64_t row, int64_t inner)
-{
-    if ((((uint64_t)row | (uint64_t)inner) >> 32) == 0) return (int64_t)((uint32_t)row / (uint32_t)inner);
-    return row / inner;
-}
-
 // One stage (16 l) of a warp's 16 rows x 8 N columns. At most eight columns: two accumulation
 // chains (even and odd l / 4), added by the caller at the end.
 template <int N, bool AK, bool BCM, int AR, int AP, int BR, int BP, int NA>
@@ -91,19 +84,12 @@ __device__ __forceinline__ void stage(const double (&sa)[AR][AP], const double (
     }
 }
 
-// The column tiles of a problem: `cols` of them per row tile, nf groups of eight columns each.
-// Tile t covers rows [BM (t / cols), ...) and columns [8 nf (t % cols), ...).
-struct Grid {
-    int64_t cols;
-    int nf;
-};
-
 // Tiles first, first + step, ... below `last`, l in [l_begin, l_end) of each; the stages of
 // consecutive tiles follow one another through the ring, so that the next tile's loads are in
 // flight while this one's results are stored. VEC: 16-byte copies of A (alignment checked by the
 // host). The caller synchronises the block between two calls that share `sm`.
 template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, bool EXACT>
-__device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t step, int64_t last, const Grid& gr,
+__device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t step, int64_t last, const ColumnGrid& gr,
                                       Smem<BM, NF, ST, AK, BCM>& sm, int64_t l_begin, int64_t l_end)
 {
     constexpr int BN = NF * 8, NT = 2 * BM, NA = NF == 1 ? 2 : NF;
@@ -119,6 +105,7 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     constexpr int WA = VEC ? 2 : 1, LA = BM * BK / WA / NT;
     constexpr int AX = (AK ? BK : BM) / WA;          // copies along the contiguous extent
     constexpr int AY = NT / AX;                      // rows of copies per pass
+    static_assert(AX <= NT && AX * WA == (AK ? BK : BM) && AY * LA == (AK ? BM : BK), "the copies of a stage cover the tile exactly");
     const int ax = (tid % AX) * WA, ay = tid / AX;
     // B copies: 8 bytes each (any alignment of m and n_q), of the columns below 8 nf only
     constexpr int BX = !BCM ? BK : NF == 1 ? 8 : NF == 2 ? 16 : NF <= 4 ? 32 : 64, BY = NT / BX;
@@ -282,17 +269,6 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
         }
     }
     }
-}
-
-// Column tiles of a problem of m columns, and the width of each in groups of eight: as even as
-// possible, at most NF groups.
-__host__ __device__ inline Grid split_columns(int64_t m, int nf_max)
-{
-    const int64_t groups = ceil_div(m, 8);
-    Grid g;
-    g.cols = ceil_div(groups, nf_max);
-    g.nf = (int)ceil_div(groups, g.cols);
-    return g;
 }
 
 }  // namespace f64

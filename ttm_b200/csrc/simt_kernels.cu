@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_f32.cuh"
 #include "gemm_f64.cuh"
 
 namespace tlibttm {
@@ -63,289 +64,52 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fma
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // ---------------------------------------------------------------------------------------------
-// simt_gemm
-//   (float; the FP64 tile is in gemm_f64.cuh)
+// simt_gemm: the slice-GEMM (tiles in gemm_f32.cuh and gemm_f64.cuh).
 //   AK   : A is K-major (inner == 1, fibres contiguous); otherwise rows (i) are contiguous.
-//   VEC  : 16-byte vector loads of A and vector stores of C (alignment and divisibility checked
-//          by the host).
+//   VEC  : 16-byte copies of A (alignment and divisibility checked by the host).
 //   BCM  : B column-major.
+// Column tiles of a row tile are next to one another in the grid, so that they share A's rows in
+// L2. With gridDim.z > 1 the l loop is split: part z covers l in [z * lper, min(n_q, (z + 1) *
+// lper)) and writes its partial tile into ws + z * (outer * m * inner), a buffer with C's own
+// layout; split_reduce_kernel then adds the parts in a fixed order, so the result does not depend
+// on scheduling.
 // ---------------------------------------------------------------------------------------------
 template <typename T>
-struct GemmSmem {
-    static constexpr int RV = 16 / sizeof(T);
-    __align__(16) T As[2][8][32 * RV];
-    __align__(16) T Bs[2][8][32 * RV];
-};
-
-// One BM x BN output tile (rows m0.., columns n0..) of the slice-GEMM, all 256 threads of the block.
-template <typename T, bool AK, bool VEC, bool BCM>
-__device__ __forceinline__ void gemm_tile(const View3& v, int64_t m0, int64_t n0, GemmSmem<T>& sm,
-                                          int64_t l_begin = 0, int64_t l_end = -1)
+__device__ __forceinline__ void split_range(View3& v, int64_t lper, T* ws, int64_t& l0, int64_t& l1)
 {
-    constexpr int RV = 16 / sizeof(T);   // elements per 16-byte vector
-    constexpr int BM = 32 * RV, BN = 32 * RV, BK = 8;
-    constexpr int TM = 2 * RV, TN = 2 * RV;
-    constexpr int NT = 256;
-    constexpr int WA = VEC ? RV : 1;
-    // A tile: BM rows x BK columns, loaded as NVA vectors of WA elements.
-    constexpr int NVA = BM * BK / WA;
-    constexpr int LA = NVA / NT;
-    constexpr int ACONT = AK ? BK : BM;          // extent of A's contiguous tile dimension
-    // B tile: BK x BN, scalar loads.
-    constexpr int LB = BN * BK / NT;
-
-    auto& As = sm.As;
-    auto& Bs = sm.Bs;
-
-    const T* __restrict__ A = static_cast<const T*>(v.a);
-    const T* __restrict__ B = static_cast<const T*>(v.b);
-    T* __restrict__ Cp = static_cast<T*>(v.c);
-    const int64_t inner = v.inner, m = v.m;
-    // the l range of this tile: all of n_q, or one part of a split K loop (l_begin % BK == 0)
-    const int64_t nq = l_end < 0 ? v.nq : l_end;
-    const int64_t nq_full = v.nq;
-    const int64_t M = v.outer * inner;
-    const int tid = threadIdx.x;
-    const int tx = tid % 16, ty = tid / 16;
-
-    // Per-slot A addressing, fixed for the whole K loop.
-    int64_t abase[LA];
-    int a_loff[LA], a_roff[LA];
-    bool arow_ok[LA];
-#pragma unroll
-    for (int s = 0; s < LA; ++s) {
-        const int vi = tid + s * NT;
-        const int c = (vi % (ACONT / WA)) * WA;
-        const int o = vi / (ACONT / WA);
-        const int roff = AK ? o : c;
-        const int loff = AK ? c : o;
-        const int64_t row = m0 + roff;
-        arow_ok[s] = row < M;
-        const int64_t k = arow_ok[s] ? row / inner : 0;
-        const int64_t i = arow_ok[s] ? row - k * inner : 0;
-        abase[s] = k * inner * nq_full + i;
-        a_loff[s] = loff;
-        a_roff[s] = roff;
-    }
-
-    T ra[LA][WA];
-    T rb[LB];
-
-    auto load_tiles = [&](int64_t l0) {
-#pragma unroll
-        for (int s = 0; s < LA; ++s) {
-            const int64_t l = l0 + a_loff[s];
-            if (arow_ok[s] && l < nq) {
-                load_vec<T, WA>(ra[s], A + abase[s] + l * inner);
-            } else {
-#pragma unroll
-                for (int w = 0; w < WA; ++w) ra[s][w] = T(0);
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < LB; ++s) {
-            const int vi = tid + s * NT;
-            int jo, lo;
-            if (BCM) { jo = vi % BN; lo = vi / BN; }
-            else     { lo = vi % BK; jo = vi / BK; }
-            const int64_t j = n0 + jo, l = l0 + lo;
-            T val = T(0);
-            if (j < m && l < nq) val = __ldg(BCM ? B + j + l * m : B + j * nq_full + l);
-            rb[s] = val;
-        }
-    };
-    auto store_tiles = [&](int buf) {
-#pragma unroll
-        for (int s = 0; s < LA; ++s) {
-#pragma unroll
-            for (int w = 0; w < WA; ++w) {
-                if (AK) As[buf][a_loff[s] + w][a_roff[s]] = ra[s][w];
-                else    As[buf][a_loff[s]][a_roff[s] + w] = ra[s][w];
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < LB; ++s) {
-            const int vi = tid + s * NT;
-            int jo, lo;
-            if (BCM) { jo = vi % BN; lo = vi / BN; }
-            else     { lo = vi % BK; jo = vi / BK; }
-            Bs[buf][lo][jo] = rb[s];
-        }
-    };
-
-    // FP32 accumulates in packed column pairs (acc2[i][j / 2], column j in the low half when j
-    // is even): half the FMA instructions of one per output
-    constexpr bool PK = std::is_same<T, float>::value;
-    T acc[TM][TN];
-    unsigned long long acc2[PK ? TM : 1][PK ? TN / 2 : 1];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
-    if constexpr (PK) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN / 2; ++j) acc2[i][j] = 0ull;
-    }
-
-    const int64_t nk = ceil_div(nq - l_begin, BK);
-    load_tiles(l_begin);
-    store_tiles(0);
-    __syncthreads();
-
-    for (int64_t kt = 0; kt < nk; ++kt) {
-        const int buf = kt & 1;
-        if (kt + 1 < nk) load_tiles(l_begin + (kt + 1) * BK);
-#pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            if constexpr (PK) {
-                const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][ty * RV]);
-                const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][kk][BM / 2 + ty * RV]);
-                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][kk][tx * RV]);
-                const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][kk][BN / 2 + tx * RV]);
-                const unsigned long long bp[TN / 2] = {b0.x, b0.y, b1.x, b1.y};
-                const float af[TM] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-                for (int i = 0; i < TM; ++i) {
-                    const unsigned long long ap = pair_dup(af[i]);
-#pragma unroll
-                    for (int j = 0; j < TN / 2; ++j) ffma2(acc2[i][j], ap, bp[j]);
-                }
-                continue;
-            }
-            T af[TM], bf[TN];
-            typedef typename V16<T>::type VT;
-            VT a0 = *reinterpret_cast<const VT*>(&As[buf][kk][ty * RV]);
-            VT a1 = *reinterpret_cast<const VT*>(&As[buf][kk][BM / 2 + ty * RV]);
-            VT b0 = *reinterpret_cast<const VT*>(&Bs[buf][kk][tx * RV]);
-            VT b1 = *reinterpret_cast<const VT*>(&Bs[buf][kk][BN / 2 + tx * RV]);
-#pragma unroll
-            for (int r = 0; r < RV; ++r) {
-                af[r] = reinterpret_cast<const T*>(&a0)[r];
-                af[RV + r] = reinterpret_cast<const T*>(&a1)[r];
-                bf[r] = reinterpret_cast<const T*>(&b0)[r];
-                bf[RV + r] = reinterpret_cast<const T*>(&b1)[r];
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fma_t(af[i], bf[j], acc[i][j]);
-        }
-        if (kt + 1 < nk) store_tiles(buf ^ 1);
-        __syncthreads();
-    }
-
-    if constexpr (PK) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN / 2; ++j) {
-                acc[i][2 * j] = pair_lo(acc2[i][j]);
-                acc[i][2 * j + 1] = pair_hi(acc2[i][j]);
-            }
-    }
-
-    // Epilogue: C(row, j) = cbase(row) + j*inner, cbase = (row/inner)*inner*m + row%inner.
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int64_t row0 = m0 + h * (BM / 2) + ty * RV;
-        if (!AK && VEC) {
-            // RV consecutive rows share one k (inner % RV == 0): one vector per column.
-            if (row0 < M) {
-                const int64_t k = row0 / inner;
-                const int64_t cb = k * inner * m + (row0 - k * inner);
-#pragma unroll
-                for (int g = 0; g < 2; ++g)
-#pragma unroll
-                    for (int c = 0; c < RV; ++c) {
-                        const int64_t j = n0 + g * (BN / 2) + tx * RV + c;
-                        if (j < m) {
-                            T r[RV];
-#pragma unroll
-                            for (int w = 0; w < RV; ++w) r[w] = acc[h * RV + w][g * RV + c];
-                            store_vec<T, RV>(Cp + cb + j * inner, r);
-                        }
-                    }
-            }
-        } else if (AK && VEC) {
-            // inner == 1 and m % RV == 0: RV consecutive columns are contiguous.
-#pragma unroll
-            for (int w = 0; w < RV; ++w) {
-                const int64_t row = row0 + w;
-                if (row < M) {
-#pragma unroll
-                    for (int g = 0; g < 2; ++g) {
-                        const int64_t j0 = n0 + g * (BN / 2) + tx * RV;
-                        if (j0 < m) {
-                            T r[RV];
-#pragma unroll
-                            for (int c = 0; c < RV; ++c) r[c] = acc[h * RV + w][g * RV + c];
-                            store_vec<T, RV>(Cp + row * m + j0, r);
-                        }
-                    }
-                }
-            }
-        } else {
-#pragma unroll
-            for (int w = 0; w < RV; ++w) {
-                const int64_t row = row0 + w;
-                if (row < M) {
-                    const int64_t k = row / inner;
-                    const int64_t cb = k * inner * m + (row - k * inner);
-#pragma unroll
-                    for (int g = 0; g < 2; ++g)
-#pragma unroll
-                        for (int c = 0; c < RV; ++c) {
-                            const int64_t j = n0 + g * (BN / 2) + tx * RV + c;
-                            if (j < m) Cp[cb + j * inner] = acc[h * RV + w][g * RV + c];
-                        }
-                }
-            }
-        }
-    }
-}
-
-// Two CTAs per SM in float (at most 128 registers a thread: 16 warps of 128 fill each
-// sub-partition's quarter of the register file), three in double (at most 80).
-template <typename T, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 3 : 2)) simt_gemm_kernel(View3 v)
-{
-    constexpr int RV = 16 / sizeof(T);
-    __shared__ GemmSmem<T> sm;
-    gemm_tile<T, AK, VEC, BCM>(v, (int64_t)blockIdx.x * (32 * RV), (int64_t)blockIdx.y * (32 * RV), sm);
-}
-
-// The K loop split `gridDim.z` ways: part z covers l in [z * lper, min(n_q, (z + 1) * lper)) and
-// writes its partial tile into ws + z * (outer * m * inner), a buffer with C's own layout;
-// split_reduce_kernel then adds the parts in a fixed order, so the result does not depend on
-// scheduling.
-template <typename T, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(256, (sizeof(T) == 8 ? 3 : 2)) simt_gemm_split_kernel(View3 v, int64_t lper, T* ws)
-{
-    constexpr int RV = 16 / sizeof(T);
-    __shared__ GemmSmem<T> sm;
-    const int64_t l0 = (int64_t)blockIdx.z * lper;
-    const int64_t l1 = l0 + lper < v.nq ? l0 + lper : v.nq;
-    View3 part = v;
-    part.c = ws + (size_t)blockIdx.z * (size_t)(v.outer * v.m * v.inner);
-    gemm_tile<T, AK, VEC, BCM>(part, (int64_t)blockIdx.x * (32 * RV), (int64_t)blockIdx.y * (32 * RV), sm, l0, l1);
-}
-
-// FP64: tiles of 128 x 8 nf (gemm_f64.cuh), column tiles next to one another so that they share
-// A's rows in L2. gridDim.z parts of the l range write partial results to ws, as above.
-template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 5) dmma_gemm_kernel(View3 v, f64::Grid gr, int64_t tiles, int64_t lper, double* ws)
-{
-    extern __shared__ __align__(16) unsigned char dmma_smem[];
-    auto& sm = *reinterpret_cast<f64::Smem<BM, NF, ST, AK, BCM>*>(dmma_smem);
-    int64_t l0 = 0, l1 = v.nq;
+    l0 = 0;
+    l1 = v.nq;
     if (gridDim.z > 1) {
         l0 = (int64_t)blockIdx.z * lper;
         l1 = l0 + lper < v.nq ? l0 + lper : v.nq;
         v.c = ws + (size_t)blockIdx.z * (size_t)(v.outer * v.m * v.inner);
     }
-    f64::tiles<BM, NF, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr, sm, l0, l1);
+}
+
+// Blocks per SM of the FP32 builds: 16 warps of at most 128 registers, or of 80-100 where the
+// accumulators are small.
+constexpr int ffma_blocks(int TX, int TM) { return TX == 8 ? 2 : TM == 8 ? 4 : 5; }
+
+template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
+__global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
+                                                                               int64_t lper, float* ws)
+{
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    int64_t l0, l1;
+    split_range(v, lper, ws, l0, l1);
+    f32::tiles<TX, TM, TN, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr,
+                                                   *reinterpret_cast<f32::Smem<TX, TM, TN, ST, AK>*>(gemm_smem), l0, l1);
+}
+
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
+__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 5) dmma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
+                                                                             int64_t lper, double* ws)
+{
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    int64_t l0, l1;
+    split_range(v, lper, ws, l0, l1);
+    f64::tiles<BM, NF, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr,
+                                               *reinterpret_cast<f64::Smem<BM, NF, ST, AK, BCM>*>(gemm_smem), l0, l1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -941,7 +705,9 @@ constexpr int kGroupNF = 8, kGroupST = 3;   // the FP64 tile of the grouped laun
 template <typename T>
 constexpr size_t grouped_smem_bytes()
 {
-    if (sizeof(T) == 4) return sizeof(GemmSmem<T>);
+    if (sizeof(T) == 4)
+        return std::max(sizeof(f32::Smem<8, kGemmRows / 32, kGroupNF, kGroupST, true>),
+                        sizeof(f32::Smem<8, kGemmRows / 32, kGroupNF, kGroupST, false>));
     const size_t rows = sizeof(f64::Smem<kGemmRows, kGroupNF, kGroupST, true, false>),
                  cols = sizeof(f64::Smem<kGemmRows, kGroupNF, kGroupST, false, true>);
     return std::max(rows, cols);   // the largest of the four forms: one pitch of A with one of B
@@ -962,7 +728,6 @@ template <typename T>
 __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __restrict__ desc, int count, int64_t total,
                                                       unsigned long long* queue)
 {
-    constexpr int BM = 128, BN = 128;
     extern __shared__ __align__(16) unsigned char grouped_smem[];
     __shared__ int64_t item_s;
     for (;;) {
@@ -988,8 +753,8 @@ __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __rest
         v.m = g.m;
         v.b_cm = g.b_cm;
         const bool ak = g.flags & 1, vec = g.flags & 2;
+        const ColumnGrid gr{g.tiles_n, g.cols / 8};
         if constexpr (sizeof(T) == 8) {
-            const f64::Grid gr{g.tiles_n, g.cols / 8};
 #define TLIBTTM_TILE(AKv, VECv, BCMv)                                                                        \
     f64::tiles<kGemmRows, kGroupNF, kGroupST, AKv, VECv, BCMv, false>(v, local, 1, local + 1, gr,                    \
                                                    *reinterpret_cast<f64::Smem<kGemmRows, kGroupNF, kGroupST, AKv, BCMv>*>(grouped_smem), \
@@ -997,9 +762,10 @@ __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __rest
             TLIBTTM_TILES
 #undef TLIBTTM_TILE
         } else {
-            auto& gm = *reinterpret_cast<GemmSmem<T>*>(grouped_smem);
-            const int64_t m0 = (local / g.tiles_n) * BM, n0 = (local % g.tiles_n) * BN;
-#define TLIBTTM_TILE(AKv, VECv, BCMv) gemm_tile<T, AKv, VECv, BCMv>(v, m0, n0, gm)
+#define TLIBTTM_TILE(AKv, VECv, BCMv)                                                                                 \
+    f32::tiles<8, kGemmRows / 32, kGroupNF, kGroupST, AKv, VECv, BCMv, false>(v, local, 1, local + 1, gr,                \
+                                                                           *reinterpret_cast<f32::Smem<8, kGemmRows / 32, kGroupNF, kGroupST, AKv>*>(grouped_smem), \
+                                                                           0, v.nq)
             TLIBTTM_TILES
 #undef TLIBTTM_TILE
         }
@@ -1070,36 +836,75 @@ cudaError_t sms_of_device(int& sms)
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, int64_t lper = 0, float* ws = nullptr)
+template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
+cudaError_t ffma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, float* ws)
 {
-    using T = float;
-    constexpr int RV = 16 / sizeof(T);
-    constexpr int BM = 32 * RV, BN = 32 * RV;
-    const bool ak = v.inner == 1;
-    bool vec = aligned16(v.a) && aligned16(split > 1 ? static_cast<const void*>(ws) : v.c);
-    if (ak) vec = vec && (v.nq % RV == 0) && (v.m % RV == 0);
-    else vec = vec && (v.inner % RV == 0);
-    const int64_t M = v.outer * v.inner;
-    dim3 grid((unsigned)ceil_div(M, BM), (unsigned)ceil_div(v.m, BN), (unsigned)split);
-    dim3 block(256);
-#define TLIBTTM_GEMM(AKv, VECv, BCMv)                                                            \
-    do {                                                                                        \
-        if (split > 1) simt_gemm_split_kernel<T, AKv, VECv, BCMv><<<grid, block, 0, s>>>(v, lper, ws); \
-        else simt_gemm_kernel<T, AKv, VECv, BCMv><<<grid, block, 0, s>>>(v);                     \
-    } while (0)
-    if (ak) {
-        if (vec) { if (v.b_cm) TLIBTTM_GEMM(true, true, true); else TLIBTTM_GEMM(true, true, false); }
-        else     { if (v.b_cm) TLIBTTM_GEMM(true, false, true); else TLIBTTM_GEMM(true, false, false); }
-    } else {
-        if (vec) { if (v.b_cm) TLIBTTM_GEMM(false, true, true); else TLIBTTM_GEMM(false, true, false); }
-        else     { if (v.b_cm) TLIBTTM_GEMM(false, false, true); else TLIBTTM_GEMM(false, false, false); }
-    }
-#undef TLIBTTM_GEMM
+    constexpr int smem = (int)sizeof(f32::Smem<TX, TM, TN, ST, AK>);
+    const auto kernel = ffma_gemm_kernel<TX, TM, TN, ST, AK, VEC, BCM>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int64_t tiles = ceil_div(v.outer * v.inner, 32 * TM) * gr.cols;
+    // as in dmma_launch (m = 64, n_q = 16, A 64 MB: 86 -> 82 us; n_q = 64: 190 us against 197)
+    const bool walk = v.nq <= 2 * f32::BK;
+    const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM);
+    const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
+    kernel<<<grid, 32 * TX, smem, s>>>(v, gr, tiles, lper, ws);
     return cudaGetLastError();
 }
 
+template <int TX, int TM, int TN, int ST>
+cudaError_t ffma_dispatch_form(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, float* ws)
+{
+#define TLIBTTM_FFMA(AKv, VECv) \
+    (v.b_cm ? ffma_launch<TX, TM, TN, ST, AKv, VECv, true>(v, s, gr, sms, split, lper, ws) \
+            : ffma_launch<TX, TM, TN, ST, AKv, VECv, false>(v, s, gr, sms, split, lper, ws))
+    const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % 4 == 0;
+    if (v.inner == 1) return vec ? TLIBTTM_FFMA(true, true) : TLIBTTM_FFMA(true, false);
+    return vec ? TLIBTTM_FFMA(false, true) : TLIBTTM_FFMA(false, false);
+#undef TLIBTTM_FFMA
+}
+
+template <int TM, int ST>
+cudaError_t ffma_dispatch_narrow(const View3& v, cudaStream_t s, int sms, int split, int64_t lper, float* ws)
+{
+    const ColumnGrid gr = split_columns(v.m, 8, 4);
+    switch (gr.nf) {
+    case 1: return ffma_dispatch_form<4, TM, 1, ST>(v, s, gr, sms, split, lper, ws);
+    case 2: return ffma_dispatch_form<4, TM, 2, ST>(v, s, gr, sms, split, lper, ws);
+    case 3: return ffma_dispatch_form<4, TM, 3, ST>(v, s, gr, sms, split, lper, ws);
+    case 4: return ffma_dispatch_form<4, TM, 4, ST>(v, s, gr, sms, split, lper, ws);
+    case 5: return ffma_dispatch_form<4, TM, 5, ST>(v, s, gr, sms, split, lper, ws);
+    case 6: return ffma_dispatch_form<4, TM, 6, ST>(v, s, gr, sms, split, lper, ws);
+    case 7: return ffma_dispatch_form<4, TM, 7, ST>(v, s, gr, sms, split, lper, ws);
+    default: return ffma_dispatch_form<4, TM, 8, ST>(v, s, gr, sms, split, lper, ws);
+    }
+}
+
+cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, int64_t lper = 0, float* ws = nullptr)
+{
+    int sms = 0;
+    const cudaError_t e = sms_of_device(sms);
+    if (e != cudaSuccess) return e;
+    const int64_t rows = (split > 1 ? split : 1) * ceil_div(v.outer * v.inner, 256);
+    // Blocks of 8 x 8 outputs a thread where they fill both slots of every SM; up to 32 columns, and
+    // problems with fewer tiles, in the narrow form (its shared-memory reads per multiply-add are
+    // those of the wide form at half the columns: m = 24, A 160 MB 74 -> 59 us), with rows of 128
+    // where 256 would leave slots empty.
+    if (v.m > 32 && rows * ceil_div(v.m, 64) >= 2 * sms) {
+        const ColumnGrid gr = split_columns(v.m, 8);
+        switch (gr.nf) {
+        case 5: return ffma_dispatch_form<8, 8, 5, 4>(v, s, gr, sms, split, lper, ws);
+        case 6: return ffma_dispatch_form<8, 8, 6, 4>(v, s, gr, sms, split, lper, ws);
+        case 7: return ffma_dispatch_form<8, 8, 7, 4>(v, s, gr, sms, split, lper, ws);
+        default: return ffma_dispatch_form<8, 8, 8, 4>(v, s, gr, sms, split, lper, ws);
+        }
+    }
+    return rows * ceil_div(v.m, 32) >= 4 * sms ? ffma_dispatch_narrow<8, 3>(v, s, sms, split, lper, ws)
+                                                   : ffma_dispatch_narrow<4, 4>(v, s, sms, split, lper, ws);
+}
+
 template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
-cudaError_t dmma_launch(const View3& v, cudaStream_t s, const f64::Grid& gr, int sms, int split, int64_t lper, double* ws)
+cudaError_t dmma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws)
 {
     constexpr int smem = (int)sizeof(f64::Smem<BM, NF, ST, AK, BCM>);
     const auto kernel = dmma_gemm_kernel<BM, NF, ST, AK, VEC, BCM>;
@@ -1117,7 +922,7 @@ cudaError_t dmma_launch(const View3& v, cudaStream_t s, const f64::Grid& gr, int
 }
 
 template <int BM, int NF, int ST>
-cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const f64::Grid& gr, int sms, int split, int64_t lper, double* ws)
+cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws)
 {
     const bool ak = v.inner == 1;
     const bool vec = aligned16(v.a) && (ak ? v.nq : v.inner) % 2 == 0;
@@ -1145,7 +950,7 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     const cudaError_t e = sms_of_device(sms);
     if (e != cudaSuccess) return e;
     const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % 2 == 0;
-    const f64::Grid gr = f64::split_columns(v.m, split > 1 ? (v.m > 16 ? 8 : 2) : dmma_width(v, sms));
+    const ColumnGrid gr = split_columns(v.m, split > 1 ? (v.m > 16 ? 8 : 2) : dmma_width(v, sms));
     switch (gr.nf) {
     case 1:
         return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws)
@@ -1536,7 +1341,7 @@ cudaError_t bvec_dispatch(const View3& v, int sms, cudaStream_t s, int* launches
 template <typename T>
 int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
 {
-    constexpr int64_t BM = 128, BN = sizeof(T) == 8 ? 64 : 128, BK = 8;
+    constexpr int64_t BM = 128, BN = 64, BK = 16;
     const int64_t tiles = ceil_div(v.outer * v.inner, BM) * ceil_div(v.m, BN);
     const int64_t slots = (int64_t)sms * 2;
     lper = v.nq;
@@ -1583,20 +1388,31 @@ cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* lau
                       : simt_gemm_launch<double>(v, s, launches, force_split, may_split);
 }
 
-// Measured over A of 2^14 to 2^26 doubles, n_q 3 to 2001, inner 1 to 1001, as time of the small-m
-// kernel over time of the slice-GEMM tile of 8 or 16 columns:
-//   m 9..16   1.1-2.8 from n_q = 12 on (0.7-1.0 at n_q = 8; fibres of at most 16 keep their kernels); rows of i off 16-byte boundaries
-//             1.3-3.6 from n_q = 64, 0.95-1.07 at 24
+// Measured over A of 2^14 to 2^26 elements, n_q 3 to 2001, inner 1 to 1001, as time of the small-m
+// kernel over time of the slice-GEMM tile of that width.
+//   double
+//   m 9..16   1.1-2.8 from n_q = 12 on (0.7-1.0 at n_q = 8; fibres of at most 16 keep their
+//             kernels); rows of i off 16-byte boundaries 1.3-3.6 from n_q = 64, 0.95-1.07 at 24
 //   m 5..8    1.1-1.6 from n_q = 250, 0.85-1.2 at 64
 //   m <= 4    1.0-1.7 from n_q = 250 where the TMA-fed kernel does not take the problem; where it
 //             does, that kernel reads A at the copy rate already
+//   float
+//   m 9..16   rows of i 1.0-3.2 from n_q = 64 on (0.65-1.2 at 24, and 0.9 with rows of 8 elements);
+//             contiguous fibres on 16-byte boundaries 1.05-1.4 from n_q = 64, off them 1.4-10 at
+//             n_q = 2001 and 0.93-2.0 at 250
+//   m <= 8    mostly 0.6-1.1
 // Few row tiles leave the GPU idle: long contiguous fibres then go to the l-split kernels, strided
-// rows to the column kernel's l split.
-bool small_m_takes_gemm_f64(const View3& v, bool tma)
+// rows to the column kernel's l split (0.8-0.9 below about 16 tiles of 128 rows).
+bool small_m_takes_gemm(const View3& v, int dtype, bool tma)
 {
     const int64_t tiles = ceil_div(v.outer * v.inner, kGemmRows);
+    const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % (dtype == 0 ? 4 : 2) == 0;
+    if (dtype == 0) {
+        if (v.m <= 8) return false;
+        if (v.inner == 1) return v.nq >= (vec ? 64 : 512) && (v.nq < 1024 || tiles >= 16);
+        return tiles >= 32 && v.nq >= 64 && v.inner >= 64;
+    }
     if (v.inner == 1) return v.nq > (v.m > 8 ? kFlatMaxNq : 127) && (v.nq < 1024 || tiles >= 16) && (v.m > 4 || !tma);
-    const bool vec = aligned16(v.a) && v.inner % 2 == 0;
     if (v.m > 8) return tiles >= 16 && v.nq >= (vec ? 12 : 32);
     return tiles >= 128 && v.nq >= 128 && (v.m > 4 || !vec);
 }
@@ -1659,20 +1475,17 @@ cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s)
 
 void grouped_columns(int64_t m, int dtype, int64_t* tiles, int* cols)
 {
-    if (dtype == 0) {
-        *cols = 128;
-        *tiles = ceil_div(m, 128);
-    } else {
-        const f64::Grid g = f64::split_columns(m, kGroupNF);
-        *tiles = g.cols;
-        *cols = g.nf * 8;
-    }
+    ColumnGrid g = split_columns(m, kGroupNF);
+    if (dtype == 0) g.nf = g.nf <= 4 ? 4 : g.nf <= 6 ? 6 : 8;   // the widths the FP32 tile is built for there
+    *tiles = ceil_div(m, g.nf * 8);
+    *cols = g.nf * 8;
 }
 
 int grouped_blocks_per_sm(int dtype)
 {
     int n = 0;
-    cudaError_t e = dtype == 0 ? cudaSuccess
+    cudaError_t e = dtype == 0 ? cudaFuncSetAttribute(grouped_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                      (int)grouped_smem_bytes<float>())
                                : cudaFuncSetAttribute(grouped_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                       (int)grouped_smem_bytes<double>());
     if (e == cudaSuccess)

@@ -268,45 +268,61 @@ __global__ void __launch_bounds__(kThreads, 1)
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            int issued[kMaxA];
-            for (int i = 0; i < kMaxA; ++i) issued[i] = -1;
+            // per slot (bit s): whether its last use was a copy of this warp, and that copy's phase
+            uint32_t copied = 0, phases = 0;
             const TcProb* last = nullptr;
             int cur = 0;
             for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 int64_t lt;
                 const TcProb& pr = tile_problem<GROUP>(one, P, t, cur, lt);
-                if (GROUP && &pr != last && !pr.ldg_a) tensormap_acquire(&pr.amap);
+                // all that the stages need, in registers before the first copy: this one lane issues
+                // every load of the CTA, and a division or a reload of the record per copy showed as
+                // 1100 of the 1200 cycles that a stage of 32 l took
+                const int kst = pr.kstages, kch = pr.kchunks, fold = pr.fold_kb;
+                const bool ldg = pr.ldg_a != 0;
+                const CUtensorMap* const amap = &pr.amap;
+                if (GROUP && &pr != last && !ldg) tensormap_acquire(amap);
                 last = &pr;
-                const int64_t mt = lt % pr.tiles_m, mper = (pr.inner + kBM - 1) / kBM;
-                for (int st = 0; st < pr.kstages; ++st) {
+                const int64_t tm = pr.tiles_m, mt = lt - slice_of(lt, tm) * tm;
+                int c0, ck = 0;   // first row (i, or the fibre for GEOM_K) and slice of the tile
+                if (GEOM == GEOM_MN && fold > 1) {
+                    // folded tile: slices mt*KB .. +KB-1, the map ordered (i, k, l)
+                    c0 = 0;
+                    ck = (int)(mt * fold);
+                } else if (GEOM == GEOM_MN) {
+                    const int64_t mper = (pr.inner + kBM - 1) / kBM, k = slice_of(mt, mper);
+                    c0 = (int)((mt - k * mper) * kBM);
+                    ck = (int)k;
+                } else {
+                    c0 = (int)(mt * kBM);
+                }
+                for (int st = 0; st < kst; ++st) {
                     if (!mbar_wait(&a_empty[s], ph ^ 1, abort_flag, P.wait_ns)) { ok = false; break; }
-                    if (pr.ldg_a) {
+                    if (ldg) {
                         // no copy: the stage is free for the converters, which load A themselves.
                         // No copy is in flight into it either (its last one landed before the
                         // stage was freed), so the final drain must not wait on it: a phase
                         // recorded by an earlier copy would by then be ambiguous by parity.
-                        issued[s] = -1;
+                        copied &= ~(1u << s);
                         mbar_arrive(&a_full[s]);
                         if (++s == AS) { s = 0; ph ^= 1; }
                         continue;
                     }
-                    issued[s] = (int)ph;
+                    copied |= 1u << s;
+                    phases = (phases & ~(1u << s)) | (ph << s);
                     // the sub-blocks within n_q (the last box's rows past n_q are zero-filled)
-                    const int nsub = min(kSub, pr.kchunks - st * kSub);
+                    const int nsub = min(kSub, kch - st * kSub);
                     mbar_expect_tx(&a_full[s], (uint32_t)nsub * LA.asub_bytes);
 #pragma unroll
                     for (int sub = 0; sub < kSub; ++sub) {
                         if (sub >= nsub) break;
                         uint8_t* dst = a_at(s) + sub * LA.asub_bytes;
                         const int l0 = (st * kSub + sub) * kBK;
-                        if (GEOM == GEOM_MN && pr.fold_kb > 1) {
-                            // folded tile: slices mt*KB .. +KB-1, the map ordered (i, k, l)
-                            tma_load_3d(dst, &pr.amap, &a_full[s], 0, (int)(mt * pr.fold_kb), l0);
-                        } else if (GEOM == GEOM_MN) {
-                            const int64_t k = mt / mper, ib = mt - k * mper;
-                            tma_load_3d(dst, &pr.amap, &a_full[s], (int)(ib * kBM), l0, (int)k);
+                        if (GEOM == GEOM_MN) {
+                            if (fold > 1) tma_load_3d(dst, amap, &a_full[s], 0, ck, l0);
+                            else tma_load_3d(dst, amap, &a_full[s], c0, l0, ck);
                         } else {
-                            tma_load_2d(dst, &pr.amap, &a_full[s], l0, (int)(mt * kBM));
+                            tma_load_2d(dst, amap, &a_full[s], l0, c0);
                         }
                     }
                     if (++s == AS) { s = 0; ph ^= 1; }
@@ -314,9 +330,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             // None of this CTA's bulk copies may still be in flight when it exits.
             for (int i = 0; i < AS; ++i) {
-                if (issued[i] < 0) continue;
+                if (!(copied >> i & 1u)) continue;
                 const unsigned long long t0 = gtimer();
-                while (!mbar_try(&a_full[i], (uint32_t)issued[i]) && gtimer() - t0 < kTimeoutNs) {}
+                while (!mbar_try(&a_full[i], phases >> i & 1u) && gtimer() - t0 < kTimeoutNs) {}
             }
         }
     } else if (warp == 2) {
@@ -325,33 +341,33 @@ __global__ void __launch_bounds__(kThreads, 1)
             int s = 0;
             uint32_t ph = 0;
             bool ok = true;
-            int issued[kMaxB];
-            for (int i = 0; i < kMaxB; ++i) issued[i] = -1;
+            uint32_t copied = 0, phases = 0;   // as in the A producer
             int cur = 0;
             for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 int64_t lt;
                 const TcProb& pr = tile_problem<GROUP>(one, P, t, cur, lt);
-                const SmemLayout Lp = smem_layout(pr.nt);
-                const int64_t jb = lt / pr.tiles_m;
-                for (int st = 0; st < pr.kstages; ++st) {
+                const int kst = pr.kstages;
+                const uint32_t bytes = smem_layout(pr.nt).bstage_bytes;
+                // the image holds kstages * kSub sub-blocks per j block: one copy per stage
+                const uint8_t* img = pr.bimg + (size_t)(slice_of(lt, pr.tiles_m) * kst) * bytes;
+                for (int st = 0; st < kst; ++st, img += bytes) {
                     if (!mbar_wait(&b_empty[s], ph ^ 1, abort_flag, P.wait_ns)) { ok = false; break; }
                     if (P.skip_b && t == blockIdx.x && st == 0) {
                         // test of the bounded waits: this stage is never filled (no copy, no arrive)
                         if (++s == BS) { s = 0; ph ^= 1; }
                         continue;
                     }
-                    issued[s] = (int)ph;
-                    mbar_expect_tx(&b_full[s], Lp.bstage_bytes);
-                    // the image holds kstages * kSub sub-blocks per j block: one copy per stage
-                    const uint8_t* img = pr.bimg + ((size_t)(jb * pr.kstages + st) * Lp.bstage_bytes);
-                    bulk_load(bhi_at(s), img, Lp.bstage_bytes, &b_full[s]);
+                    copied |= 1u << s;
+                    phases = (phases & ~(1u << s)) | (ph << s);
+                    mbar_expect_tx(&b_full[s], bytes);
+                    bulk_load(bhi_at(s), img, bytes, &b_full[s]);
                     if (++s == BS) { s = 0; ph ^= 1; }
                 }
             }
             for (int i = 0; i < BS; ++i) {
-                if (issued[i] < 0) continue;
+                if (!(copied >> i & 1u)) continue;
                 const unsigned long long t0 = gtimer();
-                while (!mbar_try(&b_full[i], (uint32_t)issued[i]) && gtimer() - t0 < kTimeoutNs) {}
+                while (!mbar_try(&b_full[i], phases >> i & 1u) && gtimer() - t0 < kTimeoutNs) {}
             }
         }
     } else if (warp == 1) {
@@ -373,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int64_t t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
                 int64_t lt;
                 const TcProb& pr = tile_problem<GROUP>(one, P, t, cur, lt);
-                const int kst = pr.kstages;
+                const int kst = pr.kstages, kch = pr.kchunks;
                 const uint32_t idesc = idesc_bf16(pr.nt, GEOM == GEOM_MN);
                 const uint32_t b_bytes = (uint32_t)pr.nt * kBK * 2;   // one part of one sub-block of B
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[ab], cph ^ 1, abort_flag, P.wait_ns))) break;
@@ -391,7 +407,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint64_t db = db0 + ((uint64_t)(bs * P.bslot) >> 4);
 #pragma unroll
                     for (int sub = 0; sub < kSub; ++sub) {
-                        if (sub > 0 && st * kSub + sub >= pr.kchunks) break;   // zeros past n_q
+                        if (sub > 0 && st * kSub + sub >= kch) break;   // zeros past n_q
                         const uint64_t dahi = da + (uint64_t)((sub * LA.asub_bytes) >> 4);
                         const uint64_t dalo = dahi + (uint64_t)(LA.abf_bytes >> 4);
                         const uint64_t dbhi = db + (uint64_t)((sub * 2 * b_bytes) >> 4);
@@ -471,8 +487,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 fkb = pr.fold_kb;
                 fsh = pr.fold_ib_shift;
                 const int64_t mper = (ginner + kBM - 1) / kBM;
-                mt = lt % pr.tiles_m;
-                tk = GEOM == GEOM_MN ? mt / mper : 0;
+                const int64_t tm = pr.tiles_m;
+                mt = lt - slice_of(lt, tm) * tm;
+                tk = GEOM == GEOM_MN ? slice_of(mt, mper) : 0;
                 r0 = GEOM == GEOM_MN ? (mt - tk * mper) * kBM : mt * kBM;
             }
             for (int st = 0; st < kst; ++st) {
@@ -570,14 +587,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int64_t mper = (pr.inner + kBM - 1) / kBM;
             if (!mbar_wait(&acc_full[ab], aph, abort_flag, P.wait_ns)) break;
             tc_fence_after();
-            const int64_t jb = lt / pr.tiles_m, mt = lt - jb * pr.tiles_m;
+            const int64_t tm = pr.tiles_m, jb = slice_of(lt, tm), mt = lt - jb * tm;
             int64_t k, r0;            // slice and first row (i for GEOM_MN, k for GEOM_K) of this warp
             if (GEOM == GEOM_MN && pr.fold_kb > 1) {
                 // this warp's 32 rows lie in one slice of the folded tile
                 k = mt * pr.fold_kb + ((q4 * 32) >> pr.fold_ib_shift);
                 r0 = (q4 * 32) & ((1 << pr.fold_ib_shift) - 1);
             } else if (GEOM == GEOM_MN) {
-                k = mt / mper;
+                k = slice_of(mt, mper);
                 r0 = (mt - k * mper) * kBM + q4 * 32;
             } else {
                 k = 0;

@@ -12,7 +12,8 @@
 //   GEOM_K  (inner == 1, the contraction mode is the fastest): MMA rows are
 //            128 consecutive k; A's tile is K-major; TMA box (32 l, 128 k).
 // MMA shape M = 128, N = NT (<= 256, the rows of B in this tile), K = 16 per
-// instruction, 32 l (two sub-blocks of 16, six MMAs) per pipeline stage.
+// instruction, 32 l (two sub-blocks of 16, six MMAs) of one M tile (N > 128) or two
+// per pipeline stage.
 //
 // Warp roles (736 threads, one CTA per SM, persistent over tiles):
 //   warp 0     TMA producer of the FP32 A tile (tensor map).
@@ -49,7 +50,8 @@ constexpr int kGroupWarps = kConvWarps / kConvGroups;
 constexpr int kThreads = (3 + kConvWarps + 4) * 32;  // A producer, MMA, B producer, converters, 4 epilogue warps
 constexpr int kBM = 128;       // MMA M
 constexpr int kBK = 16;        // l per sub-block (one MMA K step)
-constexpr int kSub = 2;        // sub-blocks per pipeline stage: 3 * kSub MMAs per barrier round
+constexpr int kSub = 2;        // sub-blocks of 16 l per pipeline stage
+constexpr int kPairNT = 128;   // widest N whose tiles go through the pipeline in pairs
 constexpr int kMaxNT = 256;    // MMA N max
 
 enum { GEOM_MN = 0, GEOM_K = 1 };
@@ -96,7 +98,8 @@ struct alignas(64) TcProb {
     const uint8_t* bimg;     // pre-split B: [jb][kc][hi|lo][NT rows x 32 B]
     int64_t outer, nq, inner, m;
     int64_t tiles_m;         // M tiles per j block
-    int64_t tiles;           // tiles of this problem
+    int64_t tiles;           // pipeline tiles of this problem: pairs of M tiles first, then single ones
+    int64_t pairs;           // how many are pairs (of one j block: only where jblocks == 1)
     int64_t first;           // grouped launch: index of its first tile among all problems' tiles
     int nt;                  // MMA N (multiple of 16, <= 256)
     int jblocks;
@@ -118,23 +121,24 @@ struct TcParams {
     int fstages;             // A ring depth (FP32 tile, converted in place)
     int ostages;             // B ring depth
     uint32_t bslot;          // bytes of one B ring slot (the largest B stage of the launch)
-    int acc_stride;          // tensor-memory columns between the two accumulators
+    int acc_stride;          // tensor-memory columns between accumulators (a tile of more columns,
+                             // never one of a pair, extends over its absent neighbour's)
     int skip_b;              // test of the bounded waits: the B producer skips its first stage
     unsigned long long wait_ns;   // bound of the pipeline's mbarrier waits
 };
 
-// Shared memory: [A ring][B ring][epilogue staging][barriers]. An A stage holds kSub FP32
-// sub-blocks of 128 rows x 16 l, each converted in place to [bf16 hi | bf16 lo]; a B stage holds
-// [hi | lo] of each sub-block's 16 l of B.
+// Shared memory: [A ring][B ring][epilogue staging][barriers]. An A stage holds H * kSub FP32
+// sub-blocks of 128 rows x 16 l (H M tiles, kSub sub-blocks of each), each converted in place to
+// [bf16 hi | bf16 lo]; a B stage holds [hi | lo] of each sub-block's 16 l of B.
 struct SmemLayout {
     uint32_t a_bytes, asub_bytes, abf_bytes, b_bytes, bstage_bytes;
 };
 
-__host__ __device__ inline SmemLayout smem_layout(int nt)
+__host__ __device__ inline SmemLayout smem_layout(int nt, int h)
 {
     SmemLayout L;
     L.asub_bytes = kBM * kBK * 4;           // 8 KB FP32 sub-block (its bf16 hi and lo halves after conversion)
-    L.a_bytes = kSub * L.asub_bytes;
+    L.a_bytes = h * kSub * L.asub_bytes;
     L.abf_bytes = kBM * kBK * 2;            // 4 KB per bf16 part
     L.b_bytes = (uint32_t)nt * kBK * 2;     // per part and sub-block, multiple of 512
     L.bstage_bytes = kSub * 2 * L.b_bytes;
@@ -147,30 +151,31 @@ constexpr uint32_t kEpiBytes = 4 * 2 * kEpiBuf;  // 4 epilogue warps, double-buf
 constexpr size_t kCtrlBytes = 1024;
 constexpr size_t kSmemBudget = 227 * 1024;
 
+// Converter groups that share a stage.
+__host__ __device__ constexpr int conv_units(int h) { return h == 2 ? kConvGroups : 1; }
+static_assert(kConvGroups == 2 * kSub, "with pairs of M tiles every sub-block of a stage has one group");
+
 // Ring depths for a given N tile; false if the minimum does not fit.
-__host__ inline bool choose_stages(int nt, int& as, int& bs, size_t& smem)
+__host__ inline bool choose_stages(int nt, int h, int& as, int& bs, size_t& smem)
 {
-    const SmemLayout L = smem_layout(nt);
+    const SmemLayout L = smem_layout(nt, h);
     const size_t avail = kSmemBudget - 1024 - kCtrlBytes - kEpiBytes;
-    // A stages: a multiple of kConvGroups. Group g converts the stages n = g (mod kConvGroups) in
-    // order, waiting on each stage's barrier by phase parity; with the ring a multiple of the
-    // groups every slot belongs to one group, which sees each phase of it in turn. Otherwise a
-    // group could wait on a slot whose previous load (another group's) has not landed yet -- loads
-    // may land out of order -- and the parity of that pending phase would read as the completed
-    // one before it.
-    // B stages (from L2) give way first, down to two, so that A keeps two stages per group
-    // (measured at N = 256: 8 A + 2 B stages beat 4 + 3 by 10 %)
+    // A stages: a multiple of the converters' rotation (see there): a slot's phases then all belong
+    // to the same groups, which see each of them in turn. Otherwise a group could wait on a slot
+    // whose previous load (another group's) has not landed yet -- loads may land out of order --
+    // and the parity of that pending phase would read as the completed one before it.
+    // B stages (from L2) give way first, down to two (measured at N = 256: 8 A + 2 B stages beat
+    // 4 + 3 by 10 %)
+    const int rot = kConvGroups / conv_units(h), amin = h == 2 ? 4 : 2 * kConvGroups;
     bs = kMaxB;
-    while (bs > 2 && (size_t)bs * L.bstage_bytes + 2 * kConvGroups * L.a_bytes > avail) --bs;
-    while (bs > 2 && (size_t)bs * L.bstage_bytes + kConvGroups * L.a_bytes > avail) --bs;
-    if ((size_t)bs * L.bstage_bytes + kConvGroups * L.a_bytes > avail) return false;
+    while (bs > 2 && (size_t)bs * L.bstage_bytes + amin * L.a_bytes > avail) --bs;
+    if ((size_t)bs * L.bstage_bytes + rot * L.a_bytes > avail) return false;
     as = (int)((avail - (size_t)bs * L.bstage_bytes) / L.a_bytes);
     if (as > kMaxA) as = kMaxA;
-    as -= as % kConvGroups;
+    as -= as % rot;
     smem = 1024 + (size_t)as * L.a_bytes + (size_t)bs * L.bstage_bytes + kEpiBytes + kCtrlBytes;
     return true;
 }
-
 
 // Named barrier of one converter group (ids 1..kConvGroups; id 0 is __syncthreads).
 __device__ __forceinline__ void conv_barrier(int g)
@@ -195,6 +200,20 @@ __device__ __forceinline__ const TcProb& tile_problem(const TcProb& one, const T
     }
 }
 
+// First M tile (numbered within the problem, j blocks outermost) of pipeline tile lt, and how many
+// it has.
+template <int H>
+__device__ __forceinline__ int64_t first_m_tile(int64_t lt, int64_t pairs, int& nh)
+{
+    if constexpr (H == 2) {
+        nh = lt < pairs ? 2 : 1;
+        return lt < pairs ? 2 * lt : lt + pairs;
+    } else {
+        nh = 1;
+        return lt;
+    }
+}
+
 // A tensor map in device memory is read through the tensor-map proxy: order that read after the
 // generic-proxy writes that made the map (the plan's upload) before the first copy using it.
 __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map)
@@ -205,13 +224,19 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map)
 // GROUP = false: one problem, `one`. GROUP = true: the P.count problems of P.group, whose tiles
 // are numbered one after the other; every role walks the same tile sequence, so the pipeline
 // runs across problem boundaries without draining.
-template <int GEOM, bool GROUP>
+// H: M tiles that go through the pipeline together (2 for N <= kPairNT). They share each stage's B,
+// and the MMA issuer's barriers and commits, about 390 cycles a stage whatever it multiplies, are
+// paid once for 12 MMAs instead of 6 (with one tile at a time the issuer was busy 700 of 920 cycles
+// a stage). Measured, one tile at a time -> pairs: A 192^4, slowest mode, m = 32 1184 -> 1045 us
+// (0.93 of the copy bandwidth), contiguous fibres 1170 -> 973 us; (300, 420, 500), m = 96 98 -> 89 us.
+// Wider tiles go one at a time: tensor memory holds two of 256 columns.
+template <int GEOM, bool GROUP, int H>
 __global__ void __launch_bounds__(kThreads, 1)
     tc_bf16x3_kernel(const __grid_constant__ TcProb one, TcParams P)
 {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const SmemLayout LA = smem_layout(kMaxNT);   // its A sizes do not depend on N
+    const SmemLayout LA = smem_layout(kMaxNT, H);   // its A sizes do not depend on N
     const int AS = P.fstages, BS = P.ostages;
     uint8_t* aring = smem;
     uint8_t* bring = smem + (size_t)AS * LA.a_bytes;
@@ -235,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (threadIdx.x == 0) {
         for (int s = 0; s < AS; ++s) {
             mbar_init(&a_full[s], 1);
-            mbar_init(&a_conv[s], kGroupWarps);
+            mbar_init(&a_conv[s], conv_units(H) * kGroupWarps);
             mbar_init(&a_empty[s], 1);
         }
         for (int s = 0; s < BS; ++s) {
@@ -283,18 +308,24 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const CUtensorMap* const amap = &pr.amap;
                 if (GROUP && &pr != last && !ldg) tensormap_acquire(amap);
                 last = &pr;
-                const int64_t tm = pr.tiles_m, mt = lt - slice_of(lt, tm) * tm;
-                int c0, ck = 0;   // first row (i, or the fibre for GEOM_K) and slice of the tile
-                if (GEOM == GEOM_MN && fold > 1) {
-                    // folded tile: slices mt*KB .. +KB-1, the map ordered (i, k, l)
-                    c0 = 0;
-                    ck = (int)(mt * fold);
-                } else if (GEOM == GEOM_MN) {
-                    const int64_t mper = (pr.inner + kBM - 1) / kBM, k = slice_of(mt, mper);
-                    c0 = (int)((mt - k * mper) * kBM);
-                    ck = (int)k;
-                } else {
-                    c0 = (int)(mt * kBM);
+                int nh;
+                const int64_t tm = pr.tiles_m, sub0 = first_m_tile<H>(lt, pr.pairs, nh), mt = sub0 - slice_of(sub0, tm) * tm;
+                int c0[H], ck[H];   // per M tile: its first row (i, or the fibre for GEOM_K) and slice
+                const int64_t mper = (pr.inner + kBM - 1) / kBM;
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    ck[h] = 0;
+                    if (GEOM == GEOM_MN && fold > 1) {
+                        // folded tile: slices mt*KB .. +KB-1, the map ordered (i, k, l)
+                        c0[h] = 0;
+                        ck[h] = (int)((mt + h) * fold);
+                    } else if (GEOM == GEOM_MN) {
+                        const int64_t k = slice_of(mt + h, mper);
+                        c0[h] = (int)((mt + h - k * mper) * kBM);
+                        ck[h] = (int)k;
+                    } else {
+                        c0[h] = (int)((mt + h) * kBM);
+                    }
                 }
                 for (int st = 0; st < kst; ++st) {
                     if (!mbar_wait(&a_empty[s], ph ^ 1, abort_flag, P.wait_ns)) { ok = false; break; }
@@ -312,19 +343,21 @@ __global__ void __launch_bounds__(kThreads, 1)
                     phases = (phases & ~(1u << s)) | (ph << s);
                     // the sub-blocks within n_q (the last box's rows past n_q are zero-filled)
                     const int nsub = min(kSub, kch - st * kSub);
-                    mbar_expect_tx(&a_full[s], (uint32_t)nsub * LA.asub_bytes);
+                    mbar_expect_tx(&a_full[s], (uint32_t)(nh * nsub) * LA.asub_bytes);
 #pragma unroll
-                    for (int sub = 0; sub < kSub; ++sub) {
-                        if (sub >= nsub) break;
-                        uint8_t* dst = a_at(s) + sub * LA.asub_bytes;
-                        const int l0 = (st * kSub + sub) * kBK;
-                        if (GEOM == GEOM_MN) {
-                            if (fold > 1) tma_load_3d(dst, amap, &a_full[s], 0, ck, l0);
-                            else tma_load_3d(dst, amap, &a_full[s], c0, l0, ck);
-                        } else {
-                            tma_load_2d(dst, amap, &a_full[s], l0, c0);
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int sub = 0; sub < kSub; ++sub) {
+                            if (h >= nh || sub >= nsub) break;
+                            uint8_t* dst = a_at(s) + (h * kSub + sub) * LA.asub_bytes;
+                            const int l0 = (st * kSub + sub) * kBK;
+                            if (GEOM == GEOM_MN) {
+                                if (fold > 1) tma_load_3d(dst, amap, &a_full[s], 0, ck[h], l0);
+                                else tma_load_3d(dst, amap, &a_full[s], c0[h], l0, ck[h]);
+                            } else {
+                                tma_load_2d(dst, amap, &a_full[s], l0, c0[h]);
+                            }
                         }
-                    }
                     if (++s == AS) { s = 0; ph ^= 1; }
                 }
             }
@@ -347,9 +380,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 int64_t lt;
                 const TcProb& pr = tile_problem<GROUP>(one, P, t, cur, lt);
                 const int kst = pr.kstages;
-                const uint32_t bytes = smem_layout(pr.nt).bstage_bytes;
+                const uint32_t bytes = smem_layout(pr.nt, H).bstage_bytes;
+                int nh;
+                const int64_t jb = slice_of(first_m_tile<H>(lt, pr.pairs, nh), pr.tiles_m);
                 // the image holds kstages * kSub sub-blocks per j block: one copy per stage
-                const uint8_t* img = pr.bimg + (size_t)(slice_of(lt, pr.tiles_m) * kst) * bytes;
+                const uint8_t* img = pr.bimg + (size_t)(jb * kst) * bytes;
                 for (int st = 0; st < kst; ++st, img += bytes) {
                     if (!mbar_wait(&b_empty[s], ph ^ 1, abort_flag, P.wait_ns)) { ok = false; break; }
                     if (P.skip_b && t == blockIdx.x && st == 0) {
@@ -394,7 +429,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const uint32_t b_bytes = (uint32_t)pr.nt * kBK * 2;   // one part of one sub-block of B
                 if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[ab], cph ^ 1, abort_flag, P.wait_ns))) break;
                 tc_fence_after();
-                const uint32_t dcol = tmem_base + (uint32_t)(ab * P.acc_stride);
+                int nh;
+                first_m_tile<H>(lt, pr.pairs, nh);
+                const uint32_t dcol = tmem_base + (uint32_t)(ab * H * P.acc_stride);
                 for (int st = 0; st < kst; ++st) {
                     const bool got = mbar_wait(&b_full[bs], bph, abort_flag, P.wait_ns) &&
                                      mbar_wait(&a_conv[as], aph, abort_flag, P.wait_ns);
@@ -406,16 +443,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint64_t da = da0 + ((uint64_t)(as * LA.a_bytes) >> 4);
                     const uint64_t db = db0 + ((uint64_t)(bs * P.bslot) >> 4);
 #pragma unroll
-                    for (int sub = 0; sub < kSub; ++sub) {
-                        if (sub > 0 && st * kSub + sub >= kch) break;   // zeros past n_q
-                        const uint64_t dahi = da + (uint64_t)((sub * LA.asub_bytes) >> 4);
-                        const uint64_t dalo = dahi + (uint64_t)(LA.abf_bytes >> 4);
-                        const uint64_t dbhi = db + (uint64_t)((sub * 2 * b_bytes) >> 4);
-                        const uint64_t dblo = dbhi + (uint64_t)(b_bytes >> 4);
-                        mma_bf16(dcol, dahi, dbhi, idesc, (st == 0 && sub == 0) ? 0u : 1u);
-                        mma_bf16(dcol, dahi, dblo, idesc, 1u);
-                        mma_bf16(dcol, dalo, dbhi, idesc, 1u);
-                    }
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int sub = 0; sub < kSub; ++sub) {
+                            // absent M tile, or zeros past n_q
+                            if (h >= nh || (sub > 0 && st * kSub + sub >= kch)) break;
+                            const uint32_t dst = dcol + (uint32_t)(h * P.acc_stride);
+                            const uint64_t dahi = da + (uint64_t)(((h * kSub + sub) * LA.asub_bytes) >> 4);
+                            const uint64_t dalo = dahi + (uint64_t)(LA.abf_bytes >> 4);
+                            const uint64_t dbhi = db + (uint64_t)((sub * 2 * b_bytes) >> 4);
+                            const uint64_t dblo = dbhi + (uint64_t)(b_bytes >> 4);
+                            mma_bf16(dst, dahi, dbhi, idesc, (st == 0 && sub == 0) ? 0u : 1u);
+                            mma_bf16(dst, dahi, dblo, idesc, 1u);
+                            mma_bf16(dst, dalo, dbhi, idesc, 1u);
+                        }
                     mma_commit_warp(&a_empty[as]);   // stages free once these MMAs have read them
                     mma_commit_warp(&b_empty[bs]);
                     if (++as == AS) { as = 0; aph ^= 1; }
@@ -433,10 +474,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
     } else if (warp < 3 + kConvWarps) {
         // ------------------------------------------------------------- converters (in place)
-        // kConvGroups groups of kGroupWarps warps; group g converts the stages with sequence number
-        // n, n % kConvGroups == g (their kSub sub-blocks one after the other), so that several
-        // stages are converted at once.
+        // kConvGroups groups of kGroupWarps warps. Pairs of M tiles (H = 2): group g converts
+        // sub-block g of every stage. Single ones: group g converts the whole stages with sequence
+        // number n, n % kConvGroups == g, one sub-block after the other.
+        constexpr int kUnits = conv_units(H), kRot = kConvGroups / kUnits, kPer = H * kSub / kUnits;
         const int g = (warp - 3) / kGroupWarps;
+        const int unit = g % kUnits * kPer, uh = unit / kSub;   // the group's first sub-block, its M tile
         const int gt = threadIdx.x - 96 - g * kGroupWarps * 32;   // 0 .. kGroupWarps*32-1
         const bool odd = lane & 1;
         constexpr int kIters = (kBM * kBK / 4) / (kGroupWarps * 32);
@@ -458,10 +501,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         bool ok = true;
         // The CTA's stages are numbered n = 0, 1, ... across its tiles; this group takes those with
-        // n % kConvGroups == g, which sit in ring slot n % AS with phase (n / AS) & 1. AS being a
-        // multiple of kConvGroups, the group's slot steps by kConvGroups and wraps with a phase flip.
-        int rot = 0;                 // n % kConvGroups
-        int s = g;                   // slot of the group's next stage
+        // n % kRot == g / kUnits, which sit in ring slot n % AS with phase (n / AS) & 1. AS being a
+        // multiple of kRot, the group's slot steps by kRot and wraps with a phase flip.
+        int rot = 0;                 // n % kRot
+        int s = g / kUnits;          // slot of the group's next stage
         uint32_t ph = 0;
         // Every thread of a group runs every iteration of its residue and reaches the group barrier
         // the same number of times; once the CTA aborts, the waits are skipped and no work is done.
@@ -474,6 +517,8 @@ __global__ void __launch_bounds__(kThreads, 1)
             // converters' own loads only where they load A
             const int kst = pr.kstages, kch = pr.kchunks;
             const bool ldg = pr.ldg_a != 0;
+            int nh;
+            const int64_t sub0 = first_m_tile<H>(lt, pr.pairs, nh);
             const float* ga = nullptr;
             int64_t gnq = 0, ginner = 0, gouter = 0;
             int fkb = 1, fsh = 0;
@@ -488,23 +533,24 @@ __global__ void __launch_bounds__(kThreads, 1)
                 fsh = pr.fold_ib_shift;
                 const int64_t mper = (ginner + kBM - 1) / kBM;
                 const int64_t tm = pr.tiles_m;
-                mt = lt - slice_of(lt, tm) * tm;
+                mt = sub0 - slice_of(sub0, tm) * tm + uh;
                 tk = GEOM == GEOM_MN ? slice_of(mt, mper) : 0;
                 r0 = GEOM == GEOM_MN ? (mt - tk * mper) * kBM : mt * kBM;
             }
             for (int st = 0; st < kst; ++st) {
-                const bool mine = rot == g;
-                if (++rot == kConvGroups) rot = 0;
+                const bool mine = rot == g / kUnits;
+                if (++rot == kRot) rot = 0;
                 if (!mine) continue;
                 const bool got = ok && mbar_wait(&a_full[s], ph, abort_flag, P.wait_ns);
                 const bool have = __all_sync(0xffffffffu, got);
                 if (!have) ok = false;
-                // sub-blocks past n_q are zeros that the MMA issuer skips: not converted
-                const int nsub = min(kSub, kch - st * kSub);
+                // sub-blocks past n_q are zeros that the MMA issuer skips: not converted, like those
+                // of an absent M tile
 #pragma unroll 1
-                for (int sub = 0; sub < nsub; ++sub) {
-                    const int kc = st * kSub + sub;
-                    uint8_t* buf = a_at(s) + sub * LA.asub_bytes;
+                for (int u = 0; u < kPer; ++u) {
+                    const int kc = st * kSub + (unit + u) % kSub;
+                    if (uh >= nh || kc >= kch) break;
+                    uint8_t* buf = a_at(s) + (unit + u) * LA.asub_bytes;
                     float4 x[kIters];
                     uint32_t off[kIters];
 #pragma unroll
@@ -565,7 +611,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&a_conv[s]);
                 }
-                s += kConvGroups;
+                s += kRot;
                 if (s >= AS) { s -= AS; ph ^= 1; }
             }
         }
@@ -587,12 +633,25 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int64_t mper = (pr.inner + kBM - 1) / kBM;
             if (!mbar_wait(&acc_full[ab], aph, abort_flag, P.wait_ns)) break;
             tc_fence_after();
-            const int64_t tm = pr.tiles_m, jb = slice_of(lt, tm), mt = lt - jb * tm;
+            const int nt = pr.nt;
+            // the record's fields the stores use, in registers: a grouped launch's records sit in
+            // global memory, where every store to C could alias them and force a reload
+            const int64_t e_inner = pr.inner, e_outer = pr.outer, e_m = pr.m;
+            float* const e_c = pr.c;
+            const bool e_tma = pr.tma_c != 0;
+            const int e_fold = pr.fold_kb, e_shift = pr.fold_ib_shift;
+            int nh;
+            const int64_t tm = pr.tiles_m, sub0 = first_m_tile<H>(lt, pr.pairs, nh), jb = slice_of(sub0, tm);
+            const int64_t jrem = e_m - jb * nt;
+            const int jleft = jrem < nt ? (int)jrem : nt;
+#pragma unroll 1
+            for (int h = 0; h < nh; ++h) {
+            const int64_t mt = sub0 + h - jb * tm;
             int64_t k, r0;            // slice and first row (i for GEOM_MN, k for GEOM_K) of this warp
-            if (GEOM == GEOM_MN && pr.fold_kb > 1) {
+            if (GEOM == GEOM_MN && e_fold > 1) {
                 // this warp's 32 rows lie in one slice of the folded tile
-                k = mt * pr.fold_kb + ((q4 * 32) >> pr.fold_ib_shift);
-                r0 = (q4 * 32) & ((1 << pr.fold_ib_shift) - 1);
+                k = mt * e_fold + ((q4 * 32) >> e_shift);
+                r0 = (q4 * 32) & ((1 << e_shift) - 1);
             } else if (GEOM == GEOM_MN) {
                 k = slice_of(mt, mper);
                 r0 = (mt - k * mper) * kBM + q4 * 32;
@@ -600,20 +659,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                 k = 0;
                 r0 = mt * kBM + q4 * 32;
             }
-            const int nt = pr.nt;
-            // the record's fields the stores use, in registers: a grouped launch's records sit in
-            // global memory, where every store to C could alias them and force a reload
-            const int64_t e_inner = pr.inner, e_outer = pr.outer, e_m = pr.m;
-            float* const e_c = pr.c;
-            const bool e_tma = pr.tma_c != 0;
-            const int64_t jrem = e_m - (int64_t)jb * nt;
-            const int jleft = jrem < nt ? (int)jrem : nt;
-            const uint32_t tbase = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(ab * P.acc_stride);
+            const uint32_t tbase =
+                tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)((ab * H + h) * P.acc_stride);
             for (int cc = 0; cc < nt; cc += 32) {
                 uint32_t v[32];
                 tmem_ld32(tbase + (uint32_t)cc, v);
                 if (cc >= jleft) continue;
-                const int j0 = jb * nt + cc;
+                const int j0 = (int)(jb * nt) + cc;
                 if (e_tma && GEOM == GEOM_MN && k >= e_outer) {
                     // folded last tile: this warp's slice lies past the end of C, nothing to store
                 } else if (e_tma) {
@@ -671,6 +723,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int row = 0; row < nrow; ++row) cb[(int64_t)row * e_m] = b32[row * 32 + (lane ^ row)];
                     __syncwarp();
                 }
+            }
             }
             tc_fence_before();
             __syncwarp();
@@ -1347,21 +1400,42 @@ void make_tc_prob(const View3& v, uint8_t* img, TcProb& pr, int* geom)
     pr.tiles_m = g == GEOM_MN ? (pr.fold_kb > 1 ? (v.outer + pr.fold_kb - 1) / pr.fold_kb
                                                 : v.outer * ((v.inner + kBM - 1) / kBM))
                               : (v.outer + kBM - 1) / kBM;
+    pr.pairs = 0;
     pr.tiles = pr.tiles_m * pr.jblocks;
     pr.first = 0;
+}
+
+// Tiles of at most kPairNT columns go through the pipeline in pairs (H = 2).
+int tiles_at_once(const TcProb& pr) { return pr.nt <= kPairNT && !pr.ldg_a ? 2 : 1; }
+
+// Numbers a problem's M tiles as `pairs` pairs and the rest single ones.
+void set_pairs(TcProb& pr, int64_t pairs)
+{
+    pr.pairs = pairs;
+    pr.tiles = pr.tiles_m * pr.jblocks - pairs;
 }
 
 // Elements of B's image a problem's operand split writes: kstages * kSub sub-blocks of 16 l per
 // j block (zero past n_q), nt rows each, in two 8-l halves.
 int64_t split_units(const TcProb& pr) { return (int64_t)pr.jblocks * (pr.kstages * kSub) * pr.nt * 2; }
 
-template <int GEOM, bool GROUP>
+template <int GEOM, bool GROUP, int H>
 cudaError_t launch_tc_kernel(const TcProb& one, const TcParams& P, size_t smem, int grid, cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(tc_bf16x3_kernel<GEOM, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e == cudaSuccess) tc_bf16x3_kernel<GEOM, GROUP><<<grid, kThreads, smem, s>>>(one, P);
+    const auto kernel = tc_bf16x3_kernel<GEOM, GROUP, H>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) kernel<<<grid, kThreads, smem, s>>>(one, P);
     return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+template <bool GROUP>
+cudaError_t launch_tc_any(int geom, int h, const TcProb& one, const TcParams& P, size_t smem, int grid, cudaStream_t s)
+{
+    if (geom == GEOM_MN)
+        return h == 2 ? launch_tc_kernel<GEOM_MN, GROUP, 2>(one, P, smem, grid, s)
+                      : launch_tc_kernel<GEOM_MN, GROUP, 1>(one, P, smem, grid, s);
+    return h == 2 ? launch_tc_kernel<GEOM_K, GROUP, 2>(one, P, smem, grid, s)
+                  : launch_tc_kernel<GEOM_K, GROUP, 1>(one, P, smem, grid, s);
 }
 
 // Splits B into `img` (tc_image_bytes(v) bytes) and launches the bf16x3 kernel for v on stream s.
@@ -1370,17 +1444,24 @@ cudaError_t run_bf16x3(const View3& v, uint8_t* img, int* status, int sms, cudaS
     TcProb pr;
     int geom = GEOM_MN;
     make_tc_prob(v, img, pr, &geom);
+    const int h = tiles_at_once(pr);
+    if (h == 2) {
+        // A block's share is at most c tiles. c even: all in pairs; odd: (c - 1) / 2 pairs for each
+        // block and the rest single, at most one per block.
+        const int64_t c = ceil_div(pr.tiles, sms);
+        set_pairs(pr, c % 2 == 0 ? pr.tiles / 2 : std::min<int64_t>(pr.tiles / 2, c / 2 * sms));
+    }
     TcParams P{};
     P.status = status;
     P.group = nullptr;
     P.count = 1;
     P.total = pr.tiles;
-    P.bslot = smem_layout(pr.nt).bstage_bytes;
+    P.bslot = smem_layout(pr.nt, h).bstage_bytes;
     P.acc_stride = pr.nt;
     P.wait_ns = wait_limit_ns();
     P.skip_b = take_skip_b() ? 1 : 0;
     size_t smem = 0;
-    if (!choose_stages(pr.nt, P.fstages, P.ostages, smem)) return cudaErrorNotSupported;
+    if (!choose_stages(pr.nt, h, P.fstages, P.ostages, smem)) return cudaErrorNotSupported;
 
     const int64_t total = split_units(pr);
     const int blocks = (int)std::min<int64_t>((total + 255) / 256, 4096);
@@ -1388,22 +1469,22 @@ cudaError_t run_bf16x3(const View3& v, uint8_t* img, int* status, int sms, cudaS
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int grid = (int)std::min<int64_t>(pr.tiles, sms);
-    return geom == GEOM_MN ? launch_tc_kernel<GEOM_MN, false>(pr, P, smem, grid, s)
-                           : launch_tc_kernel<GEOM_K, false>(pr, P, smem, grid, s);
+    return launch_tc_any<false>(geom, h, pr, P, smem, grid, s);
 }
 
 }  // namespace
 
 // ------------------------------------------------------------------ grouped bf16x3 launch
 struct TcGroup {
-    TcProb* d_probs = nullptr;    // device records: the GEOM_MN problems, then the GEOM_K ones
+    TcProb* d_probs = nullptr;    // device records, one class after the other
     uint8_t* d_img = nullptr;     // all pre-split B images
     int* status = nullptr;
     int count = 0;
     int split_x = 1;              // blocks per problem of the operand split
-    TcParams P[2] = {};           // per geometry (count 0: none)
-    size_t smem[2] = {0, 0};
-    int grid[2] = {0, 0};
+    // launches by class: geometry (GEOM_MN, GEOM_K) x tiles at once (2, 1); count 0: none
+    TcParams P[4] = {};
+    size_t smem[4] = {};
+    int grid[4] = {};
 };
 
 namespace {
@@ -1435,10 +1516,24 @@ cudaError_t tc_group_create(const View3* views, int count, TcGroup** out)
     }
     if ((e = dev_malloc(reinterpret_cast<void**>(&G->d_img), img_total)) != cudaSuccess) return e;
     std::vector<TcProb> probs(count);
-    std::vector<int> geom(count);
-    for (int i = 0; i < count; ++i) make_tc_prob(views[i], G->d_img + img_off[i], probs[i], &geom[i]);
-    // GEOM_MN first, then GEOM_K; within each, the problems with the heaviest tiles first, so
-    // that the round robin of tiles over the persistent CTAs ends on light ones
+    std::vector<int> geom(count);   // geometry, then class
+    int64_t ctiles[4] = {};
+    for (int i = 0; i < count; ++i) {
+        make_tc_prob(views[i], G->d_img + img_off[i], probs[i], &geom[i]);
+        geom[i] = geom[i] * 2 + (2 - tiles_at_once(probs[i]));   // the class
+        ctiles[geom[i]] += probs[i].tiles;
+    }
+    // A class of few tiles joins the other class of its geometry: another launch costs more than
+    // the narrow tiles going one at a time, or the wide ones through the pairs' shorter ring.
+    const int64_t few = 4 * (int64_t)sms;
+    for (int i = 0; i < count; ++i) {
+        const int pair = geom[i] & ~1, one = geom[i] | 1;
+        if (ctiles[one] && ctiles[pair] && (ctiles[one] < few || ctiles[pair] < few))
+            geom[i] = ctiles[pair] < few ? one : pair;
+        if (geom[i] == pair && tiles_at_once(probs[i]) == 2) set_pairs(probs[i], probs[i].tiles / 2);
+    }
+    // class by class; within each, the problems with the heaviest tiles first, so that the round
+    // robin of tiles over the persistent CTAs ends on light ones
     std::vector<int> order(count);
     for (int i = 0; i < count; ++i) order[i] = i;
     auto tile_cost = [&](int i) { return (int64_t)probs[i].kstages * probs[i].nt; };
@@ -1447,8 +1542,8 @@ cudaError_t tc_group_create(const View3* views, int count, TcGroup** out)
         return tile_cost(x) > tile_cost(y);
     });
     std::vector<TcProb> sorted(count);
-    int64_t first[2] = {0, 0};
-    int ntmax[2] = {16, 16}, n[2] = {0, 0};
+    int64_t first[4] = {};
+    int ntmax[4] = {16, 16, 16, 16}, n[4] = {};
     int64_t max_units = 0;
     for (int r = 0; r < count; ++r) {
         const int i = order[r], g = geom[i];
@@ -1463,17 +1558,19 @@ cudaError_t tc_group_create(const View3* views, int count, TcGroup** out)
     if ((e = cudaMemcpy(G->d_probs, sorted.data(), sizeof(TcProb) * count, cudaMemcpyHostToDevice)) != cudaSuccess)
         return e;
     G->split_x = (int)std::max<int64_t>(1, std::min<int64_t>((max_units + 255) / 256, 64));
-    for (int g = 0; g < 2; ++g) {
+    const TcProb* at = G->d_probs;
+    for (int g = 0; g < 4; at += n[g++]) {
         TcParams& P = G->P[g];
         P = TcParams{};
         P.count = n[g];
         if (n[g] == 0) continue;
+        const int h = 2 - g % 2;
         P.status = G->status;
-        P.group = G->d_probs + (g == 0 ? 0 : n[0]);
+        P.group = at;
         P.total = first[g];
-        P.bslot = smem_layout(ntmax[g]).bstage_bytes;
-        P.acc_stride = ntmax[g];
-        if (!choose_stages(ntmax[g], P.fstages, P.ostages, G->smem[g])) return cudaErrorNotSupported;
+        P.bslot = smem_layout(ntmax[g], h).bstage_bytes;
+        P.acc_stride = h == 2 ? std::min(ntmax[g], kPairNT) : ntmax[g];
+        if (!choose_stages(ntmax[g], h, P.fstages, P.ostages, G->smem[g])) return cudaErrorNotSupported;
         G->grid[g] = (int)std::min<int64_t>(P.total, sms);
     }
     *out = G.release();
@@ -1489,13 +1586,12 @@ cudaError_t tc_group_run(TcGroup* G, cudaStream_t s)
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    for (int g = 0; g < 2; ++g) {
+    for (int g = 0; g < 4; ++g) {
         TcParams P = G->P[g];
         if (P.count == 0) continue;
         P.wait_ns = wait_limit_ns();
         P.skip_b = take_skip_b() ? 1 : 0;
-        cudaError_t e = g == 0 ? launch_tc_kernel<GEOM_MN, true>(g_no_prob, P, G->smem[g], G->grid[g], s)
-                               : launch_tc_kernel<GEOM_K, true>(g_no_prob, P, G->smem[g], G->grid[g], s);
+        cudaError_t e = launch_tc_any<true>(g / 2, 2 - g % 2, g_no_prob, P, G->smem[g], G->grid[g], s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1504,7 +1600,9 @@ cudaError_t tc_group_run(TcGroup* G, cudaStream_t s)
 int tc_group_launches(const TcGroup* G)
 {
     if (!G || G->count == 0) return 0;
-    return (G->count + 65534) / 65535 + (G->P[0].count > 0) + (G->P[1].count > 0);
+    int n = (G->count + 65534) / 65535;
+    for (const TcParams& P : G->P) n += P.count > 0;
+    return n;
 }
 
 void tc_group_destroy(TcGroup* G)
@@ -2127,7 +2225,7 @@ size_t tc_image_bytes(const View3& v)
     const int nt = (int)std::min<int64_t>(kMaxNT, ((v.m + 15) / 16) * 16);
     const int64_t jblocks = (v.m + nt - 1) / nt;
     const int64_t kpad = (v.nq + kSub * kBK - 1) / (kSub * kBK) * kSub;   // sub-blocks, a whole number of stages
-    return (size_t)(jblocks * kpad * 2) * smem_layout(nt).b_bytes;
+    return (size_t)(jblocks * kpad * 2) * smem_layout(nt, 1).b_bytes;
 }
 
 cudaError_t launch_tc_noalloc(const View3& v, cudaStream_t s, int* kid)

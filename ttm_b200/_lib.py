@@ -85,10 +85,17 @@ def lib():
     return _lib
 
 
+_SZ_ARRAYS = [C.c_size_t * max(n, 1) for n in range(33)]   # orders up to 32
+
+
 def sz(v):
     """A C size_t[] holding the integers of v."""
-    v = [int(x) for x in v]
-    return (C.c_size_t * max(len(v), 1))(*v)
+    n = len(v)
+    arr = _SZ_ARRAYS[n] if n < 33 else C.c_size_t * n
+    try:
+        return arr(*v)
+    except TypeError:   # numpy integers and the like
+        return arr(*[int(x) for x in v])
 
 
 def check(rc: int):
@@ -99,11 +106,10 @@ def check(rc: int):
 def ttm_raw(dtype: int, precision: int, q: int, p: int, a_ptr: int, na, wa, pia, b_ptr: int, nb, pib,
             c_ptr: int, nc, wc, stream: int = 0):
     """One call of tlibttm_ttm_ex with raw addresses (host or device) and host metadata."""
-    L = lib()
-    rc = L.tlibttm_ttm_ex(dtype, precision, q, p, C.c_void_p(a_ptr), sz(na), sz(wa), sz(pia),
-                          C.c_void_p(b_ptr), sz(nb), sz(pib) if pib is not None else None,
-                          C.c_void_p(c_ptr), sz(nc), sz(wc), C.c_void_p(stream))
-    check(rc)
+    rc = (_lib or lib()).tlibttm_ttm_ex(dtype, precision, q, p, a_ptr, sz(na), sz(wa), sz(pia), b_ptr, sz(nb),
+                                        sz(pib) if pib is not None else None, c_ptr, sz(nc), sz(wc), stream)
+    if rc != OK:
+        check(rc)
 
 
 def last_kernel() -> str:

@@ -101,8 +101,7 @@ def _device_view(x):
 def _layout_from_strides(shape, strides):
     """One-based layout pi listing modes from smallest to largest stride (ties: higher mode first)."""
     p = len(shape)
-    order = sorted(range(p), key=lambda r: (strides[r], -r))
-    return [r + 1 for r in order]
+    return [-r for _, r in sorted(zip(strides, range(-1, -p - 1, -1)))]
 
 
 def _dense_strides(shape, pi):
@@ -195,9 +194,8 @@ def _ttm_torch(q, A, B, precision, out=None):
             B = torch.as_tensor(np.asarray(B_in), device=A.device)
     if B.dim() != 2:
         raise ValueError("Error calling ttmpy::ttm: second input should be a mtrix with order equal to 2.")
-    B = B.to(device=A.device, dtype=A.dtype)
-    if any(s < 0 for s in A.stride()):
-        A = A.contiguous()
+    if B.dtype != A.dtype or B.device != A.device:
+        B = B.to(device=A.device, dtype=A.dtype)
     if B.is_contiguous():
         pib = [2, 1]
     elif B.t().is_contiguous():
@@ -233,14 +231,18 @@ def _ttm_torch(q, A, B, precision, out=None):
         return C
     if precision == "tuned":
         precision = "auto" if A.dtype == torch.float32 else "plain"
-    if A.is_cuda:
-        with torch.cuda.device(A.device):
-            _lib.ttm_raw(_dtype_id(A.dtype), _prec(precision), q, p, A.data_ptr(), na, wa, pia,
-                         B.data_ptr(), nb, pib, C.data_ptr(), nc, wc, stream)
-    else:
-        _lib.ttm_raw(_dtype_id(A.dtype), _prec(precision), q, p, A.data_ptr(), na, wa, pia,
-                     B.data_ptr(), nb, pib, C.data_ptr(), nc, wc, 0)
+    _on_device(A, _dtype_id(A.dtype), _prec(precision), q, p, A.data_ptr(), na, wa, pia, B.data_ptr(), nb, pib,
+               C.data_ptr(), nc, wc, stream)
     return C
+
+
+def _on_device(A, *args):
+    """_lib.ttm_raw(*args) with A's device current (host tensors: whichever is)."""
+    if not A.is_cuda or A.get_device() == torch.cuda.current_device():
+        _lib.ttm_raw(*args)
+    else:
+        with torch.cuda.device(A.device):
+            _lib.ttm_raw(*args)
 
 
 def ttm(q, A, B, precision="default", out=None):
@@ -316,11 +318,10 @@ def ttms(q, A, Bs, order="forward", precision="default"):
 
     ``order`` is "forward" (ascending modes), "backward" (descending) or
     "optimal" (ascending 1/n_k - 1/m_k, i.e. the most shrinking factors first).
-    The whole chain runs as one plan (include/tlibttm.h, tlibttm_plan_chain):
-    numpy inputs are moved to the GPU once, intermediates stay in device
-    buffers the plan owns, and only the final tensor returns to the host.
-    Device arrays (torch, CUDA array interface, DLPack) are read in place and
-    the result is a torch CUDA tensor.
+    The products run one after the other on the current torch stream: numpy inputs are moved to
+    the GPU once, intermediates come from torch's caching allocator, and only the final tensor
+    returns to the host. Device arrays (torch, CUDA array interface, DLPack) are read in place and
+    the result is a torch CUDA tensor, complete when the call returns.
     """
     q = int(q)
     dA = _device_view(A)
@@ -335,37 +336,49 @@ def ttms(q, A, Bs, order="forward", precision="default"):
         for r, k in seq:
             c = ttm(r, c, Bs[k], precision)
         return c
-    from .plans import ChainPlan
     host = not _is_torch(A)
     if host:
         A = np.asarray(A)
         if A.dtype not in (np.float32, np.float64):
             A = A.astype(np.float64)
         dev = torch.device("cuda", torch.cuda.current_device())
-        tA = torch.from_numpy(np.ascontiguousarray(A)).to(dev)
+        c = torch.from_numpy(np.ascontiguousarray(A)).to(dev)
     else:
-        tA = A.contiguous()
-        if tA.dtype not in (torch.float32, torch.float64):
-            tA = tA.to(torch.float64)
-        dev = tA.device
-    dt = tA.dtype
+        c = A.contiguous()
+        if c.dtype not in (torch.float32, torch.float64):
+            c = c.to(torch.float64)
+        dev = c.device
+    dt = c.dtype
     # C-ordered tensor: mode r has extent shape[r-1]; layout is last-order (p, ..., 1).
-    na = list(tA.shape)
+    ext = list(c.shape)
     pia = list(range(p, 0, -1))
-    bs = []
-    ext = list(na)
+    steps = []
     for r, k in seq:
         b = Bs[k]
         if int(b.shape[1]) != ext[r - 1]:
             # what tlib::ttm raises for this contraction (include/tlib/ttm.h:80)
             raise RuntimeError("Error in tlib::tensor_times_matrix: contraction dimension of A and B are not equal.")
         b = b.to(device=dev, dtype=dt) if _is_torch(b) else torch.from_numpy(np.asarray(b)).to(device=dev, dtype=dt)
-        bs.append(b.contiguous())
+        steps.append((r, b.contiguous()))
         ext[r - 1] = int(b.shape[0])
-    out = torch.empty(ext, device=dev, dtype=dt)
-    with torch.cuda.device(dev):
-        plan = ChainPlan(tA.reshape(-1), na, pia, [r for r, _ in seq], bs, out.reshape(-1), precision=precision)
-        plan.run()
-        torch.cuda.current_stream(dev).synchronize()
-        plan.close()
-    return out.cpu().numpy() if host else out
+    prec = _lib.PRECISIONS.get(precision, precision) if isinstance(precision, str) else int(precision)
+    stream = torch.cuda.current_stream(dev)
+    if not steps:
+        raise _lib.TtmError(_lib.ERR_ARG, "tlibttm_plan_chain: the chain is empty.")
+    for s, (r, b) in enumerate(steps):
+        na = list(c.shape)
+        nc = list(na)
+        nc[r - 1] = int(b.shape[0])
+        out = torch.empty(nc, device=dev, dtype=dt)
+        try:
+            _on_device(c, _dtype_id(dt), prec, r, p, c.data_ptr(), na, _dense_strides(na, pia), pia, b.data_ptr(),
+                       list(b.shape), [2, 1], out.data_ptr(), nc, _dense_strides(nc, pia), stream.cuda_stream)
+        except _lib.TtmError as e:
+            if e.code != _lib.ERR_ARG:
+                raise
+            raise _lib.TtmError(e.code, f"step {s}: {e}") from None
+        c = out
+    if host:
+        return c.cpu().numpy()
+    stream.synchronize()
+    return c

@@ -26,9 +26,12 @@
 //
 // MMA kernel warp roles (320 threads, one CTA per SM, persistent over tiles):
 //   warp 0     bulk-copy producer: the A and B image blocks of one l chunk per stage
-//   warp 1     TMEM allocator and MMA issuer (one lane)
-//   warps 2-9  epilogue: TMEM -> registers -> scaled C, direct stores; two warps per TMEM lane
-//              quarter, taking alternate 32-column chunks
+//   warp 1     TMEM allocator and MMA issuer (the whole warp, one elected lane per MMA)
+//   warps 2-17 epilogue: TMEM -> registers -> scaled C, direct stores; four warps per TMEM lane
+//              quarter, taking every fourth chunk of 32 (fp8) or 16 (ozaki) columns. Ozaki's 7
+//              accumulators fill tensor memory, so its epilogue is not overlapped: with two warps
+//              per quarter and a lone lane issuing the MMAs the kernel took 144 us on A 256^3,
+//              m = 128; with four, and the whole warp issuing, 90 us.
 // Every mbarrier wait is bounded; on expiry the CTA aborts as the bf16x3 kernel does.
 #include <cuda.h>
 #include <cuda_fp8.h>
@@ -49,7 +52,8 @@ constexpr int kRows = 128;             // MMA M
 constexpr int kLChunk = 32;            // l per stage (one 8-bit MMA K step)
 constexpr int kBlock = kRows * 32;     // bytes of one 128-row image block
 constexpr int kOzakiSlices = 7;       // the epilogue's exact two-part combination assumes 7
-constexpr int kThreads8 = 10 * 32;           // producer, MMA, 8 epilogue warps
+constexpr int kEpiWarps8 = 16;
+constexpr int kThreads8 = (2 + kEpiWarps8) * 32;   // producer, MMA, epilogue warps
 constexpr int kMaxStages8 = 8;
 constexpr int kMaxNq8 = 16384;         // int32 accumulators stay exact: 7 * nq * 127^2 < 2^31
 enum { MODE_FP8 = 0, MODE_I8 = 1 };
@@ -113,6 +117,151 @@ __device__ __forceinline__ double pow2d(int e)
     return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52) : ldexp(1.0, e);
 }
 
+// Digits of 16 doubles, |x_t| 2^sh < 2^49 truncated to an integer and cut into 7 signed 7-bit
+// digits: word w of digit s holds those of elements 4 w .. 4 w + 3, one byte each.
+struct Digits {
+    uint32_t lo[16], hi[16];   // the integer's low 28 and high 21 bits
+    uint32_t neg[4];           // 0xff in the bytes of negative elements
+
+    __device__ __forceinline__ void set(const double (&x)[16], int sh)
+    {
+        const bool fast = sh >= -1022 && sh <= 1023;
+        const double sc = fast ? pow2d(sh) : 1.0;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) {
+            // exact scaling; adding 2^52 with rounding toward zero leaves the truncated integer in
+            // the low bits of the sum
+            const double y = fabs(fast ? x[t] * sc : ldexp(x[t], sh));
+            const unsigned long long b = (unsigned long long)__double_as_longlong(__dadd_rz(y, 0x1p52));
+            lo[t] = (uint32_t)b & 0xfffffffu;
+            hi[t] = (uint32_t)(b >> 28) & 0x1fffffu;
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            neg[w] = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (__double_as_longlong(x[4 * w + t]) < 0) neg[w] |= 0xffu << (8 * t);
+        }
+    }
+
+    template <int SL>
+    __device__ __forceinline__ uint4 digit() const
+    {
+        uint32_t r[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            uint32_t d = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const uint32_t v = SL < 3 ? hi[4 * w + t] >> (7 * (2 - SL)) : lo[4 * w + t] >> (7 * (6 - SL));
+                d |= (v & 127u) << (8 * t);
+            }
+            // two's complement of the negative bytes, without carries between bytes
+            const uint32_t f = d ^ neg[w];
+            r[w] = ((f & 0x7f7f7f7fu) + (neg[w] & 0x01010101u)) ^ (f & 0x80808080u);
+        }
+        return make_uint4(r[0], r[1], r[2], r[3]);
+    }
+
+    __device__ __forceinline__ void store(uint8_t* dst, uint32_t block) const
+    {
+        *reinterpret_cast<uint4*>(dst) = digit<0>();
+        *reinterpret_cast<uint4*>(dst + block) = digit<1>();
+        *reinterpret_cast<uint4*>(dst + 2 * block) = digit<2>();
+        *reinterpret_cast<uint4*>(dst + 3 * block) = digit<3>();
+        *reinterpret_cast<uint4*>(dst + 4 * block) = digit<4>();
+        *reinterpret_cast<uint4*>(dst + 5 * block) = digit<5>();
+        *reinterpret_cast<uint4*>(dst + 6 * block) = digit<6>();
+    }
+};
+
+// Exponents and digits of A in one launch (ozaki): a block takes 32 rows, finds their maxima, then
+// reads them again (from L2: 148 SMs x a few blocks x 32 rows) and writes the image as slice_kernel
+// does. Bound by reading A and writing 7/8 of its bytes; on A 256^3 the two kernels took 39 and 125
+// us, the second on 64-bit digit arithmetic, this one 70 us (contiguous fibres 93).
+__global__ void __launch_bounds__(256, 2) exponent_slice_kernel(RowView v, int64_t r0, int64_t nrows, int* __restrict__ ex,
+                                                               int kchunks, uint8_t* __restrict__ img)
+{
+    __shared__ double red[8][32];
+    __shared__ int es[32];
+    const double* a = static_cast<const double*>(v.base);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t b0 = (int64_t)blockIdx.x * 32;   // first row of the block within the chunk
+    if (v.ls == 1) {
+        // contiguous fibres: a warp reads four rows, lanes along l
+        double mx[4] = {0.0, 0.0, 0.0, 0.0};
+        const double* p[4];
+        bool ok[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int64_t rr = b0 + warp * 4 + r;
+            ok[r] = rr < nrows;
+            p[r] = a + (ok[r] ? row_off(v, r0 + rr) : 0);
+        }
+#pragma unroll 4
+        for (int64_t l = lane; l < v.nq; l += 32) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) mx[r] = fmax(mx[r], ok[r] ? fabs(__ldg(p[r] + l)) : 0.0);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mx[r] = fmax(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
+            if (lane == 0) {
+                int e = 0;
+                if (mx[r] > 0.0) frexp(mx[r], &e);
+                es[warp * 4 + r] = e;
+            }
+        }
+    } else {
+        // a lane reads one row; the warps split l
+        double mx = 0.0;
+        if (b0 + lane < nrows) {
+            const double* p = a + row_off(v, r0 + b0 + lane);
+#pragma unroll 8
+            for (int64_t l = warp; l < v.nq; l += 8) mx = fmax(mx, fabs(__ldg(p + l * v.ls)));
+        }
+        red[warp][lane] = mx;
+        __syncthreads();
+        if (warp == 0) {
+#pragma unroll
+            for (int w = 1; w < 8; ++w) mx = fmax(mx, red[w][lane]);
+            int e = 0;
+            if (mx > 0.0) frexp(mx, &e);
+            es[lane] = e;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32 && b0 + threadIdx.x < nrows) ex[b0 + threadIdx.x] = es[threadIdx.x];
+    // thread: half c of a 32-l chunk of one row; neighbouring lanes the two halves of a row
+    const int c = threadIdx.x & 1, row = (threadIdx.x >> 1) & 31;
+    const int64_t rr = b0 + row, tile = b0 / kRows;
+    const bool rv = rr < nrows;
+    const double* p = a + (rv ? row_off(v, r0 + rr) : 0);
+    const int sh = 7 * kOzakiSlices - es[row];
+    const bool vec = v.ls == 1 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;   // the thread's 16 l contiguous
+    const uint32_t off = kmaj_sw32_off((uint32_t)(rr - tile * kRows), (uint32_t)c);
+    for (int kc = threadIdx.x >> 6; kc < kchunks; kc += 4) {
+        const int64_t l0 = (int64_t)kc * kLChunk + c * 16;
+        double x[16];
+        if (vec && rv && l0 + 16 <= v.nq) {
+#pragma unroll
+            for (int t = 0; t < 16; t += 2) {
+                const double2 y = __ldg(reinterpret_cast<const double2*>(p + l0 + t));
+                x[t] = y.x;
+                x[t + 1] = y.y;
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < 16; ++t) x[t] = rv && l0 + t < v.nq ? __ldg(p + (l0 + t) * v.ls) : 0.0;
+        }
+        Digits d;
+        d.set(x, sh);
+        d.store(img + (size_t)((tile * kchunks + kc) * kOzakiSlices) * kBlock + off, kBlock);
+    }
+}
+
 // Slicer: rows [r0, r0 + nrows) -> image blocks [tile][kc][S][tile_rows x 32 B], tile_rows rows
 // per tile (zero beyond the operand's rows and l extent). One thread per (row, l chunk, half):
 // 16 consecutive l -> one 16-byte chunk per slice; the two halves of a row are neighbouring
@@ -156,31 +305,12 @@ __global__ void slice_kernel(RowView v, int64_t r0, int64_t nrows, const int* __
                 }
                 *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
             } else {
-                // |x| 2^(-e) < 1: its first 7 S bits, truncated, as one integer (exact scaling and
-                // truncation toward zero), then cut into base-128 digits carrying x's sign
-                const int sh = 7 * S - e;
-                const bool fast = sh >= -1022 && sh <= 1023;
-                const double sc = fast ? pow2d(sh) : 1.0;
-                long long mag[16];
-                bool neg[16];
+                double x[16];
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    const int64_t l = l0 + t;
-                    const double x = (rv && l < v.nq) ? (double)p[l * v.ls] : 0.0;
-                    const long long X = __double2ll_rz(fast ? x * sc : ldexp(x, sh));
-                    neg[t] = X < 0;
-                    mag[t] = X < 0 ? -X : X;
-                }
-                for (int s = 0; s < S; ++s) {
-                    const int shift = 7 * (S - 1 - s);
-                    uint32_t w[4] = {0, 0, 0, 0};
-#pragma unroll
-                    for (int t = 0; t < 16; ++t) {
-                        const int d = (int)((mag[t] >> shift) & 127);
-                        w[t >> 2] |= (uint32_t)(uint8_t)(int8_t)(neg[t] ? -d : d) << ((t & 3) * 8);
-                    }
-                    *reinterpret_cast<uint4*>(dst + (size_t)s * block) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
+                for (int t = 0; t < 16; ++t) x[t] = (rv && l0 + t < v.nq) ? (double)p[(l0 + t) * v.ls] : 0.0;
+                Digits d;
+                d.set(x, 7 * kOzakiSlices - e);
+                d.store(dst, block);
             }
         }
     }
@@ -212,14 +342,14 @@ __device__ __forceinline__ void mma_8bit(uint32_t tmem_d, uint64_t adesc, uint64
 {
     if (MODE == MODE_FP8)
         asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n"
+            "{\n .reg .pred p, e;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+            " @e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n"
             ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
             : "memory");
     else
         asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n"
+            "{\n .reg .pred p, e;\n elect.sync _|e, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n"
+            " @e tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}\n"
             ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
             : "memory");
 }
@@ -251,7 +381,7 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 8);
+            mbar_init(&acc_empty[b], kEpiWarps8);
         }
         mbar_init(drain, 1);
         *abort_flag = 0;
@@ -294,46 +424,48 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = idesc_8bit(MODE, NT);
-            int s = 0;
-            uint32_t ph = 0;
-            int ab = 0;
-            uint32_t cph = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < P.tiles && ok; t += gridDim.x) {
-                if (!mbar_wait(&acc_empty[ab], cph ^ 1, abort_flag)) break;
+        // warp-uniform descriptors, plain additions of multiples of 16 bytes in their address field
+        constexpr int SC = MODE == MODE_FP8 ? 1 : kOzakiSlices;
+        const uint32_t idesc = idesc_8bit(MODE, NT);
+        const uint64_t da0 = smem_desc(su32(ring), 16u, 256u, kLayoutSW32), db0 = da0 + (uint64_t)(a_bytes >> 4);
+        int s = 0;
+        uint32_t ph = 0;
+        int ab = 0;
+        uint32_t cph = 0;
+        bool ok = true;
+        for (int64_t t = blockIdx.x; t < P.tiles && ok; t += gridDim.x) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[ab], cph ^ 1, abort_flag))) break;
+            tc_fence_after();
+            const uint32_t dcol = tmem_base + (uint32_t)(ab * D * NT);
+            for (int kc = 0; kc < kchunks; ++kc) {
+                if (!__all_sync(0xffffffffu, mbar_wait(&full[s], ph, abort_flag))) { ok = false; break; }
                 tc_fence_after();
-                const uint32_t dcol = tmem_base + (uint32_t)(ab * D * NT);
-                for (int kc = 0; kc < kchunks; ++kc) {
-                    if (!mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t sa = su32(ring + (size_t)s * stage_bytes), sb = sa + a_bytes;
-                    // digit pairs (x, y) with x + y < S, accumulated on diagonal x + y; x = 0
-                    // opens every diagonal at the first l chunk
-                    for (int x = 0; x < S; ++x) {
-                        const uint64_t ad = smem_desc(sa + (uint32_t)x * kBlock, 16u, 256u, kLayoutSW32);
-                        for (int y = 0; x + y < S; ++y) {
-                            const uint64_t bd = smem_desc(sb + (uint32_t)y * b_block, 16u, 256u, kLayoutSW32);
-                            const int d = MODE == MODE_FP8 ? 0 : x + y;
-                            mma_8bit<MODE>(dcol + (uint32_t)(d * NT), ad, bd, idesc, (kc == 0 && x == 0) ? 0u : 1u);
-                        }
-                    }
-                    mma_commit(&empty[s]);
-                    if (++s == ST) { s = 0; ph ^= 1; }
-                }
-                if (!ok) break;
-                mma_commit(&acc_full[ab]);
-                if (++ab == P.nbuf) { ab = 0; cph ^= 1; }
+                const uint64_t da = da0 + (uint64_t)(s * stage_bytes >> 4), db = db0 + (uint64_t)(s * stage_bytes >> 4);
+                // digit pairs (x, y) with x + y < S, accumulated on diagonal x + y; x = 0
+                // opens every diagonal at the first l chunk
+#pragma unroll
+                for (int x = 0; x < SC; ++x)
+#pragma unroll
+                    for (int y = 0; x + y < SC; ++y)
+                        mma_8bit<MODE>(dcol + (uint32_t)((MODE == MODE_FP8 ? 0 : x + y) * NT),
+                                       da + (uint64_t)(x * kBlock >> 4), db + (uint64_t)(y * b_block >> 4), idesc,
+                                       (kc == 0 && x == 0) ? 0u : 1u);
+                mma_commit_warp(&empty[s]);
+                if (++s == ST) { s = 0; ph ^= 1; }
             }
-            mma_commit(drain);
-            const unsigned long long t0 = gtimer();
-            while (!mbar_try(drain, 0) && gtimer() - t0 < kTimeoutNs) {}
+            if (!ok) break;
+            mma_commit_warp(&acc_full[ab]);
+            if (++ab == P.nbuf) { ab = 0; cph ^= 1; }
         }
+        mma_commit_warp(drain);
+        const unsigned long long t0 = gtimer();
+        while (!mbar_try(drain, 0) && gtimer() - t0 < kTimeoutNs) {}
+        __syncwarp();
     } else {
         // ---------------------------------------------------------------- epilogue
         const int q4 = warp & 3;                 // TMEM lane quarter
-        const int half = (warp - 2) >> 2;        // 32-column chunks of this parity
+        const int part = (warp - 2) >> 2;        // every fourth chunk of columns, from this one
+        constexpr int kCols = MODE == MODE_FP8 ? 32 : 16;
         int ab = 0;
         uint32_t aph = 0;
         for (int64_t t = blockIdx.x; t < P.tiles; t += gridDim.x) {
@@ -343,13 +475,13 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
             const int64_t rl = mt * kRows + q4 * 32 + lane;           // row within the chunk
             const bool rv = rl < P.nrows;
             const int64_t R = P.r0 + rl;
-            const int64_t kk = R / P.inner;
+            const int64_t kk = slice_of(R, P.inner);
             const int64_t cbase = kk * P.m * P.inner + (R - kk * P.inner);
             const int ea = rv ? P.aexp[rl] : 0;
             const uint32_t tb = tmem_base + ((uint32_t)(q4 * 32) << 16) + (uint32_t)(ab * D * NT);
-            for (int cc = half * 32; cc < NT; cc += 64) {
+            for (int cc = part * kCols; cc < NT; cc += 4 * kCols) {
                 const int64_t j0 = jb * NT + cc;
-                const int eb_l = (j0 + lane < P.m) ? P.bexp[j0 + lane] : 0;
+                const int eb_l = (lane < kCols && j0 + lane < P.m) ? P.bexp[j0 + lane] : 0;
                 if (MODE == MODE_FP8) {
                     // C = acc 2^(ea-8) 2^(eb-8): two exact power-of-two products
                     uint32_t v[32];
@@ -376,38 +508,34 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
                     // H = sum_{d<3} acc_d 2^7(2-d) (< 2^43) and L = sum_{d>=3} acc_d 2^7(6-d) (< 2^52)
                     const double sa = pow2d(ea), sb_l = pow2d(eb_l - 28);   // row / this lane's column
                     double* C = static_cast<double*>(P.c);
+                    long long H[16], Lo[16];
 #pragma unroll
-                    for (int h16 = 0; h16 < 32; h16 += 16) {
-                        long long H[16], Lo[16];
+                    for (int c = 0; c < 16; ++c) H[c] = Lo[c] = 0;
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) H[c] = Lo[c] = 0;
+                    for (int d = 0; d < kOzakiSlices; ++d) {
+                        uint32_t v[16];
+                        tmem_ld16(tb + (uint32_t)(d * NT + cc), v);
 #pragma unroll
-                        for (int d = 0; d < kOzakiSlices; ++d) {
-                            uint32_t v[16];
-                            tmem_ld16(tb + (uint32_t)(d * NT + cc + h16), v);
-#pragma unroll
-                            for (int c = 0; c < 16; ++c) {
-                                const long long x = (long long)(int)v[c];
-                                if (d < 3) H[c] += x * (1LL << (7 * (2 - d)));
-                                else Lo[c] += x * (1LL << (7 * (6 - d)));
-                            }
+                        for (int c = 0; c < 16; ++c) {
+                            const long long x = (long long)(int)v[c];
+                            if (d < 3) H[c] += x * (1LL << (7 * (2 - d)));
+                            else Lo[c] += x * (1LL << (7 * (6 - d)));
                         }
-                        double y[16];
+                    }
+                    double y[16];
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        y[c] = fma((double)Lo[c], 0x1p-28, (double)H[c]) * sa * __shfl_sync(0xffffffffu, sb_l, c);
+                    if (P.inner == 1 && j0 + 16 <= P.m && (((cbase + j0) & 1) == 0)) {
+                        if (rv) {
+                            double2* cp = reinterpret_cast<double2*>(C + cbase + j0);
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) cp[c] = make_double2(y[2 * c], y[2 * c + 1]);
+                        }
+                    } else {
 #pragma unroll
                         for (int c = 0; c < 16; ++c)
-                            y[c] = fma((double)Lo[c], 0x1p-28, (double)H[c]) * sa * __shfl_sync(0xffffffffu, sb_l, h16 + c);
-                        const int64_t jc = j0 + h16;
-                        if (P.inner == 1 && jc + 16 <= P.m && (((cbase + jc) & 1) == 0)) {
-                            if (rv) {
-                                double2* cp = reinterpret_cast<double2*>(C + cbase + jc);
-#pragma unroll
-                                for (int c = 0; c < 8; ++c) cp[c] = make_double2(y[2 * c], y[2 * c + 1]);
-                            }
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < 16; ++c)
-                                if (rv && jc + c < P.m) C[cbase + (jc + c) * P.inner] = y[c];
-                        }
+                            if (rv && j0 + c < P.m) C[cbase + (j0 + c) * P.inner] = y[c];
                     }
                 }
             }
@@ -508,7 +636,8 @@ int tc8_launches(const View3& v, int precision)
     if (!plan8(v, precision, p)) return 0;
     const int64_t rows = v.outer * v.inner;
     const int64_t chunk = std::min<int64_t>(p.chunk_rows, ((rows + kRows - 1) / kRows) * kRows);
-    return (int)(2 + 3 * ((rows + chunk - 1) / chunk));   // B exponents + slicer, then per chunk three
+    // B exponents + slicer, then per chunk of rows the operand kernels (fp8 two, ozaki one) and the MMA kernel
+    return (int)(2 + (p.mode == MODE_FP8 ? 3 : 2) * ((rows + chunk - 1) / chunk));
 }
 
 cudaError_t launch_tc8(const View3& v, int precision, int dtype, cudaStream_t s, int* kid, int* launches)
@@ -567,8 +696,9 @@ cudaError_t launch_tc8(const View3& v, int precision, int dtype, cudaStream_t s,
             e = launch_exponents<float>(av, r0, nr, aexp, s);
             if (e == cudaSuccess) e = launch_slices<float, MODE_FP8>(av, r0, nr, aexp, p.S, kRows, p.kchunks, aimg, s);
         } else {
-            e = launch_exponents<double>(av, r0, nr, aexp, s);
-            if (e == cudaSuccess) e = launch_slices<double, MODE_I8>(av, r0, nr, aexp, p.S, kRows, p.kchunks, aimg, s);
+            const int64_t tiles = (nr + kRows - 1) / kRows;
+            exponent_slice_kernel<<<(unsigned)(tiles * (kRows / 32)), 256, 0, s>>>(av, r0, nr, aexp, p.kchunks, aimg);
+            e = cudaGetLastError();
         }
         if (e != cudaSuccess) break;
         Tc8Params P{};
@@ -593,7 +723,7 @@ cudaError_t launch_tc8(const View3& v, int precision, int dtype, cudaStream_t s,
         if (fp8) tc8_kernel<MODE_FP8><<<grid, kThreads8, p.smem, s>>>(P);
         else tc8_kernel<MODE_I8><<<grid, kThreads8, p.smem, s>>>(P);
         e = cudaGetLastError();
-        n += 3;
+        n += fp8 ? 3 : 2;
     }
     cudaFreeAsync(scratch, s);
     *launches = n;

@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "few_columns.cuh"
 #include "gemm_f32.cuh"
 #include "gemm_f64.cuh"
 
@@ -368,6 +369,14 @@ __global__ void __launch_bounds__(256) colvec_async_kernel(View3 v)
 {
     __shared__ ColvecAsyncSmem<T, MB> sm;
     colvec_async_tile<T, MB, LS>(v, (int64_t)blockIdx.x * (kColWarps / LS) * 32, sm);
+}
+
+// few_columns.cuh: rows of i off 16-byte boundaries, m <= 8, long l ranges.
+template <int TN, bool BCM>
+__global__ void __launch_bounds__(few::NT, 3) few_columns_kernel(View3 v)
+{
+    extern __shared__ __align__(16) unsigned char few_smem[];
+    few::tile<TN, BCM>(v, blockIdx.x, *reinterpret_cast<few::Smem<TN>*>(few_smem));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -994,11 +1003,38 @@ cudaError_t colvec_dispatch_w(const View3& v, cudaStream_t s)
     return row_warps < 148 * 32 ? colvec_dispatch_ls<T, W, 8>(v, s) : colvec_dispatch_ls<T, W, 1>(v, s);
 }
 
+template <int TN>
+cudaError_t few_columns_launch(const View3& v, cudaStream_t s)
+{
+    constexpr int smem = (int)sizeof(few::Smem<TN>);
+    const auto kernel = v.b_cm ? few_columns_kernel<TN, true> : few_columns_kernel<TN, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<(unsigned)(v.outer * ceil_div(v.inner, few::BM)), few::NT, smem, s>>>(v);
+    return cudaGetLastError();
+}
+
+// Measured against the column kernel on A of 160 MB, as its time over the few-column kernel's: with
+// tiles full 1.2-1.6 at m = 1 from n_q = 17, 1.25-1.9 at m = 2..4 and 1.1-1.8 at m = 5..8 from n_q =
+// 33 (0.75-1.0 at 17); half-full tiles (inner 129, 257) 1.2-1.3 at m = 1, 1.05-1.1 at 2..4, 0.9 at
+// 5..8, and 1.04 there at 0.59 full (inner 301). Fewer tiles than this leave SMs idle, where the
+// column kernel splits l.
+bool few_columns_takes(const View3& v)
+{
+    const int64_t per_slice = ceil_div(v.inner, few::BM), room = per_slice * few::BM;
+    return v.m <= 8 && v.inner % 4 != 0 && aligned16(v.a) && v.outer * per_slice >= 128 && v.nq >= (v.m == 1 ? 17 : 33) &&
+           16 * v.inner >= (v.m <= 4 ? 8 : 9) * room;
+}
+
 template <typename T>
 cudaError_t colvec_dispatch(const View3& v, cudaStream_t s)
 {
     constexpr int RV = 16 / sizeof(T);
     const bool vec = aligned16(v.a) && aligned16(v.c) && (v.inner % RV == 0);
+    if constexpr (sizeof(T) == 4)
+        if (few_columns_takes(v))
+            return v.m <= 1 ? few_columns_launch<1>(v, s) : v.m <= 2 ? few_columns_launch<2>(v, s)
+                 : v.m <= 4 ? few_columns_launch<4>(v, s) : few_columns_launch<8>(v, s);
     return vec ? colvec_dispatch_w<T, RV>(v, s) : colvec_dispatch_w<T, 1>(v, s);
 }
 

@@ -109,6 +109,7 @@ struct alignas(64) TcProb {
     int tma_c;               // epilogue stores C through the C tensor map
     int fold_kb;             // GEOM_MN with inner <= 64: slices per 128-row tile (1: unfolded)
     int fold_ib_shift;       // log2 of the rows each slice takes in a folded tile (32 or 64)
+    int halves;              // GEOM_MN: M tiles are two half tiles of 64 rows, numbered through the slices
     int b_cm;
 };
 
@@ -230,7 +231,9 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map)
 // a stage). Measured, one tile at a time -> pairs: A 192^4, slowest mode, m = 32 1184 -> 1045 us
 // (0.93 of the copy bandwidth), contiguous fibres 1170 -> 973 us; (300, 420, 500), m = 96 98 -> 89 us.
 // Wider tiles go one at a time: tensor memory holds two of 256 columns.
-template <int GEOM, bool GROUP, int H>
+// HALF: some problem of the launch has M tiles in halves (a build of its own: the checks cost the
+// converters of full tiles 8 %).
+template <int GEOM, bool GROUP, int H, bool HALF>
 __global__ void __launch_bounds__(kThreads, 1)
     tc_bf16x3_kernel(const __grid_constant__ TcProb one, TcParams P)
 {
@@ -304,14 +307,28 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // every load of the CTA, and a division or a reload of the record per copy showed as
                 // 1100 of the 1200 cycles that a stage of 32 l took
                 const int kst = pr.kstages, kch = pr.kchunks, fold = pr.fold_kb;
-                const bool ldg = pr.ldg_a != 0;
+                const bool ldg = pr.ldg_a != 0, halves = HALF && pr.halves != 0;
                 const CUtensorMap* const amap = &pr.amap;
                 if (GROUP && &pr != last && !ldg) tensormap_acquire(amap);
                 last = &pr;
                 int nh;
                 const int64_t tm = pr.tiles_m, sub0 = first_m_tile<H>(lt, pr.pairs, nh), mt = sub0 - slice_of(sub0, tm) * tm;
-                int c0[H], ck[H];   // per M tile: its first row (i, or the fibre for GEOM_K) and slice
+                // per M tile: its first row (i, or the fibre for GEOM_K) and slice; of its second half too
+                int c0[H], ck[H], d0[H], dk[H];
                 const int64_t mper = (pr.inner + kBM - 1) / kBM;
+                int absent = 0;   // half tiles past the last slice
+                if (halves) {
+                    const int64_t hper = (pr.inner + kBM / 2 - 1) / (kBM / 2);
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        const int64_t b = 2 * (mt + h), k0 = slice_of(b, hper), k1 = slice_of(b + 1, hper);
+                        ck[h] = (int)k0;
+                        c0[h] = (int)(b - k0 * hper) * (kBM / 2);
+                        dk[h] = (int)k1;
+                        d0[h] = (int)(b + 1 - k1 * hper) * (kBM / 2);
+                        if (h < nh && k1 >= pr.outer) ++absent;
+                    }
+                } else
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
                     ck[h] = 0;
@@ -343,7 +360,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     phases = (phases & ~(1u << s)) | (ph << s);
                     // the sub-blocks within n_q (the last box's rows past n_q are zero-filled)
                     const int nsub = min(kSub, kch - st * kSub);
-                    mbar_expect_tx(&a_full[s], (uint32_t)(nh * nsub) * LA.asub_bytes);
+                    mbar_expect_tx(&a_full[s], (uint32_t)((2 * nh - absent) * nsub) * (LA.asub_bytes / 2));
 #pragma unroll
                     for (int h = 0; h < H; ++h)
 #pragma unroll
@@ -354,6 +371,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                             if (GEOM == GEOM_MN) {
                                 if (fold > 1) tma_load_3d(dst, amap, &a_full[s], 0, ck[h], l0);
                                 else tma_load_3d(dst, amap, &a_full[s], c0[h], l0, ck[h]);
+                                if (halves && !(absent && h == nh - 1))
+                                    tma_load_3d(dst + LA.asub_bytes / 2, amap, &a_full[s], d0[h], l0, dk[h]);
                             } else {
                                 tma_load_2d(dst, amap, &a_full[s], l0, c0[h]);
                             }
@@ -486,6 +505,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         // this thread's float4 positions in a sub-block: where it reads the FP32 tile and where
         // its 16-byte chunks of the bf16 parts go (the same for every sub-block)
         uint32_t rdo[kIters], wro[kIters];
+        // in half tiles a line is 64 rows long
+        const uint32_t rdh = (uint32_t)((gt & 31) >> 4) * (LA.asub_bytes / 2) + (uint32_t)((gt >> 5) * 256 + (gt & 15) * 16);
 #pragma unroll
         for (int it = 0; it < kIters; ++it) {
             const int v = gt + kGroupWarps * 32 * it;
@@ -517,6 +538,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             // converters' own loads only where they load A
             const int kst = pr.kstages, kch = pr.kchunks;
             const bool ldg = pr.ldg_a != 0;
+            const bool halves = HALF && pr.halves != 0;
             int nh;
             const int64_t sub0 = first_m_tile<H>(lt, pr.pairs, nh);
             const float* ga = nullptr;
@@ -553,6 +575,13 @@ __global__ void __launch_bounds__(kThreads, 1)
                     uint8_t* buf = a_at(s) + (unit + u) * LA.asub_bytes;
                     float4 x[kIters];
                     uint32_t off[kIters];
+                    if (HALF && halves && have) {
+#pragma unroll
+                        for (int it = 0; it < kIters; ++it) {
+                            x[it] = *reinterpret_cast<const float4*>(buf + rdh + it * (kGroupWarps * 256));
+                            off[it] = wro[it];
+                        }
+                    } else
 #pragma unroll
                     for (int it = 0; it < kIters; ++it) {
                         const int v = gt + kGroupWarps * 32 * it;   // float4 index within the 8 KB tile
@@ -640,6 +669,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             float* const e_c = pr.c;
             const bool e_tma = pr.tma_c != 0;
             const int e_fold = pr.fold_kb, e_shift = pr.fold_ib_shift;
+            const bool e_halves = HALF && pr.halves != 0;
             int nh;
             const int64_t tm = pr.tiles_m, sub0 = first_m_tile<H>(lt, pr.pairs, nh), jb = slice_of(sub0, tm);
             const int64_t jrem = e_m - jb * nt;
@@ -652,6 +682,10 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // this warp's 32 rows lie in one slice of the folded tile
                 k = mt * e_fold + ((q4 * 32) >> e_shift);
                 r0 = (q4 * 32) & ((1 << e_shift) - 1);
+            } else if (e_halves) {
+                const int64_t hper = (e_inner + kBM / 2 - 1) / (kBM / 2), b = 2 * mt + (q4 >> 1);
+                k = slice_of(b, hper);
+                r0 = (b - k * hper) * (kBM / 2) + (q4 & 1) * 32;
             } else if (GEOM == GEOM_MN) {
                 k = slice_of(mt, mper);
                 r0 = (mt - k * mper) * kBM + q4 * 32;
@@ -667,7 +701,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (cc >= jleft) continue;
                 const int j0 = (int)(jb * nt) + cc;
                 if (e_tma && GEOM == GEOM_MN && k >= e_outer) {
-                    // folded last tile: this warp's slice lies past the end of C, nothing to store
+                    // last tile, folded or in halves: this warp's slice lies past the end of C
                 } else if (e_tma) {
                     // Stage a 32 x 32 block in shared memory and store it with one TMA copy.
                     uint8_t* buf = stage0 + sb * kEpiBuf;
@@ -1283,7 +1317,7 @@ EncodeTiledFn encode_fn()
     return fn;
 }
 
-bool encode_a_map(const View3& v, int geom, CUtensorMap* map)
+bool encode_a_map(const View3& v, int geom, CUtensorMap* map, int rows = kBM)
 {
     EncodeTiledFn cuTensorMapEncodeTiled = encode_fn();
     if (!cuTensorMapEncodeTiled) return false;
@@ -1291,7 +1325,7 @@ bool encode_a_map(const View3& v, int geom, CUtensorMap* map)
     if (geom == GEOM_MN) {
         cuuint64_t dims[3] = {(cuuint64_t)v.inner, (cuuint64_t)v.nq, (cuuint64_t)v.outer};
         cuuint64_t strides[2] = {(cuuint64_t)v.inner * 4, (cuuint64_t)v.inner * v.nq * 4};
-        cuuint32_t box[3] = {kBM, kBK, 1};
+        cuuint32_t box[3] = {(cuuint32_t)rows, kBK, 1};
         cuuint32_t es[3] = {1, 1, 1};
         r = cuTensorMapEncodeTiled(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(v.a), dims, strides, box,
                                    es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -1363,6 +1397,13 @@ bool tma_a_ok(const View3& v, int geom)
     return geom == GEOM_K ? v.nq % 4 == 0 : v.inner % 4 == 0;
 }
 
+// M tiles as two half tiles of 64 rows, each with its own slice and first row, where a slice's last
+// 128-row tile would be at most half full.
+bool half_tiles(const View3& v)
+{
+    return v.inner > 64 && (v.inner - 1) % kBM < kBM / 2 && v.outer * ceil_div(v.inner, kBM / 2) < (int64_t(1) << 31);
+}
+
 // Fills the problem record of the bf16x3 kernel for view v, its pre-split B image at `img`
 // (tc_image_bytes(v) bytes); *geom receives its geometry.
 void make_tc_prob(const View3& v, uint8_t* img, TcProb& pr, int* geom)
@@ -1385,10 +1426,14 @@ void make_tc_prob(const View3& v, uint8_t* img, TcProb& pr, int* geom)
         pr.fold_ib_shift = v.inner <= 32 ? 5 : 6;
         pr.fold_kb = kBM >> pr.fold_ib_shift;
     }
+    pr.halves = !pr.ldg_a && half_tiles(v) ? 1 : 0;
     if (!pr.ldg_a && !(pr.fold_kb > 1 ? encode_a_map_folded(v, 1 << pr.fold_ib_shift, pr.fold_kb, &pr.amap)
-                                      : encode_a_map(v, g, &pr.amap)))
+                                      : encode_a_map(v, g, &pr.amap, pr.halves ? kBM / 2 : kBM)))
         pr.ldg_a = 1;   // the driver declined the map: the converters load A
-    if (pr.ldg_a) std::memset(&pr.amap, 0, sizeof(pr.amap));
+    if (pr.ldg_a) {
+        std::memset(&pr.amap, 0, sizeof(pr.amap));
+        pr.halves = 0;
+    }
     pr.tma_c = encode_c_map(v, g, &pr.cmap) ? 1 : 0;
     if (!pr.tma_c) std::memset(&pr.cmap, 0, sizeof(pr.cmap));
     pr.c = static_cast<float*>(v.c);
@@ -1398,6 +1443,7 @@ void make_tc_prob(const View3& v, uint8_t* img, TcProb& pr, int* geom)
     pr.inner = v.inner;
     pr.m = v.m;
     pr.tiles_m = g == GEOM_MN ? (pr.fold_kb > 1 ? (v.outer + pr.fold_kb - 1) / pr.fold_kb
+                                 : pr.halves    ? ceil_div(v.outer * ceil_div(v.inner, kBM / 2), 2)
                                                 : v.outer * ((v.inner + kBM - 1) / kBM))
                               : (v.outer + kBM - 1) / kBM;
     pr.pairs = 0;
@@ -1419,23 +1465,26 @@ void set_pairs(TcProb& pr, int64_t pairs)
 // j block (zero past n_q), nt rows each, in two 8-l halves.
 int64_t split_units(const TcProb& pr) { return (int64_t)pr.jblocks * (pr.kstages * kSub) * pr.nt * 2; }
 
-template <int GEOM, bool GROUP, int H>
+template <int GEOM, bool GROUP, int H, bool HALF>
 cudaError_t launch_tc_kernel(const TcProb& one, const TcParams& P, size_t smem, int grid, cudaStream_t s)
 {
-    const auto kernel = tc_bf16x3_kernel<GEOM, GROUP, H>;
+    const auto kernel = tc_bf16x3_kernel<GEOM, GROUP, H, HALF>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) kernel<<<grid, kThreads, smem, s>>>(one, P);
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 template <bool GROUP>
-cudaError_t launch_tc_any(int geom, int h, const TcProb& one, const TcParams& P, size_t smem, int grid, cudaStream_t s)
+cudaError_t launch_tc_any(int geom, int h, bool half, const TcProb& one, const TcParams& P, size_t smem, int grid, cudaStream_t s)
 {
-    if (geom == GEOM_MN)
-        return h == 2 ? launch_tc_kernel<GEOM_MN, GROUP, 2>(one, P, smem, grid, s)
-                      : launch_tc_kernel<GEOM_MN, GROUP, 1>(one, P, smem, grid, s);
-    return h == 2 ? launch_tc_kernel<GEOM_K, GROUP, 2>(one, P, smem, grid, s)
-                  : launch_tc_kernel<GEOM_K, GROUP, 1>(one, P, smem, grid, s);
+    if (geom == GEOM_K)
+        return h == 2 ? launch_tc_kernel<GEOM_K, GROUP, 2, false>(one, P, smem, grid, s)
+                      : launch_tc_kernel<GEOM_K, GROUP, 1, false>(one, P, smem, grid, s);
+    if (half)
+        return h == 2 ? launch_tc_kernel<GEOM_MN, GROUP, 2, true>(one, P, smem, grid, s)
+                      : launch_tc_kernel<GEOM_MN, GROUP, 1, true>(one, P, smem, grid, s);
+    return h == 2 ? launch_tc_kernel<GEOM_MN, GROUP, 2, false>(one, P, smem, grid, s)
+                  : launch_tc_kernel<GEOM_MN, GROUP, 1, false>(one, P, smem, grid, s);
 }
 
 // Splits B into `img` (tc_image_bytes(v) bytes) and launches the bf16x3 kernel for v on stream s.
@@ -1469,7 +1518,7 @@ cudaError_t run_bf16x3(const View3& v, uint8_t* img, int* status, int sms, cudaS
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int grid = (int)std::min<int64_t>(pr.tiles, sms);
-    return launch_tc_any<false>(geom, h, pr, P, smem, grid, s);
+    return launch_tc_any<false>(geom, h, pr.halves != 0, pr, P, smem, grid, s);
 }
 
 }  // namespace
@@ -1485,6 +1534,7 @@ struct TcGroup {
     TcParams P[4] = {};
     size_t smem[4] = {};
     int grid[4] = {};
+    bool half[4] = {};            // a problem of the class has M tiles in halves
 };
 
 namespace {
@@ -1551,6 +1601,7 @@ cudaError_t tc_group_create(const View3* views, int count, TcGroup** out)
         sorted[r].first = first[g];
         first[g] += probs[i].tiles;
         ntmax[g] = std::max(ntmax[g], probs[i].nt);
+        if (probs[i].halves) G->half[g] = true;
         ++n[g];
         max_units = std::max(max_units, split_units(probs[i]));
     }
@@ -1591,7 +1642,7 @@ cudaError_t tc_group_run(TcGroup* G, cudaStream_t s)
         if (P.count == 0) continue;
         P.wait_ns = wait_limit_ns();
         P.skip_b = take_skip_b() ? 1 : 0;
-        cudaError_t e = launch_tc_any<true>(g / 2, 2 - g % 2, g_no_prob, P, G->smem[g], G->grid[g], s);
+        cudaError_t e = launch_tc_any<true>(g / 2, 2 - g % 2, G->half[g], g_no_prob, P, G->smem[g], G->grid[g], s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -9,8 +9,9 @@
 // DFMA) once m passes about 24; below that, reading A. A k-step of four l costs a warp 1 or 2 A and
 // NF B shared loads for 2 NF mma of 256 multiply-adds each; the DFMA tile of 64 x 64 it replaced
 // needed 8 loads for 16 DFMA of 32. Measured, before -> now: A 256^3, m = 128, middle mode
-// 323 -> 150 us (29 TFLOP/s); (150, 171, 333), m = 100 189 -> 91 us; (200, 180, 160), m = 20
-// 84 -> 21 us; contiguous fibres of 384, 78000 rows, m = 16 (TMA row kernel) 139 -> 54 us.
+// 323 -> 144 us (30 TFLOP/s); (150, 171, 333), m = 100 189 -> 84 us; (200, 180, 160), m = 20
+// 84 -> 19 us; contiguous fibres of 384, 78000 rows, m = 16 (TMA row kernel) 139 -> 50 us. (Running
+// pointers in place of addresses recomputed per copy gave 5-15 % of that.)
 // Rows of 64 for at most 16 columns (five blocks of 128 threads per SM, 16-byte copies): 59 us at
 // 128 rows against 53; with 8-byte copies 128 rows are faster (73 against 119 us).
 #pragma once
@@ -112,47 +113,44 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     constexpr int LB = ((BCM ? BK : BN) + BY - 1) / BY;
     const int bx = tid % BX, by = tid / BX;
 
-    // the tile being loaded, and where in its l range
-    int64_t lt = first, ll = l_begin, ln0 = 0;
-    int a_rows = 0;          // contiguous fibres: rows of the tile in A; else 1 if this thread's row is
+    // the tile being loaded: this thread's first element of A and of B at the current stage, and
+    // how much of the l range is left
+    int64_t lt = first, left = 0;
+    int a_rows = 0;          // rows of the tile in A
+    int64_t b_cols = 0;      // columns of B from this tile's first
     const double* ap = A;
+    const double* bp = B;
     auto start = [&]() {
         const int64_t rt = gr.cols == 1 ? lt : slice_of(lt, gr.cols);
-        const int64_t m0 = rt * BM;
-        ln0 = (lt - rt * gr.cols) * gr.nf * 8;
+        const int64_t m0 = rt * BM, n0 = (lt - rt * gr.cols) * gr.nf * 8;
+        left = l_end - l_begin;
+        b_cols = m - n0;
+        if (!EXACT && b_cols > gr.nf * 8) b_cols = gr.nf * 8;
+        a_rows = (int)(M - m0 < BM ? M - m0 : BM);
         if (AK) {
-            a_rows = (int)(M - m0 < BM ? M - m0 : BM);
-            ap = A + (m0 + ay) * nq + ax;
+            ap = A + (m0 + ay) * nq + l_begin + ax;
         } else {
-            const int64_t row = m0 + ax;
-            a_rows = row < M;
-            const int64_t k = a_rows ? slice_of(row, inner) : 0;
-            ap = A + (a_rows ? k * inner * nq + (row - k * inner) : 0) + (int64_t)ay * inner;
+            const int64_t row = m0 + ax, k = slice_of(row, inner);
+            ap = A + (k * nq + l_begin + ay) * inner + (row - k * inner);
         }
+        bp = BCM ? B + (l_begin + by) * m + n0 + bx : B + (n0 + by) * nq + l_begin + bx;
     };
+    // copies with !ok zero their destination and read nothing (their addresses may lie outside)
+    const int64_t a_step = AK ? (int64_t)AY * nq : (int64_t)AY * inner, b_step = BCM ? BY * m : BY * nq;
     auto issue = [&](int st) {
+        const int n = left < BK ? (int)left : BK;
 #pragma unroll
         for (int s = 0; s < LA; ++s) {
-            if (AK) {
-                const bool ok = ay + s * AY < a_rows && ll + ax < l_end;
-                const double* src = ok ? ap + (int64_t)s * AY * nq + ll : A;
-                if (VEC) copy16(&sm.a[st][ay + s * AY][ax], src, ok);
-                else copy8(&sm.a[st][ay + s * AY][ax], src, ok);
-            } else {
-                const bool ok = a_rows && ll + ay + s * AY < l_end;
-                const double* src = ok ? ap + (ll + s * AY) * inner : A;
-                if (VEC) copy16(&sm.a[st][ay + s * AY][ax], src, ok);
-                else copy8(&sm.a[st][ay + s * AY][ax], src, ok);
-            }
+            const int yo = ay + s * AY;   // [row][l] or [l][row]
+            const bool ok = AK ? yo < a_rows && ax < n : ax < a_rows && yo < n;
+            if (VEC) copy16(&sm.a[st][yo][ax], ap + s * a_step, ok);
+            else copy8(&sm.a[st][yo][ax], ap + s * a_step, ok);
         }
 #pragma unroll
         for (int s = 0; s < LB; ++s) {
             const int jo = BCM ? bx : by + s * BY, lo = BCM ? by + s * BY : bx;
-            if (jo >= (EXACT ? BN : gr.nf * 8) || lo >= BK) continue;
-            const int64_t j = ln0 + jo, l = ll + lo;
-            const bool ok = j < m && l < l_end;
-            const double* src = ok ? (BCM ? B + j + l * m : B + j * nq + l) : B;
-            copy8(BCM ? &sm.b[st][lo][jo] : &sm.b[st][jo][lo], src, ok);
+            if (jo >= BN || lo >= BK) continue;
+            copy8(BCM ? &sm.b[st][lo][jo] : &sm.b[st][jo][lo], bp + s * b_step, jo < b_cols && lo < n);
         }
     };
     // loads one stage (none past the last tile) and moves on; one commit group per call, empty
@@ -160,9 +158,10 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     auto load_next = [&](int st) {
         if (lt < last) {
             issue(st);
-            ll += BK;
-            if (ll >= l_end) {
-                ll = l_begin;
+            left -= BK;
+            ap += AK ? BK : BK * inner;
+            bp += BCM ? BK * m : BK;
+            if (left <= 0) {
                 lt += step;
                 if (lt < last) start();
             }

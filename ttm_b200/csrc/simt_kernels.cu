@@ -489,6 +489,78 @@ __global__ void __launch_bounds__(256) rowdot_kernel(View3 v)
 }
 
 // ---------------------------------------------------------------------------------------------
+// rowwarp: small m (<= MB <= 8), float fibres whose ends are not on 16-byte boundaries (inner == 1).
+// A warp takes R rows at a time, lanes along l: its loads are 128 contiguous bytes whatever the
+// alignment, and a value of B from shared memory serves R rows. The R * MB sums of 32 lanes are
+// reduced by halving: a lane ends with one output (or a group of lanes with the same one), so that a
+// warp's outputs leave in one store. B's n_q <= kRowWarpNq columns are staged once per block.
+// The tile kernel above copied such rows through shared memory an element at a time: fibres of 1023,
+// m = 1 130 -> 46 us (3.5 TB/s), m = 8 188 -> 81 us; of 99, m = 2 56 -> 40 us. At m = 8 the reads of B
+// bind it (a warp's 1 KB of B per 512 bytes of A).
+// ---------------------------------------------------------------------------------------------
+constexpr int kRowWarpNq = 1024;
+
+template <int MB>
+__global__ void __launch_bounds__(256) rowwarp_kernel(View3 v)
+{
+    constexpr int R = MB == 8 ? 4 : 8, N = R * MB;
+    extern __shared__ __align__(16) float rw_smem[];   // [j][l], l padded with zeros to a multiple of 32
+    const float* __restrict__ A = static_cast<const float*>(v.a);
+    const float* __restrict__ B = static_cast<const float*>(v.b);
+    float* __restrict__ C = static_cast<float*>(v.c);
+    const int nq = (int)v.nq, m = (int)v.m, np = (nq + 31) / 32 * 32;
+    for (int e = threadIdx.x; e < MB * np; e += 256) {
+        const int j = e / np, l = e - j * np;
+        rw_smem[e] = j < m && l < nq ? (v.b_cm ? B[j + (int64_t)l * m] : B[(int64_t)j * nq + l]) : 0.0f;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t rows = v.outer, warps = (int64_t)gridDim.x * 8;
+    for (int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); g * R < rows; g += warps) {
+        const int64_t row0 = g * R;
+        const int have = (int)(rows - row0 < R ? rows - row0 : R);
+        const float* p = A + row0 * nq + lane;
+        float acc[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) acc[i] = 0.0f;
+#pragma unroll 2
+        for (int l0 = 0; l0 < np; l0 += 32) {
+            const bool ok = l0 + lane < nq;
+            float a[R], b[MB];
+#pragma unroll
+            for (int r = 0; r < R; ++r) a[r] = ok && r < have ? __ldg(p + (int64_t)r * nq + l0) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < MB; ++j) b[j] = rw_smem[j * np + l0 + lane];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int j = 0; j < MB; ++j) acc[r * MB + j] = __fmaf_rn(a[r], b[j], acc[r * MB + j]);
+        }
+        // output i ends in lanes i * 32 / N ..
+        int n = N;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            if (n > 1) {
+                n /= 2;
+                const bool up = lane & s;
+#pragma unroll
+                for (int i = 0; i < N / 2; ++i) {
+                    if (i < n) {
+                        const float send = up ? acc[i] : acc[i + n], keep = up ? acc[i + n] : acc[i];
+                        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+                    }
+                }
+            } else {
+                acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], s);
+            }
+        }
+        constexpr int G = 32 / N;   // lanes that hold the same output
+        const int i = lane / G, r = i / MB, j = i % MB;
+        if (lane % G == 0 && r < have && j < m) C[(row0 + r) * m + j] = acc[0];
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
 // rowflat: small m, contiguous fibres of at most kFlatMaxNq elements (inner == 1, short rows).
 // A warp's wr consecutive rows are wr * nq contiguous elements: the warp copies them with
 // coalesced loads into shared memory with rows padded to nq + 1 (conflict-free row reads), then
@@ -1097,6 +1169,27 @@ cudaError_t rowspan_launch(const View3& v, cudaStream_t s)
     return cudaGetLastError();
 }
 
+template <int MB>
+cudaError_t rowwarp_launch(const View3& v, cudaStream_t s)
+{
+    int sms = 0;
+    const cudaError_t e = sms_of_device(sms);
+    if (e != cudaSuccess) return e;
+    constexpr int R = MB == 8 ? 4 : 8;
+    const size_t smem = (size_t)MB * ceil_div(v.nq, 32) * 32 * sizeof(float);   // at most 32 KB
+    const int64_t blocks = std::min<int64_t>(ceil_div(v.outer, 8 * R), (int64_t)sms * 6);
+    rowwarp_kernel<MB><<<(unsigned)std::max<int64_t>(1, blocks), 256, smem, s>>>(v);
+    return cudaGetLastError();
+}
+
+// Measured against the tile kernel on A of 160 MB, its time over this one's: m <= 2 1.1-1.3 from n_q =
+// 33 (0.7 at 17 and 23, where lanes idle), m = 3, 4 1.06-1.1 from 99 (0.96 at 63), m = 5..8 1.05-1.07
+// at 263 (1.0 at 99); 1.4-2.8 everywhere at n_q = 511 and 1023.
+bool rowwarp_takes(const View3& v)
+{
+    return v.m <= 8 && v.nq >= (v.m <= 2 ? 32 : v.m <= 4 ? 96 : 256) && v.nq <= kRowWarpNq;
+}
+
 template <typename T>
 cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s)
 {
@@ -1121,6 +1214,10 @@ cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s)
     }
     constexpr int RV = 16 / sizeof(T);
     const bool vec = aligned16(v.a) && (v.nq % RV == 0);
+    if constexpr (sizeof(T) == 4)
+        if (!vec && rowwarp_takes(v))
+            return v.m <= 1 ? rowwarp_launch<1>(v, s) : v.m <= 2 ? rowwarp_launch<2>(v, s)
+                 : v.m <= 4 ? rowwarp_launch<4>(v, s) : rowwarp_launch<8>(v, s);
     return vec ? rowdot_dispatch_v<T, true>(v, s) : rowdot_dispatch_v<T, false>(v, s);
 }
 

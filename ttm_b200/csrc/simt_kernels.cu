@@ -235,7 +235,6 @@ __global__ void __launch_bounds__(256) colvec_kernel(View3 v)
 // holding them in registers. A thread reads back only what it copied itself: the ring needs no block barrier,
 // only the thread's own wait on its copy groups. B is staged per chunk of LB l as in colvec.
 constexpr int kColAsyncStages = 4;
-constexpr bool kColAsync = true;   // rows without 16-byte alignment take colvec_async
 
 template <typename T, int MB>
 struct ColvecAsyncSmem {
@@ -765,20 +764,22 @@ __global__ void __launch_bounds__(256) strided_kernel(StridedProblem sp)
 // counter; an item is one slice-GEMM tile of a problem (m > 16) or a block of 256 rows of a
 // small-m problem. Problems are ordered largest first by the host, so the tail is short.
 // ---------------------------------------------------------------------------------------------
-// ASYNC: unaligned column items take colvec_async (its ring must be part of SM).
-template <typename T, int MB, bool ASYNC, class SM>
-__device__ __forceinline__ void grouped_small(const View3& v, int flags, int64_t local, SM& sm)
+template <typename T>
+union SmallSmem {
+    ColvecAsyncSmem<T, 16> cola;
+    RowdotSmem<T, 16> row;
+};
+
+// One small-m work item: 256 rows of contiguous fibres, or of one strided fibre per lane.
+template <typename T, int MB>
+__device__ __forceinline__ void grouped_small(const View3& v, int flags, int64_t local, SmallSmem<T>& sm)
 {
-    constexpr int RV = 16 / sizeof(T);
-    auto& col = reinterpret_cast<ColvecSmem<T, MB>&>(sm.col);
     auto& row = reinterpret_cast<RowdotSmem<T, MB>&>(sm.row);
     if (flags & 1) {
         if (flags & 2) rowdot_tile<T, MB, true>(v, local * 256, row);
         else rowdot_tile<T, MB, false>(v, local * 256, row);
     } else {
-        if (!ASYNC && (flags & 2)) colvec_tile<T, MB, RV, 1>(v, local * kColWarps * 32 * RV, col);
-        else if constexpr (ASYNC) colvec_async_tile<T, MB, 1>(v, local * kColWarps * 32, reinterpret_cast<ColvecAsyncSmem<T, MB>&>(sm.cola));
-        else colvec_tile<T, MB, 1, 1>(v, local * kColWarps * 32, col);
+        colvec_async_tile<T, MB, 1>(v, local * kColWarps * 32, reinterpret_cast<ColvecAsyncSmem<T, MB>&>(sm.cola));
     }
 }
 
@@ -854,13 +855,6 @@ __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __rest
     }
 }
 
-template <typename T>
-union SmallSmem {
-    ColvecSmem<T, 16> col;
-    ColvecAsyncSmem<T, 16> cola;
-    RowdotSmem<T, 16> row;
-};
-
 // Grouped launch of small-m problems only: the same work items as grouped_kernel's small-m ones,
 // without the slice-GEMM's registers and shared memory, so that more blocks share an SM (their
 // loads in flight are what these bandwidth-bound items need). Measured against one launch per
@@ -892,11 +886,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) grouped_small_ker
         v.inner = g.inner;
         v.m = g.m;
         v.b_cm = g.b_cm;
-        if (g.m <= 1) grouped_small<T, 1, kColAsync>(v, g.flags, local, sm);
-        else if (g.m <= 2) grouped_small<T, 2, kColAsync>(v, g.flags, local, sm);
-        else if (g.m <= 4) grouped_small<T, 4, kColAsync>(v, g.flags, local, sm);
-        else if (g.m <= 8) grouped_small<T, 8, kColAsync>(v, g.flags, local, sm);
-        else grouped_small<T, 16, kColAsync>(v, g.flags, local, sm);
+        if (g.m <= 1) grouped_small<T, 1>(v, g.flags, local, sm);
+        else if (g.m <= 2) grouped_small<T, 2>(v, g.flags, local, sm);
+        else if (g.m <= 4) grouped_small<T, 4>(v, g.flags, local, sm);
+        else if (g.m <= 8) grouped_small<T, 8>(v, g.flags, local, sm);
+        else grouped_small<T, 16>(v, g.flags, local, sm);
         __syncthreads();
     }
 }
@@ -1055,7 +1049,7 @@ cudaError_t colvec_dispatch_ls(const View3& v, cudaStream_t s)
     dim3 grid((unsigned)ceil_div(M, (kColWarps / LS) * 32 * W)), block(256);
 #define TLIBTTM_COLVEC(MBv)                                                                \
     do {                                                                                   \
-        if (W == 1 && kColAsync) colvec_async_kernel<T, MBv, LS><<<grid, block, 0, s>>>(v); \
+        if (W == 1) colvec_async_kernel<T, MBv, LS><<<grid, block, 0, s>>>(v); \
         else colvec_kernel<T, MBv, W, LS><<<grid, block, 0, s>>>(v);                       \
     } while (0)
     if (v.m <= 1) TLIBTTM_COLVEC(1);

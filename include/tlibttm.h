@@ -51,7 +51,7 @@ enum tlibttm_dtype {
 
 /*
  * Arithmetic used for the contraction.
- *  PLAIN   exact IEEE FMA in the I/O type (FP32 FFMA / FP64 DFMA). Default.
+ *  PLAIN   exact IEEE FMA in the I/O type (FP32 FFMA / FP64 DFMA or FP64 mma). Default.
  *  BF16X3  float only: each FP32 operand is split into bf16 hi + lo parts and
  *          hi*hi + hi*lo + lo*hi run on the tcgen05 tensor cores with FP32
  *          accumulation in TMEM.
@@ -62,7 +62,7 @@ enum tlibttm_dtype {
  *          FP64 recombination.
  *  AUTO    the library picks per problem (tuned choice among the exact and
  *          the FP32-accurate paths; never FP8).
- * Small-m problems (bandwidth-bound) always run the PLAIN bandwidth kernels.
+ * Small-m problems (m <= 16, bandwidth-bound) always run PLAIN kernels.
  */
 enum tlibttm_precision {
     TLIBTTM_PREC_DEFAULT = 0,
@@ -142,7 +142,7 @@ int tlibttm_ttm_f32_bf16x3_noalloc(unsigned q, unsigned p,
  */
 enum tlibttm_schedule {
     TLIBTTM_SCHED_HEURISTIC = 0,   /* the planner's built-in choice (as tlibttm_ttm_ex, PLAIN) */
-    TLIBTTM_SCHED_SIMT_GEMM = 1,   /* slice-GEMM on FFMA/DFMA, any m */
+    TLIBTTM_SCHED_SIMT_GEMM = 1,   /* slice-GEMM on FFMA / FP64 mma, any m */
     TLIBTTM_SCHED_COLS = 2,        /* small-m kernel for strided fibres, rows spread over warps (m <= 16, inner >= 2) */
     TLIBTTM_SCHED_COLS_SPLIT = 3,  /* small-m kernel for strided fibres, l split over 8 warps (m <= 16, inner >= 2) */
     TLIBTTM_SCHED_ROWS = 4,        /* small-m kernel for contiguous fibres (m <= 16, q == pia[0]) */
@@ -151,7 +151,7 @@ enum tlibttm_schedule {
                                       contiguous fibres of >= 16 floats / 8 doubles on 16-byte boundaries */
     TLIBTTM_SCHED_TC_BF16X3_PAIR = 7, /* tensor-core bf16x3 on pairs of SMs with B in tensor memory, float only
                                       (128 < m <= 256, n_q <= 256; inner >= 128 or q == pia[0]) */
-    TLIBTTM_SCHED_SIMT_SPLIT = 8,  /* slice-GEMM on FFMA/DFMA with its l loop split over blocks whatever the tile
+    TLIBTTM_SCHED_SIMT_SPLIT = 8,  /* slice-GEMM on FFMA / FP64 mma with its l loop split over blocks whatever the tile
                                       count (n_q >= 2048); a fixed-order second kernel adds the parts */
     TLIBTTM_SCHED_BVEC = 9,        /* few output rows (outer * inner <= 8), 16 < m <= 256, n_q >= 4096: B streamed
                                       by the whole GPU, l split over blocks, fixed-order reduction */
@@ -230,7 +230,7 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
                             unsigned flags, tlibttm_plan** plan);
 
 /*
- * Chain plan (Tucker projection, ttmpy.ttms): C = A x_{modes[0]} B_0 x_{modes[1]} B_1 ... in
+ * Chain plan (Tucker projection): C = A x_{modes[0]} B_0 x_{modes[1]} B_1 ... in
  * the given order. A has order p, extents na and layout pia (dense); B_s has shape
  * (ms[s], n) with n the current extent of mode modes[s] and layout pibs[2s..2s+1];
  * every intermediate and C are dense with layout pia. Intermediates live in

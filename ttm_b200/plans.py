@@ -129,7 +129,7 @@ class BatchPlan(_Plan):
 
 
 class ChainPlan(_Plan):
-    """C = A x_{modes[0]} Bs[0] x_{modes[1]} Bs[1] ... (Tucker projection, ttmpy.ttms).
+    """C = A x_{modes[0]} Bs[0] x_{modes[1]} Bs[1] ... (Tucker projection).
 
     A: dense torch CUDA tensor with mode extents ``na`` and layout ``pia``; Bs[s] of shape
     (m_s, current extent of mode modes[s]), row-major; C preallocated with the final extents."""

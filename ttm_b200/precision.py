@@ -5,7 +5,7 @@
 A is order 4 with extents (S, S, S, S), first-order layout, contracted on each q = 1..4 with a
 column-major B of shape (m, S). Two data sets: entries N(0,1), and magnitudes log-uniform on
 [1e-4, 1e4] with random signs. The FP64 input (seeded, on the device) runs through the plain
-FP64 kernel (the oracle: exact DFMA) and through the ozaki path; its FP32 copy runs through the
+FP64 kernel (the oracle: exact FMA chains) and through the ozaki path; its FP32 copy runs through the
 plain FP32, bf16x3 and fp8 paths. For every path and case the study reports
 
     max_rel = max|c - r| / max|r|        (relative error in the infinity norm)

@@ -55,3 +55,21 @@ def test_random_entries(cuda, outer, nq, inner, m):
     want = np.einsum("kli,jl->kji", a.astype(np.longdouble), b.astype(np.longdouble)).astype(np.float64)
     got = _run(cuda, a, b)
     assert np.linalg.norm(got - want) / np.linalg.norm(want) <= 1e-12
+
+
+@pytest.mark.parametrize("outer,nq,inner,m", [(3, 70, 43, 20), (129, 70, 1, 33)])
+def test_non_finite_entries(cuda, outer, nq, inner, m):
+    """A NaN of either sign has zero digits; an infinity spoils its own fibre only."""
+    rng = np.random.default_rng(2)
+    a = rng.integers(-1000, 1001, (outer, nq, inner)).astype(np.float64)
+    b = rng.integers(-1000, 1001, (m, nq)).astype(np.float64)
+    nan = rng.random(a.shape) < 0.1
+    want = np.einsum("kli,jl->kji", np.where(nan, 0.0, a), b)
+    bad = np.where(nan, np.where(rng.random(a.shape) < 0.5, np.nan, -np.nan), a)
+    assert np.array_equal(_run(cuda, bad, b), want)
+    bad[1, 7, 0] = np.inf
+    bad[2, 9, 0] = -np.inf
+    got = _run(cuda, bad, b)
+    keep = np.ones((outer, 1, inner), bool)
+    keep[1, 0, 0] = keep[2, 0, 0] = False
+    assert np.array_equal(np.where(keep, got, 0.0), np.where(keep, want, 0.0))

@@ -127,6 +127,7 @@ struct Digits {
     {
         const bool fast = sh >= -1022 && sh <= 1023;
         const double sc = fast ? pow2d(sh) : 1.0;
+        uint32_t big = 0;
 #pragma unroll
         for (int t = 0; t < 16; ++t) {
             // exact scaling; adding 2^52 with rounding toward zero leaves the truncated integer in
@@ -135,6 +136,17 @@ struct Digits {
             const unsigned long long b = (unsigned long long)__double_as_longlong(__dadd_rz(y, 0x1p52));
             lo[t] = (uint32_t)b & 0xfffffffu;
             hi[t] = (uint32_t)(b >> 28) & 0x1fffffu;
+            big |= (uint32_t)(b >> 32) ^ 0x43300000u;   // its exponent is not 2^52's: y >= 2^52 or NaN
+        }
+        if (big >> 20) {
+            // a row with infinities or NaN: the saturating conversion (a NaN has zero digits)
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const long long i = __double2ll_rz(fast ? x[t] * sc : ldexp(x[t], sh));
+                const unsigned long long b = i < 0 ? 0ull - (unsigned long long)i : (unsigned long long)i;
+                lo[t] = (uint32_t)b & 0xfffffffu;
+                hi[t] = (uint32_t)(b >> 28) & 0x1fffffu;
+            }
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w) {

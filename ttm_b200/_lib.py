@@ -90,6 +90,7 @@ _SZ_ARRAYS = [C.c_size_t * max(n, 1) for n in range(33)]   # orders up to 32
 
 def sz(v):
     """A C size_t[] holding the integers of v."""
+    v = v if hasattr(v, "__len__") else list(v)
     n = len(v)
     arr = _SZ_ARRAYS[n] if n < 33 else C.c_size_t * n
     try:

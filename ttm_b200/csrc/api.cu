@@ -253,7 +253,14 @@ int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t s
         // TMA-fed row mode measured 0.87-0.88 of HBM against 0.65-0.72 at m = 8).
         const int64_t a_bytes = v.outer * v.nq * v.inner * (x.dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= stream_min_bytes && stream_supported(v, x.dtype);
-        if (small_m_takes_gemm(v, x.dtype, tma))
+        const SmallGemm gemm = small_m_takes_gemm(v, x.dtype, tma);
+        if (gemm == SmallGemm::Split) {
+            int n = 1;
+            const cudaError_t e = launch_simt_gemm(v, x.dtype, s, &n, true);
+            if (e == cudaSuccess && n > 1) g_launches += (unsigned long long)(n - 1);   // the reduction
+            return note_launch(e, K_SIMT_GEMM);
+        }
+        if (gemm == SmallGemm::Whole)
             return note_launch(launch_simt_gemm(v, x.dtype, s, nullptr, false, false), K_SIMT_GEMM);
         // Few rows (outer * inner <= 8) and a long l range the TMA kernel does not take: the
         // column and row kernels would run a block or two; the l range goes over the GPU instead.
@@ -632,7 +639,8 @@ int launches_of(const Single& sg, int dtype, int precision)
         const View3& v = sg.pl.v;
         const int64_t a_bytes = v.outer * v.nq * v.inner * (dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= kPlanStreamMinBytes && stream_supported(v, dtype);
-        if (small_m_takes_gemm(v, dtype, tma)) return 1;
+        const SmallGemm gemm = small_m_takes_gemm(v, dtype, tma);
+        if (gemm != SmallGemm::No) return gemm == SmallGemm::Split ? 2 : 1;
         return (!tma && bvec_small_supported(v)) ? 2 : 1;
     }
     int pr = precision == TLIBTTM_PREC_DEFAULT ? g_precision.load() : precision;

@@ -121,8 +121,9 @@ const char* kernel_name(int id);
 cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr,
                              bool force_split = false, bool may_split = true);
 // m <= kSmallM: whether the slice-GEMM is the faster choice against the small-m kernels (`tma`: the
-// TMA-fed one would take the problem).
-bool small_m_takes_gemm(const View3& v, int dtype, bool tma);
+// TMA-fed one would take the problem), in one launch or with its l range split (two).
+enum class SmallGemm { No, Whole, Split };
+SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma);
 int simt_gemm_launch_count(const View3& v, int dtype);
 // Few output rows (outer * inner <= 8), 16 < m <= 256, n_q >= 4096: a kernel that streams B with
 // the l range split over the GPU, then a fixed-order reduction (*launches = 2).

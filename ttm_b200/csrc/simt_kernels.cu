@@ -16,6 +16,7 @@
 //
 // All index arithmetic is 64-bit (a 256^4 tensor has 2^32 elements).
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1462,6 +1463,8 @@ cudaError_t bvec_dispatch(const View3& v, int sms, cudaStream_t s, int* launches
     return e;
 }
 
+constexpr int64_t kMaxSplit = 256, kSplitChainF32 = 1024;
+
 // Parts of the K loop for a slice-GEMM whose tiles cannot fill the GPU (1 when none is needed).
 // `force` (a tuner's schedule): split whenever n_q >= 2048, into enough parts for two rounds of
 // blocks.
@@ -1475,13 +1478,32 @@ int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
     if (v.nq < 2048 || (!force && tiles * 2 > slots)) return 1;
     int64_t S = std::min<int64_t>(ceil_div(slots, tiles), v.nq / 1024);
     if (force) S = std::max<int64_t>(2, std::min<int64_t>(ceil_div(2 * slots, tiles), v.nq / 1024));
-    S = std::min<int64_t>(S, 256);
+    if (sizeof(T) == 4 && v.m <= kSmallM) S = std::max<int64_t>(S, ceil_div(v.nq, kSplitChainF32));
+    S = std::min<int64_t>(S, kMaxSplit);
     // workspace of S partial results at most 1 GiB
     const int64_t nc = v.outer * v.m * v.inner;
     while (S > 1 && S * nc * (int64_t)sizeof(T) > (int64_t(1) << 30)) --S;
     if (S <= 1) return 1;
     lper = ceil_div(ceil_div(v.nq, S), BK) * BK;
     return (int)ceil_div(v.nq, lper);
+}
+
+// Workspaces come from the stream-ordered pool, which by default hands its memory back to the driver
+// at every synchronisation (a call after one then took 200 us more): up to 64 MB stay cached. The
+// paths with larger scratch keep all of theirs.
+void keep_small_workspaces(cudaStream_t s)
+{
+    static std::atomic<uint64_t> done{0};   // bit per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || (done.load() >> dev & 1)) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
+    cudaMemPool_t pool;
+    uint64_t now = 0, want = uint64_t(64) << 20;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &now) == cudaSuccess && now < want)
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want);
+    done.fetch_or(uint64_t(1) << dev);
 }
 
 template <typename T>
@@ -1496,6 +1518,7 @@ cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool
     if (S <= 1) return simt_gemm_dispatch(v, s, 1, 0, static_cast<T*>(nullptr));
     const int64_t nc = v.outer * v.m * v.inner;
     T* ws = nullptr;
+    keep_small_workspaces(s);
     if ((e = dev_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess) return e;
     e = simt_gemm_dispatch(v, s, S, lper, ws);
     if (e == cudaSuccess) {
@@ -1528,20 +1551,53 @@ cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* lau
 //             contiguous fibres on 16-byte boundaries 1.05-1.4 from n_q = 64, off them 1.4-10 at
 //             n_q = 2001 and 0.93-2.0 at 250
 //   m <= 8    mostly 0.6-1.1
-// Few row tiles leave the GPU idle: long contiguous fibres then go to the l-split kernels, strided
-// rows to the column kernel's l split (0.8-0.9 below about 16 tiles of 128 rows).
-bool small_m_takes_gemm(const View3& v, int dtype, bool tma)
+// Few row tiles leave the GPU idle. From n_q = 2048 on the l range is then split over more blocks
+// (two launches) where the tiles come to less than 1.7 blocks an SM, as time of the kernel otherwise
+// taken over time of the split tile, A of 2^21 elements and more:
+//   l-split kernels (long fibres, very long strided ranges): 1.4-3.5 from 32 to 2048 rows, 3.6-25
+//             beyond, any m; of unsplit tiles with n_q 1024-2047 2.2-6 from 16 tiles on
+//   TMA-fed kernels, m 9..16: 1.0-1.5 float, 1.3-3.2 double (unsplit 0.3-0.9), fibres of double m 5..8
+//             1.0-1.3; at most 128 rows leave its stages of 512 fibres empty: 1.4-12 (float, m 5..8
+//             1.3 at 512 rows)
+//   column kernel: double m 5..8 3.4-6, float m 9..16 2.1-5.4; m below that, to 8192 rows 1.7-4
+// Float keeps to ranges whose parts are at most kSplitChainF32 l long, and splits whatever the block
+// count in place of the l-split kernels: a chain of 1024 FMAs is 5.7e-7 off (relative, N(0,1)
+// entries), the chains of the kernels it replaces 1e-7 to 6e-7.
+// Shorter ranges of few tiles keep to the TMA-fed kernel (m 9..16: 0.5-0.8 at 64 blocks, 1.1 at 128; m
+// 5..8 0.9 at 128, 1.1 at 256), or to the l-split kernels and the column kernel's l split (0.8-0.9
+// below about 16 tiles of 128 rows).
+SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma)
 {
-    const int64_t tiles = ceil_div(v.outer * v.inner, kGemmRows);
-    const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % (dtype == 0 ? 4 : 2) == 0;
-    if (dtype == 0) {
-        if (v.m <= 8) return false;
-        if (v.inner == 1) return v.nq >= (vec ? 64 : 512) && (v.nq < 1024 || tiles >= 16);
-        return tiles >= 32 && v.nq >= 64 && v.inner >= 64;
+    int sms = 0;
+    if (sms_of_device(sms) != cudaSuccess) return SmallGemm::No;
+    const int64_t rows = v.outer * v.inner, tiles = ceil_div(rows, kGemmRows);
+    const bool f64 = dtype != 0, fibres = v.inner == 1;
+    const bool vec = aligned16(v.a) && (fibres ? v.nq : v.inner) % (f64 ? 2 : 4) == 0;
+    const int64_t blocks = ceil_div(rows, f64 && vec ? kGemmRows / 2 : kGemmRows);
+    const bool lsplit = !tma && bvec_small_supported(v);   // the l-split kernels would take it
+    const bool few = 10 * blocks < 17 * sms;
+    if ((few || (lsplit && !f64)) && v.nq >= 2048 && (f64 || v.nq <= kSplitChainF32 * kMaxSplit) && rows > kBvecMaxR &&
+        rows * v.nq >= (int64_t(1) << 21)) {
+        bool take = lsplit;
+        if (fibres) take = take || v.m > (f64 ? 4 : 8) || rows <= (v.m > 4 ? 4 : 1) * kGemmRows;
+        else if (f64) take = take || v.m > 8 || (!tma && (v.m > 4 || tiles <= 64));
+        else take = take || (v.inner >= 64 && (v.m > 8 || (!tma && tiles <= 64)));
+        if (take) return SmallGemm::Split;
     }
-    if (v.inner == 1) return v.nq > (v.m > 8 ? kFlatMaxNq : 127) && (v.nq < 1024 || tiles >= 16) && (v.m > 4 || !tma);
-    if (v.m > 8) return tiles >= 16 && v.nq >= (vec ? 12 : 32);
-    return tiles >= 128 && v.nq >= 128 && (v.m > 4 || !vec);
+    if (tma && (v.m > 8 ? 20 * blocks < 17 * sms : few)) return SmallGemm::No;
+    bool take;
+    if (dtype == 0) {
+        if (v.m <= 8) take = lsplit && tiles >= 16;
+        else if (v.inner == 1) take = v.nq >= (vec ? 64 : 512) && (v.nq < 1024 || tiles >= 16);
+        else take = tiles >= 32 && v.nq >= 64 && v.inner >= 64;
+    } else if (v.inner == 1) {
+        take = v.nq > (v.m > 8 ? kFlatMaxNq : 127) && (v.nq < 1024 || tiles >= 16) && (v.m > 4 || !tma);
+    } else if (v.m > 8) {
+        take = tiles >= 16 && v.nq >= (vec ? 12 : 32);
+    } else {
+        take = tiles >= 128 && v.nq >= 128 && (v.m > 4 || !vec);
+    }
+    return take ? SmallGemm::Whole : SmallGemm::No;
 }
 
 int simt_gemm_launch_count(const View3& v, int dtype)

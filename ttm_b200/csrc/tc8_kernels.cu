@@ -503,8 +503,9 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
                     float y[32];
 #pragma unroll
                     for (int c = 0; c < 32; ++c) y[c] = __uint_as_float(v[c]) * sa * __shfl_sync(0xffffffffu, sb_l, c);
-                    if (P.inner == 1 && j0 + 32 <= P.m && (((cbase + j0) & 3) == 0)) {
-                        // this row's 32 columns are contiguous: 128-bit stores
+                    if (P.inner == 1 && j0 + 32 <= P.m && (reinterpret_cast<uintptr_t>(C + cbase + j0) & 15u) == 0) {
+                        // this row's 32 columns are contiguous, from a 16-byte boundary (C itself may
+                        // lie off one): 128-bit stores
                         if (rv) {
                             float4* cp = reinterpret_cast<float4*>(C + cbase + j0);
 #pragma unroll
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(kThreads8, 1) tc8_kernel(Tc8Params P)
 #pragma unroll
                     for (int c = 0; c < 16; ++c)
                         y[c] = fma((double)Lo[c], 0x1p-28, (double)H[c]) * sa * __shfl_sync(0xffffffffu, sb_l, c);
-                    if (P.inner == 1 && j0 + 16 <= P.m && (((cbase + j0) & 1) == 0)) {
+                    if (P.inner == 1 && j0 + 16 <= P.m && (reinterpret_cast<uintptr_t>(C + cbase + j0) & 15u) == 0) {
                         if (rv) {
                             double2* cp = reinterpret_cast<double2*>(C + cbase + j0);
 #pragma unroll

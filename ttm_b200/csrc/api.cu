@@ -230,7 +230,6 @@ int note_launch(cudaError_t e, int kid)
     return TLIBTTM_OK;
 }
 
-constexpr int64_t kStreamMinBytes = int64_t(64) << 20;
 constexpr int64_t kPlanStreamMinBytes = int64_t(4) << 20;
 
 // All operands are device memory: enqueue on stream s.

@@ -13,6 +13,24 @@ static __device__ __forceinline__ void ffma2(unsigned long long& d, unsigned lon
 {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
+static __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+static __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+static __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 static __device__ __forceinline__ unsigned long long pair_dup(float x)
 {
     unsigned long long r;
@@ -27,6 +45,34 @@ static __device__ __forceinline__ unsigned long long pair_of(float lo, float hi)
 }
 static __device__ __forceinline__ float pair_lo(unsigned long long r) { return __uint_as_float((unsigned)r); }
 static __device__ __forceinline__ float pair_hi(unsigned long long r) { return __uint_as_float((unsigned)(r >> 32)); }
+
+// A running sum s with what its additions rounded off in e (Dekker's fast two-sum, whose order of
+// magnitudes may be wrong here: e then misses a part of a rounding). Where s has left the finite
+// numbers, e is not one either, and the total is s alone, as of plain additions.
+static __device__ __forceinline__ void add_kept(float& s, float& e, float x)
+{
+    const float t = __fadd_rn(s, x);
+    e = __fadd_rn(e, __fsub_rn(x, __fsub_rn(t, s)));
+    s = t;
+}
+static __device__ __forceinline__ void add_kept(double& s, double& e, double x)
+{
+    const double t = __dadd_rn(s, x);
+    e = __dadd_rn(e, __dsub_rn(x, __dsub_rn(t, s)));
+    s = t;
+}
+static __device__ __forceinline__ void add_kept(unsigned long long& s, unsigned long long& e, unsigned long long x)
+{
+    const unsigned long long t = add2(s, x);
+    e = add2(e, sub2(x, sub2(t, s)));
+    s = t;
+}
+static __device__ __forceinline__ float kept_total(float s, float e) { return isfinite(e) ? s + e : s; }
+static __device__ __forceinline__ double kept_total(double s, double e) { return isfinite(e) ? s + e : s; }
+static __device__ __forceinline__ unsigned long long kept_total(unsigned long long s, unsigned long long e)
+{
+    return pair_of(kept_total(pair_lo(s), pair_lo(e)), kept_total(pair_hi(s), pair_hi(e)));
+}
 #endif
 
 // Dense slice view of one mode-q TTM.
@@ -156,6 +202,8 @@ int grouped_blocks_per_sm(int dtype);
 
 // Largest m handled by the small-m bandwidth kernels.
 constexpr int64_t kSmallM = 16;
+// Bytes of A from which a single call takes the TMA-fed small-m kernel.
+constexpr int64_t kStreamMinBytes = int64_t(64) << 20;
 
 __host__ __device__ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -6,7 +6,10 @@
 // its line in shared memory; a line's last copy stops at its end, so that only the elements before a
 // line in its first 16 bytes are read besides it. Lane t holds rows t, t + 32, ... of the tile, so that
 // shared-memory reads hit 32 banks whatever the shift, and all TN columns; the four warps take every
-// fourth l, and their sums are added in a fixed order at the end.
+// fourth l, and their sums are added in a fixed order at the end. Where the column kernel would add up in
+// eight chains per output, one chain per warp was further off (1.9e-7 against 1.4e-7 at n_q = 400,
+// relative to FP64): a warp's l are cut into chains of 8, or 16 from n_q = 128 on (1.0e-7), at 15 or 8 %
+// of the time at m = 8.
 //
 // What bounds it: reading A. The column kernel's copies of one element per lane (colvec_async) took
 // 12 cycles an instruction and SM and held it to 2.7-3.1 TB/s; the slice-GEMM tile reads each
@@ -43,9 +46,10 @@ __device__ __forceinline__ void copy4(void* dst, const void* src, bool ok)
                  : "memory");
 }
 
-// Tile `t` of outer * ceil(inner / 256).
+// Tile `t` of outer * ceil(inner / 256). A warp's chains are `chain` + 1 stages (a power of two) of four l
+// of its own.
 template <int TN, bool BCM>
-__device__ __forceinline__ void tile(const View3& v, int64_t t, Smem<TN>& sm)
+__device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<TN>& sm)
 {
     const float* __restrict__ A = static_cast<const float*>(v.a);
     const float* __restrict__ B = static_cast<const float*>(v.b);
@@ -85,11 +89,11 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, Smem<TN>& sm)
     // this warp's l (warp, warp + 4, ...) all have one residue mod 4, and so one shift: BK inner and
     // BM are multiples of four
     const int sh = (int)((((uint32_t)k * (uint32_t)nq + (uint32_t)warp) * (uint32_t)inner) & 3u);
-    unsigned long long acc[RPL / 2][TN];   // rows 64 p + lane and 64 p + 32 + lane
+    unsigned long long acc[RPL / 2][TN], sum[RPL / 2][TN];   // rows 64 p + lane and 64 p + 32 + lane
 #pragma unroll
     for (int p = 0; p < RPL / 2; ++p)
 #pragma unroll
-        for (int q = 0; q < TN; ++q) acc[p][q] = 0ull;
+        for (int q = 0; q < TN; ++q) acc[p][q] = sum[p][q] = 0ull;
     int rd = 0, wr = ST - 1;
     const int nk = (int)ceil_div(nq, BK);
     for (int kt = 0; kt < nk; ++kt) {
@@ -113,6 +117,15 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, Smem<TN>& sm)
                 for (int p = 0; p < RPL / 2; ++p) ffma2(acc[p][q], a[p], bq);
             }
         }
+        if ((kt & chain) == chain || kt + 1 == nk) {   // a chain ends
+#pragma unroll
+            for (int p = 0; p < RPL / 2; ++p)
+#pragma unroll
+                for (int q = 0; q < TN; ++q) {
+                    sum[p][q] = add2(sum[p][q], acc[p][q]);
+                    acc[p][q] = 0ull;
+                }
+        }
         rd = rd + 1 == ST ? 0 : rd + 1;
         wr = wr + 1 == ST ? 0 : wr + 1;
     }
@@ -127,8 +140,8 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, Smem<TN>& sm)
         for (int q = 0; q < QC; ++q)
 #pragma unroll
             for (int p = 0; p < RPL / 2; ++p) {
-                sm.red[warp][q][64 * p + lane] = pair_lo(acc[p][q0 + q]);
-                sm.red[warp][q][64 * p + 32 + lane] = pair_hi(acc[p][q0 + q]);
+                sm.red[warp][q][64 * p + lane] = pair_lo(sum[p][q0 + q]);
+                sm.red[warp][q][64 * p + 32 + lane] = pair_hi(sum[p][q0 + q]);
             }
         __syncthreads();
 #pragma unroll

@@ -1,5 +1,6 @@
 // FP32 slice-GEMM on packed FFMA pairs: every output is one chain of correctly rounded fused
-// multiply-adds in the order of l.
+// multiply-adds in the order of l (tiles of 128 rows and at most 16 columns: chains of eight, added up in
+// two more levels).
 //
 // One tile is 32 TM rows (flattened (k, i) pairs) x TX TN columns j; 32 x TX threads (TX 8 or 4), each
 // TM x TN outputs. Accumulators pair neighbouring rows, which come from shared memory as 64-bit
@@ -81,18 +82,55 @@ __device__ __forceinline__ void load_columns(float (&b)[TN], const float (&sb)[B
     if constexpr (TN & 1) b[TN - 1] = sb[column<TX, TN>(TN - 1, tx)];
 }
 
+// Tiles of 128 rows and at most 16 columns (FOLD) add up in levels: chains of kFoldChain l in acc, their sums over
+// kFoldStages stages in mid, and those in sum with what the additions round off in err. The kernels that
+// they take problems from add up in several shorter chains (eight, or chains of 32 in the l-split
+// kernels), which one chain of n_q would be further off than. Relative error against FP64, N(0,1)
+// entries: one chain 1.4e-7 at n_q = 64, 5.7e-7 at 1024, 1.6e-6 at 8000; the kernels replaced 0.8e-7
+// to 4.1e-7; these levels 0.8e-7 to 1.0e-7 at any n_q. They want 128 registers: at 96 (five blocks
+// an SM) they took 37 us on 4096 rows of i, n_q = 1024, m = 16 in place of 31 (one chain: 29).
+constexpr int kFoldChain = 8, kFoldStages = 8;
+
 // A thread's outputs where rows of i are contiguous: acc[p][q] holds rows 2 p and 2 p + 1 of its TM
 // (chunks of four rows 128 apart), column q.
-template <int TX, int TM, int NA>
+template <int TX, int TM, int NA, bool FOLD>
 struct AccRows {
     unsigned long long acc[TM / 2][NA];
+    static constexpr int FP = FOLD ? TM / 2 : 1, FQ = FOLD ? NA : 1;
+    unsigned long long mid[FP][FQ], sum[FP][FQ], err[FP][FQ];
 
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
         for (int p = 0; p < TM / 2; ++p)
 #pragma unroll
-            for (int q = 0; q < NA; ++q) acc[p][q] = 0ull;
+            for (int q = 0; q < NA; ++q) {
+                acc[p][q] = 0ull;
+                if constexpr (FOLD) mid[p][q] = sum[p][q] = err[p][q] = 0ull;
+            }
+    }
+
+    // FOLD: the sum of kFoldStages stages goes into the total
+    __device__ __forceinline__ void fold()
+    {
+#pragma unroll
+        for (int p = 0; p < TM / 2; ++p)
+#pragma unroll
+            for (int q = 0; q < NA; ++q) {
+                add_kept(sum[p][q], err[p][q], mid[p][q]);
+                mid[p][q] = 0ull;
+            }
+    }
+
+    __device__ __forceinline__ void finish()
+    {
+#pragma unroll
+        for (int p = 0; p < TM / 2; ++p)
+#pragma unroll
+            for (int q = 0; q < NA; ++q) {
+                add_kept(sum[p][q], err[p][q], mid[p][q]);
+                acc[p][q] = kept_total(sum[p][q], err[p][q]);
+            }
     }
 
     // one stage (16 l)
@@ -115,7 +153,12 @@ struct AccRows {
 #pragma unroll
             for (int p = 0; p < TM / 2; ++p)
 #pragma unroll
-                for (int q = 0; q < TN; ++q) ffma2(acc[p][q], a[p], bq[q]);
+                for (int q = 0; q < TN; ++q) {
+                    if (FOLD && kk % kFoldChain == 0) acc[p][q] = mul2(a[p], bq[q]);
+                    else ffma2(acc[p][q], a[p], bq[q]);
+                    if constexpr (FOLD)
+                        if (kk % kFoldChain == kFoldChain - 1) mid[p][q] = add2(mid[p][q], acc[p][q]);
+                }
         }
     }
 
@@ -166,18 +209,54 @@ struct AccRows {
 
 // A thread's outputs where fibres are contiguous: rows 32 apart, acc[r][p] holds columns 2 p and
 // 2 p + 1 of row r, last[r] the column left over. A's rows come four l at a time.
-template <int TX, int TM, int NA>
+template <int TX, int TM, int NA, bool FOLD>
 struct AccFibres {
-    unsigned long long acc[TM][NA / 2 > 0 ? NA / 2 : 1];
+    static constexpr int NP = NA / 2;   // column pairs
+    unsigned long long acc[TM][NP > 0 ? NP : 1];
     float last[TM];
+    static constexpr int FR = FOLD ? TM : 1;
+    unsigned long long mid[FR][NP > 0 ? NP : 1], sum[FR][NP > 0 ? NP : 1], err[FR][NP > 0 ? NP : 1];
+    float mid_last[FR], sum_last[FR], err_last[FR];
 
     __device__ __forceinline__ void clear()
     {
 #pragma unroll
         for (int r = 0; r < TM; ++r) {
 #pragma unroll
-            for (int p = 0; p < (NA / 2 > 0 ? NA / 2 : 1); ++p) acc[r][p] = 0ull;
+            for (int p = 0; p < NP; ++p) {
+                acc[r][p] = 0ull;
+                if constexpr (FOLD) mid[r][p] = sum[r][p] = err[r][p] = 0ull;
+            }
             last[r] = 0.0f;
+            if constexpr (FOLD) mid_last[r] = sum_last[r] = err_last[r] = 0.0f;
+        }
+    }
+
+    __device__ __forceinline__ void fold()
+    {
+#pragma unroll
+        for (int r = 0; r < TM; ++r) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                add_kept(sum[r][p], err[r][p], mid[r][p]);
+                mid[r][p] = 0ull;
+            }
+            add_kept(sum_last[r], err_last[r], mid_last[r]);
+            mid_last[r] = 0.0f;
+        }
+    }
+
+    __device__ __forceinline__ void finish()
+    {
+#pragma unroll
+        for (int r = 0; r < TM; ++r) {
+#pragma unroll
+            for (int p = 0; p < NP; ++p) {
+                add_kept(sum[r][p], err[r][p], mid[r][p]);
+                acc[r][p] = kept_total(sum[r][p], err[r][p]);
+            }
+            add_kept(sum_last[r], err_last[r], mid_last[r]);
+            last[r] = kept_total(sum_last[r], err_last[r]);
         }
     }
 
@@ -197,9 +276,21 @@ struct AccFibres {
                 for (int r = 0; r < TM; ++r) {
                     const float x = kk == 0 ? a[r].x : a[r].y;
                     const unsigned long long xx = pair_dup(x);
+                    const bool open = FOLD && (k2 + kk) % kFoldChain == 0;
+                    const bool close = FOLD && (k2 + kk) % kFoldChain == kFoldChain - 1;
 #pragma unroll
-                    for (int p = 0; p < TN / 2; ++p) ffma2(acc[r][p], xx, pair_of(b[2 * p], b[2 * p + 1]));
-                    if constexpr (TN & 1) last[r] = __fmaf_rn(x, b[TN - 1], last[r]);
+                    for (int p = 0; p < TN / 2; ++p) {
+                        const unsigned long long bp = pair_of(b[2 * p], b[2 * p + 1]);
+                        if (open) acc[r][p] = mul2(xx, bp);
+                        else ffma2(acc[r][p], xx, bp);
+                        if constexpr (FOLD)
+                            if (close) mid[r][p] = add2(mid[r][p], acc[r][p]);
+                    }
+                    if constexpr (TN & 1) {
+                        last[r] = open ? __fmul_rn(x, b[TN - 1]) : __fmaf_rn(x, b[TN - 1], last[r]);
+                        if constexpr (FOLD)
+                            if (close) mid_last[r] = __fadd_rn(mid_last[r], last[r]);
+                    }
                 }
             }
         }
@@ -243,6 +334,8 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
                                       Smem<TX, TM, TN, ST, AK>& sm, int64_t l_begin, int64_t l_end)
 {
     constexpr int BM = 32 * TM, BN = TX * TN, NT = 32 * TX;
+    constexpr bool FOLD = TM == 4 && TX * TN <= 16;
+    static_assert(!FOLD || EXACT, "the narrower widths of an inexact build are not folded");
     const float* __restrict__ A = static_cast<const float*>(v.a);
     const float* __restrict__ B = static_cast<const float*>(v.b);
     const int64_t inner = v.inner, m = v.m, nq = v.nq;
@@ -331,7 +424,7 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     const int nk = (int)ceil_div(l_end - l_begin, BK);
 
     for (int64_t t = first; t < last; t += step) {
-        typename std::conditional<AK, AccFibres<TX, TM, TN>, AccRows<TX, TM, TN>>::type out;
+        typename std::conditional<AK, AccFibres<TX, TM, TN, FOLD>, AccRows<TX, TM, TN, FOLD>>::type out;
         out.clear();
         for (int kt = 0; kt < nk; ++kt) {
             asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
@@ -339,6 +432,8 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
             load_next(wr);
             if constexpr (EXACT) {
                 out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx);
+                if constexpr (FOLD)
+                    if (kt % kFoldStages == kFoldStages - 1) out.fold();
             } else {
                 if (gr.nf > 6) out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx);
                 else if (gr.nf > 4) out.template stage<6>(sm.a[rd], sm.b[rd], ty, tx);
@@ -347,6 +442,7 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
             rd = rd + 1 == ST ? 0 : rd + 1;
             wr = wr + 1 == ST ? 0 : wr + 1;
         }
+        if constexpr (FOLD) out.finish();
         const int64_t rt = gr.cols == 1 ? t : slice_of(t, gr.cols);
         const int64_t n0 = (t - rt * gr.cols) * gr.nf * TX;
         if constexpr (EXACT) {

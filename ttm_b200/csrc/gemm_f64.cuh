@@ -41,6 +41,14 @@ __device__ __forceinline__ void mma(double (&c)[2], double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// The first of a chain: c = a b.
+__device__ __forceinline__ void mma_open(double (&c)[2], double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+                 : "=d"(c[0]), "=d"(c[1])
+                 : "d"(a), "d"(b), "d"(0.0));
+}
+
 // Copies 16 or 8 bytes; zeroes the destination where !ok (src is then not read).
 __device__ __forceinline__ void copy16(void* dst, const void* src, bool ok)
 {
@@ -55,9 +63,16 @@ __device__ __forceinline__ void copy8(void* dst, const void* src, bool ok)
                  : "memory");
 }
 
+// Builds for m <= 16 that take problems from kernels with several short chains (FOLD, the chains' length;
+// 0: one chain) add up in levels: chains of FOLD l in acc, their sums over kFoldStages stages in mid, and
+// those in sum, for contiguous fibres with what the additions round off in err. One chain of n_q would be
+// further off than the eight chains of the column kernel or the chains of 32 of the l-split kernels
+// (relative error at n_q = 1027: 1.0e-15 against 1.9e-16, 1.6e-16 with FOLD).
+constexpr int kFoldStages = 8;
+
 // One stage (16 l) of a warp's 16 rows x 8 N columns. At most eight columns: two accumulation
-// chains (even and odd l / 4), added by the caller at the end.
-template <int N, bool AK, bool BCM, int AR, int AP, int BR, int BP, int NA>
+// chains (even and odd l / 4), added by the caller. FOLD: new chains, one or two of a stage.
+template <int N, bool AK, bool BCM, int FOLD, int AR, int AP, int BR, int BP, int NA>
 __device__ __forceinline__ void stage(const double (&sa)[AR][AP], const double (&sb)[BR][BP], int warp, int g, int c,
                                       double (&acc)[2][NA][2])
 {
@@ -77,9 +92,14 @@ __device__ __forceinline__ void stage(const double (&sa)[AR][AP], const double (
 #pragma unroll
             for (int f = 0; f < N; ++f) {
                 const double b = BCM ? sb[kk + c][8 * f + g] : sb[8 * f + g][kk + c];
-                const int to = N == 1 ? (kk >> 2) & 1 : f;
-                mma(acc[0][to], a0, b);
-                mma(acc[1][to], a1, b);
+                const int to = N == 1 ? (kk >> 2) & 1 : FOLD == 8 ? f + kk / 8 * N : f;
+                if (FOLD && (N == 1 ? kk < 8 : kk % (FOLD ? FOLD : BK) == 0)) {
+                    mma_open(acc[0][to], a0, b);
+                    mma_open(acc[1][to], a1, b);
+                } else {
+                    mma(acc[0][to], a0, b);
+                    mma(acc[1][to], a1, b);
+                }
             }
         }
     }
@@ -89,11 +109,14 @@ __device__ __forceinline__ void stage(const double (&sa)[AR][AP], const double (
 // consecutive tiles follow one another through the ring, so that the next tile's loads are in
 // flight while this one's results are stored. VEC: 16-byte copies of A (alignment checked by the
 // host). The caller synchronises the block between two calls that share `sm`.
-template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, bool EXACT>
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, bool EXACT, int FOLD>
 __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t step, int64_t last, const ColumnGrid& gr,
                                       Smem<BM, NF, ST, AK, BCM>& sm, int64_t l_begin, int64_t l_end)
 {
-    constexpr int BN = NF * 8, NT = 2 * BM, NA = NF == 1 ? 2 : NF;
+    constexpr int BN = NF * 8, NT = 2 * BM, NA = NF == 1 || FOLD == 8 ? 2 * NF : NF;
+    constexpr int SETS = FOLD == 8 || NF == 1 ? 2 : 1;   // chains of an output in a stage
+    constexpr int NM = FOLD ? NF : 1;
+    static_assert(!FOLD || (EXACT && NF <= 2 && BK % FOLD == 0), "folded builds are narrow and of one width");
     const double* __restrict__ A = static_cast<const double*>(v.a);
     const double* __restrict__ B = static_cast<const double*>(v.b);
     double* __restrict__ C = static_cast<double*>(v.c);
@@ -184,31 +207,74 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     for (int r = 0; r < 2; ++r)
 #pragma unroll
         for (int f = 0; f < NA; ++f) acc[r][f][0] = acc[r][f][1] = 0.0;
+    double mid[2][NM][2], sum[2][NM][2], err[2][NM][2];
+    // the last stage's chains into mid. Called once the next stage's copies are on their way: right after
+    // the stage the additions would wait for its last mma (43 us against 37 at 4096 rows, n_q = 4096, m = 16)
+    auto close_chains = [&]() {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int f = 0; f < NM; ++f)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    mid[r][f][e] += SETS == 2 ? acc[r][f][e] + acc[r][f + NF < NA ? f + NF : 0][e] : acc[r][f][e];
+    };
+    auto fold = [&]() {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int f = 0; f < NM; ++f)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    if (AK) add_kept(sum[r][f][e], err[r][f][e], mid[r][f][e]);
+                    else sum[r][f][e] += mid[r][f][e];
+                    mid[r][f][e] = 0.0;
+                }
+    };
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int f = 0; f < NM; ++f)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) mid[r][f][e] = sum[r][f][e] = err[r][f][e] = 0.0;
 
     for (int kt = 0; kt < nk; ++kt) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncthreads();   // stage rd has landed for all, and all have read stage wr's last contents
         load_next(wr);
         if constexpr (EXACT) {
-            stage<NF, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc);
+            if constexpr (FOLD != 0) {
+                if (kt > 0) close_chains();
+                if (kt % kFoldStages == 0) fold();
+            }
+            stage<NF, AK, BCM, FOLD>(sm.a[rd], sm.b[rd], warp, g, c, acc);
         } else {
             // one build per width: predicated-off mma would take the pipe as long as executed ones
             switch (nf) {
-            case 1: stage<1, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 2: stage<2, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 3: stage<3, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 4: stage<4, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 5: stage<5, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 6: stage<6, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            case 7: stage<7, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
-            default: stage<NF, AK, BCM>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 1: stage<1, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 2: stage<2, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 3: stage<3, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 4: stage<4, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 5: stage<5, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 6: stage<6, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            case 7: stage<7, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
+            default: stage<NF, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
             }
         }
         rd = rd + 1 == ST ? 0 : rd + 1;
         wr = wr + 1 == ST ? 0 : wr + 1;
     }
 
-    if (nf == 1) {
+    if constexpr (FOLD != 0) {
+        close_chains();
+        fold();
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int f = 0; f < NM; ++f)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) acc[r][f][e] = AK ? kept_total(sum[r][f][e], err[r][f][e]) : sum[r][f][e];
+    } else if (nf == 1) {
 #pragma unroll
         for (int r = 0; r < 2; ++r)
 #pragma unroll

@@ -23,6 +23,7 @@
 #include "few_columns.cuh"
 #include "gemm_f32.cuh"
 #include "gemm_f64.cuh"
+#include "tc_kernels.cuh"
 
 namespace tlibttm {
 namespace {
@@ -88,12 +89,12 @@ __device__ __forceinline__ void split_range(View3& v, int64_t lper, T* ws, int64
     }
 }
 
-// Blocks per SM of the FP32 builds: 16 warps of at most 128 registers, or of 80-100 where the
-// accumulators are small.
-constexpr int ffma_blocks(int TX, int TM) { return TX == 8 ? 2 : TM == 8 ? 4 : 5; }
+// Blocks per SM of the FP32 builds: 16 warps of at most 128 registers, or 20 of 100 where the
+// accumulators are small (and not folded).
+constexpr int ffma_blocks(int TX, int TM, int TN) { return TX == 8 ? 2 : TM == 8 || TN <= 4 ? 4 : 5; }
 
 template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
+__global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM, TN)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
                                                                                int64_t lper, float* ws)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
@@ -103,14 +104,18 @@ __global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM)) ffma_gemm_kernel
                                                    *reinterpret_cast<f32::Smem<TX, TM, TN, ST, AK>*>(gemm_smem), l0, l1);
 }
 
-template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 5) dmma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
+// Blocks per SM of the FP64 builds (tiles of 64 rows of fibres: four by their shared memory; with folded
+// sums by their registers).
+constexpr int dmma_blocks(int BM, bool AK, int FOLD) { return BM == 128 ? 2 : AK || FOLD ? 4 : 5; }
+
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, int FOLD>
+__global__ void __launch_bounds__(2 * BM, dmma_blocks(BM, AK, FOLD)) dmma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
                                                                              int64_t lper, double* ws)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
     int64_t l0, l1;
     split_range(v, lper, ws, l0, l1);
-    f64::tiles<BM, NF, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr,
+    f64::tiles<BM, NF, ST, AK, VEC, BCM, true, FOLD>(v, blockIdx.x, gridDim.x, tiles, gr,
                                                *reinterpret_cast<f64::Smem<BM, NF, ST, AK, BCM>*>(gemm_smem), l0, l1);
 }
 
@@ -123,6 +128,8 @@ __global__ void __launch_bounds__(2 * BM, BM == 128 ? 2 : 5) dmma_gemm_kernel(Vi
 // streams per row chunk (problems with few rows). B is staged in shared memory as [l][MB].
 // ---------------------------------------------------------------------------------------------
 constexpr int kColWarps = 8;
+constexpr int64_t kBvecSmallMaxRows = 65536;   // small m: the l-split kernels' row tiles up to this many rows
+constexpr int64_t kColSplitWarps = 148 * 32;   // fewer warps of rows than this: l split over eight warps
 constexpr int kColUnroll1 = 8;   // l steps unrolled with one scalar row per lane
 
 template <typename T, int MB>
@@ -373,10 +380,10 @@ __global__ void __launch_bounds__(256) colvec_async_kernel(View3 v)
 
 // few_columns.cuh: rows of i off 16-byte boundaries, m <= 8, long l ranges.
 template <int TN, bool BCM>
-__global__ void __launch_bounds__(few::NT, 3) few_columns_kernel(View3 v)
+__global__ void __launch_bounds__(few::NT, 3) few_columns_kernel(View3 v, int chain)
 {
     extern __shared__ __align__(16) unsigned char few_smem[];
-    few::tile<TN, BCM>(v, blockIdx.x, *reinterpret_cast<few::Smem<TN>*>(few_smem));
+    few::tile<TN, BCM>(v, blockIdx.x, chain, *reinterpret_cast<few::Smem<TN>*>(few_smem));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -839,7 +846,7 @@ __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __rest
         const ColumnGrid gr{g.tiles_n, g.cols / 8};
         if constexpr (sizeof(T) == 8) {
 #define TLIBTTM_TILE(AKv, VECv, BCMv)                                                                        \
-    f64::tiles<kGemmRows, kGroupNF, kGroupST, AKv, VECv, BCMv, false>(v, local, 1, local + 1, gr,                    \
+    f64::tiles<kGemmRows, kGroupNF, kGroupST, AKv, VECv, BCMv, false, 0>(v, local, 1, local + 1, gr,                    \
                                                    *reinterpret_cast<f64::Smem<kGemmRows, kGroupNF, kGroupST, AKv, BCMv>*>(grouped_smem), \
                                                    0, v.nq)
             TLIBTTM_TILES
@@ -922,7 +929,7 @@ cudaError_t ffma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, in
     const int64_t tiles = ceil_div(v.outer * v.inner, 32 * TM) * gr.cols;
     // as in dmma_launch (m = 64, n_q = 16, A 64 MB: 86 -> 82 us; n_q = 64: 190 us against 197)
     const bool walk = v.nq <= 2 * f32::BK;
-    const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM);
+    const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM, TN);
     const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
     kernel<<<grid, 32 * TX, smem, s>>>(v, gr, tiles, lper, ws);
     return cudaGetLastError();
@@ -940,15 +947,41 @@ cudaError_t ffma_dispatch_form(const View3& v, cudaStream_t s, const ColumnGrid&
 #undef TLIBTTM_FFMA
 }
 
+// m <= 16: whether the kernels that the slice-GEMM tile replaces add up in one chain per output, so that
+// one chain of its own is no further off. They do not where the range is split here; for rows of i that
+// the column kernel takes with its eight warps, for fibres that the l-split kernels take, and where the
+// TMA-fed kernel may split the l range (tiles that leave SMs idle, or a last round worth splitting; its
+// shape model never splits ranges below 160 l).
+bool one_chain_before(const View3& v, int dtype, int split)
+{
+    if (split > 1) return false;
+    const int64_t rows = v.outer * v.inner, rv = dtype == 0 ? 4 : 2;
+    const bool tma = rows * v.nq * (16 / rv) >= kStreamMinBytes && stream_supported(v, dtype);
+    if (v.inner == 1) return tma ? rows >= 148 * 512 && v.nq <= 1024 : rows > kBvecSmallMaxRows || v.nq < 1024;
+    if (tma) return v.nq < 160 || (rows >= 2 * 148 * 256 * rv && v.nq <= 1024);
+    const int64_t w = aligned16(v.a) && aligned16(v.c) && v.inner % rv == 0 ? rv : 1;
+    return rows > kColSplitWarps * 32 * w;
+}
+
+// At most 16 columns: tiles of 256 rows in one chain where that is no further off and they fill the GPU
+// (four blocks per SM), else tiles of 128 rows in folded sums, whose levels fit the registers.
+template <int TM, int ST>
+cudaError_t ffma_dispatch_small(const View3& v, cudaStream_t s, int sms, int split, int64_t lper, float* ws)
+{
+    const ColumnGrid gr = split_columns(v.m, 4, 4);
+    switch (gr.nf) {
+    case 1: return ffma_dispatch_form<4, TM, 1, ST>(v, s, gr, sms, split, lper, ws);
+    case 2: return ffma_dispatch_form<4, TM, 2, ST>(v, s, gr, sms, split, lper, ws);
+    case 3: return ffma_dispatch_form<4, TM, 3, ST>(v, s, gr, sms, split, lper, ws);
+    default: return ffma_dispatch_form<4, TM, 4, ST>(v, s, gr, sms, split, lper, ws);
+    }
+}
+
 template <int TM, int ST>
 cudaError_t ffma_dispatch_narrow(const View3& v, cudaStream_t s, int sms, int split, int64_t lper, float* ws)
 {
     const ColumnGrid gr = split_columns(v.m, 8, 4);
     switch (gr.nf) {
-    case 1: return ffma_dispatch_form<4, TM, 1, ST>(v, s, gr, sms, split, lper, ws);
-    case 2: return ffma_dispatch_form<4, TM, 2, ST>(v, s, gr, sms, split, lper, ws);
-    case 3: return ffma_dispatch_form<4, TM, 3, ST>(v, s, gr, sms, split, lper, ws);
-    case 4: return ffma_dispatch_form<4, TM, 4, ST>(v, s, gr, sms, split, lper, ws);
     case 5: return ffma_dispatch_form<4, TM, 5, ST>(v, s, gr, sms, split, lper, ws);
     case 6: return ffma_dispatch_form<4, TM, 6, ST>(v, s, gr, sms, split, lper, ws);
     case 7: return ffma_dispatch_form<4, TM, 7, ST>(v, s, gr, sms, split, lper, ws);
@@ -962,6 +995,9 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     const cudaError_t e = sms_of_device(sms);
     if (e != cudaSuccess) return e;
     const int64_t rows = (split > 1 ? split : 1) * ceil_div(v.outer * v.inner, 256);
+    if (v.m <= kSmallM)
+        return rows >= 4 * sms && one_chain_before(v, 0, split) ? ffma_dispatch_small<8, 3>(v, s, sms, split, lper, ws)
+                                                                : ffma_dispatch_small<4, 4>(v, s, sms, split, lper, ws);
     // Blocks of 8 x 8 outputs a thread where they fill both slots of every SM; up to 32 columns, and
     // problems with fewer tiles, in the narrow form (its shared-memory reads per multiply-add are
     // those of the wide form at half the columns: m = 24, A 160 MB 74 -> 59 us), with rows of 128
@@ -979,11 +1015,11 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
                                                    : ffma_dispatch_narrow<4, 4>(v, s, sms, split, lper, ws);
 }
 
-template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM>
+template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, int FOLD>
 cudaError_t dmma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws)
 {
     constexpr int smem = (int)sizeof(f64::Smem<BM, NF, ST, AK, BCM>);
-    const auto kernel = dmma_gemm_kernel<BM, NF, ST, AK, VEC, BCM>;
+    const auto kernel = dmma_gemm_kernel<BM, NF, ST, AK, VEC, BCM, FOLD>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int64_t tiles = ceil_div(v.outer * v.inner, BM) * gr.cols;
@@ -991,23 +1027,48 @@ cudaError_t dmma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, in
     // them (n_q = 16, A 256 MB: m = 64 147 -> 114 us, m = 8 94 -> 67 us). Longer ones: a block per
     // tile, which the scheduler balances better (m = 64, n_q = 48: 97 us against 113).
     const bool walk = v.nq <= (NF <= 2 ? 8 : 2) * f64::BK;
-    const int64_t slots = (int64_t)sms * (BM == 128 ? 2 : 5);
+    const int64_t slots = (int64_t)sms * dmma_blocks(BM, AK, FOLD);
     const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
     kernel<<<grid, 2 * BM, smem, s>>>(v, gr, tiles, lper, ws);
     return cudaGetLastError();
 }
 
+template <int BM, int NF, int ST, bool AK, bool VEC>
+cudaError_t dmma_dispatch_form(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws,
+                               int fold)
+{
+    if constexpr (NF <= 2) {
+        if (fold == 16)
+            return v.b_cm ? dmma_launch<BM, NF, ST, AK, VEC, true, 16>(v, s, gr, sms, split, lper, ws)
+                          : dmma_launch<BM, NF, ST, AK, VEC, false, 16>(v, s, gr, sms, split, lper, ws);
+        if constexpr (!AK)
+            if (fold == 8)
+                return v.b_cm ? dmma_launch<BM, NF, ST, AK, VEC, true, 8>(v, s, gr, sms, split, lper, ws)
+                              : dmma_launch<BM, NF, ST, AK, VEC, false, 8>(v, s, gr, sms, split, lper, ws);
+    }
+    return v.b_cm ? dmma_launch<BM, NF, ST, AK, VEC, true, 0>(v, s, gr, sms, split, lper, ws)
+                  : dmma_launch<BM, NF, ST, AK, VEC, false, 0>(v, s, gr, sms, split, lper, ws);
+}
+
 template <int BM, int NF, int ST>
-cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws)
+cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws,
+                             int fold = 0)
 {
     const bool ak = v.inner == 1;
     const bool vec = aligned16(v.a) && (ak ? v.nq : v.inner) % 2 == 0;
-#define TLIBTTM_DMMA(AKv, VECv) \
-    (v.b_cm ? dmma_launch<BM, NF, ST, AKv, VECv, true>(v, s, gr, sms, split, lper, ws) \
-            : dmma_launch<BM, NF, ST, AKv, VECv, false>(v, s, gr, sms, split, lper, ws))
-    if (ak) return vec ? TLIBTTM_DMMA(true, true) : TLIBTTM_DMMA(true, false);
-    return vec ? TLIBTTM_DMMA(false, true) : TLIBTTM_DMMA(false, false);
-#undef TLIBTTM_DMMA
+    if (ak)
+        return vec ? dmma_dispatch_form<BM, NF, ST, true, true>(v, s, gr, sms, split, lper, ws, fold)
+                   : dmma_dispatch_form<BM, NF, ST, true, false>(v, s, gr, sms, split, lper, ws, fold);
+    return vec ? dmma_dispatch_form<BM, NF, ST, false, true>(v, s, gr, sms, split, lper, ws, fold)
+               : dmma_dispatch_form<BM, NF, ST, false, false>(v, s, gr, sms, split, lper, ws, fold);
+}
+
+// The length of the tile's chains (0: one chain of n_q). Chains of 8 take 5-9 % more time than those of 16
+// and are as good as the column kernel's eight chains up to n_q = 160, those of 16 from there.
+int dmma_chain(const View3& v, int split)
+{
+    if (v.m > kSmallM || one_chain_before(v, 1, split)) return 0;
+    return v.inner > 1 && v.nq < 160 ? 8 : 16;
 }
 
 // Widest column tile in groups of eight: 64 columns where the tiles fill the GPU, narrower ones
@@ -1027,13 +1088,14 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     if (e != cudaSuccess) return e;
     const bool vec = aligned16(v.a) && (v.inner == 1 ? v.nq : v.inner) % 2 == 0;
     const ColumnGrid gr = split_columns(v.m, split > 1 ? (v.m > 16 ? 8 : 2) : dmma_width(v, sms));
+    const int fold = dmma_chain(v, split);
     switch (gr.nf) {
     case 1:
-        return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws)
-                   : dmma_dispatch_nf<128, 1, 4>(v, s, gr, sms, split, lper, ws);
+        return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws, fold)
+                   : dmma_dispatch_nf<128, 1, 4>(v, s, gr, sms, split, lper, ws, fold);
     case 2:
-        return vec ? dmma_dispatch_nf<64, 2, 4>(v, s, gr, sms, split, lper, ws)
-                   : dmma_dispatch_nf<128, 2, 4>(v, s, gr, sms, split, lper, ws);
+        return vec ? dmma_dispatch_nf<64, 2, 4>(v, s, gr, sms, split, lper, ws, fold)
+                   : dmma_dispatch_nf<128, 2, 4>(v, s, gr, sms, split, lper, ws, fold);
     case 3: return dmma_dispatch_nf<128, 3, 4>(v, s, gr, sms, split, lper, ws);
     case 4: return dmma_dispatch_nf<128, 4, 4>(v, s, gr, sms, split, lper, ws);
     case 5: return dmma_dispatch_nf<128, 5, 3>(v, s, gr, sms, split, lper, ws);
@@ -1067,7 +1129,7 @@ template <typename T, int W>
 cudaError_t colvec_dispatch_w(const View3& v, cudaStream_t s)
 {
     const int64_t row_warps = ceil_div(v.outer * v.inner, 32 * W);
-    return row_warps < 148 * 32 ? colvec_dispatch_ls<T, W, 8>(v, s) : colvec_dispatch_ls<T, W, 1>(v, s);
+    return row_warps < kColSplitWarps ? colvec_dispatch_ls<T, W, 8>(v, s) : colvec_dispatch_ls<T, W, 1>(v, s);
 }
 
 template <int TN>
@@ -1077,7 +1139,10 @@ cudaError_t few_columns_launch(const View3& v, cudaStream_t s)
     const auto kernel = v.b_cm ? few_columns_kernel<TN, true> : few_columns_kernel<TN, false>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kernel<<<(unsigned)(v.outer * ceil_div(v.inner, few::BM)), few::NT, smem, s>>>(v);
+    // the column kernel would split l over eight warps below this many rows
+    const bool chains = v.outer * v.inner <= kColSplitWarps * 32;
+    const int chain = !chains ? 0x7fffffff : v.nq < 128 ? 1 : 3;
+    kernel<<<(unsigned)(v.outer * ceil_div(v.inner, few::BM)), few::NT, smem, s>>>(v, chain);
     return cudaGetLastError();
 }
 
@@ -1216,14 +1281,23 @@ cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s)
     return vec ? rowdot_dispatch_v<T, true>(v, s) : rowdot_dispatch_v<T, false>(v, s);
 }
 
-// Sum of the `parts` partial results of a split K loop, in a fixed order: c[i] = sum_z ws[z][i].
+// Sum of the `parts` partial results of a split K loop, in a fixed order: c[i] = sum_z ws[z][i], in
+// double (sixteen at a time), so that many parts cost no accuracy.
 template <typename T>
 __global__ void __launch_bounds__(256) split_reduce_kernel(const T* __restrict__ ws, int parts, int64_t n, T* __restrict__ c)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        T sum = ws[i];
-        for (int z = 1; z < parts; ++z) sum += ws[(size_t)z * n + i];
-        c[i] = sum;
+        double sum = 0.0;
+        for (int z0 = 0; z0 < parts; z0 += 16) {
+            T x[16];   // sixteen loads in flight
+#pragma unroll
+            for (int z = 0; z < 16; ++z) x[z] = z0 + z < parts ? ws[(size_t)(z0 + z) * n + i] : T(0);
+            double s = x[0];
+#pragma unroll
+            for (int z = 1; z < 16; ++z) s += x[z];
+            sum += s;
+        }
+        c[i] = (T)sum;
     }
 }
 
@@ -1241,7 +1315,6 @@ __global__ void __launch_bounds__(256) split_reduce_kernel(const T* __restrict__
 // W = 16 / sizeof(T) when the vector accesses are aligned (VEC), else 1.
 // ---------------------------------------------------------------------------------------------
 constexpr int kBvecMaxR = 8, kBvecMaxM = 256, kBvecTile = 1024;
-constexpr int64_t kBvecSmallMaxRows = 65536;   // small m: row tiles of 8 up to this many rows
 
 // Offsets in A of (row r0 + r, l = 0) for the R rows of a row tile (r = k inner + i); A's element
 // (row, l) is then at offset + l inner.

@@ -88,3 +88,12 @@ def test_no_further_off_than_one_chain(cuda, dt, outer, nq, inner, m, b_cm):
     err, kernel = _error(cuda, dt, outer, nq, inner, m, b_cm)
     assert kernel == "simt_gemm"
     assert err <= (2.0 ** -24 if dt == np.float32 else 2.0 ** -53) * ((_chain(nq) + 1) / 3) ** 0.5
+
+
+# m > 64 with a long l range and few tiles: parts of nq / S, S two blocks per SM over the tiles of 128 x 128
+# (and parts of 1024 l at least)
+@pytest.mark.parametrize("outer,nq,inner,m,parts", [(9600, 4096, 1, 100, 4), (1, 9000, 9500, 70, 4), (1000, 30000, 1, 256, 19)])
+def test_split_parts(cuda, outer, nq, inner, m, parts):
+    err, kernel = _error(cuda, np.float32, outer, nq, inner, m, False)
+    assert kernel == "simt_gemm"
+    assert err <= 2.0 ** -24 * ((_chain(-(-nq // parts) + 16) + 2) / 3) ** 0.5

@@ -1544,7 +1544,9 @@ constexpr int64_t kMaxSplit = 256, kSplitChainF32 = 1024;
 template <typename T>
 int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
 {
-    constexpr int64_t BM = 128, BN = 64, BK = 16;
+    // (float: counted in tiles of 128 columns, for parts, and so chains, no longer than those of the 128 x
+    // 128 tiles before)
+    constexpr int64_t BM = 128, BN = sizeof(T) == 4 ? 128 : 64, BK = 16;
     const int64_t tiles = ceil_div(v.outer * v.inner, BM) * ceil_div(v.m, BN);
     const int64_t slots = (int64_t)sms * 2;
     lper = v.nq;

@@ -1001,8 +1001,10 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     // Blocks of 8 x 8 outputs a thread where they fill both slots of every SM; up to 32 columns, and
     // problems with fewer tiles, in the narrow form (its shared-memory reads per multiply-add are
     // those of the wide form at half the columns: m = 24, A 160 MB 74 -> 59 us), with rows of 128
-    // where 256 would leave slots empty.
-    if (v.m > 32 && rows * ceil_div(v.m, 64) >= 2 * sms) {
+    // where 256 would leave slots empty, or be padding for a quarter of its rows or more (split ranges of
+    // few rows: A (128, 2^17), m = 256 430 -> 231 us, (300, 2^17), m = 100 402 -> 316).
+    const bool tall = 5 * ceil_div(v.outer * v.inner, 128) >= 8 * ceil_div(v.outer * v.inner, 256);
+    if (v.m > 32 && tall && rows * ceil_div(v.m, 64) >= 2 * sms) {
         const ColumnGrid gr = split_columns(v.m, 8);
         switch (gr.nf) {
         case 5: return ffma_dispatch_form<8, 8, 5, 4>(v, s, gr, sms, split, lper, ws);
@@ -1011,7 +1013,7 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
         default: return ffma_dispatch_form<8, 8, 8, 4>(v, s, gr, sms, split, lper, ws);
         }
     }
-    return rows * ceil_div(v.m, 32) >= 4 * sms ? ffma_dispatch_narrow<8, 3>(v, s, sms, split, lper, ws)
+    return tall && rows * ceil_div(v.m, 32) >= 4 * sms ? ffma_dispatch_narrow<8, 3>(v, s, sms, split, lper, ws)
                                                    : ffma_dispatch_narrow<4, 4>(v, s, sms, split, lper, ws);
 }
 

@@ -1661,6 +1661,8 @@ SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma)
         else take = take || (v.inner >= 64 && (v.m > 8 || (!tma && tiles <= 64)));
         if (take) return SmallGemm::Split;
     }
+    // ranges too long for parts of kSplitChainF32: one block per tile would leave most SMs idle
+    if (lsplit && !f64 && v.nq >= 2048) return SmallGemm::No;
     if (tma && (v.m > 8 ? 20 * blocks < 17 * sms : few)) return SmallGemm::No;
     bool take;
     if (dtype == 0) {

@@ -296,7 +296,7 @@ unsigned long long tlibttm_launch_count(int reset);
 /* Waits for all work the library enqueued on `stream`. */
 int tlibttm_synchronize(void* stream);
 
-/* Releases the library's staging buffers on the current device. */
+/* Releases the library's staging buffers on the current device, and the workspace memory it keeps. */
 int tlibttm_release_buffers(void);
 
 /*

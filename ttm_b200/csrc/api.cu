@@ -61,6 +61,60 @@ cudaError_t dev_malloc_async(void** p, size_t bytes, cudaStream_t s)
     return cudaMallocAsync(p, bytes, s);
 }
 
+bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;   // the legacy stream while another one is captured
+}
+
+namespace {
+constexpr uint64_t kSplitPoolKeeps = uint64_t(64) << 20;
+std::mutex g_split_pools_mu;
+std::unordered_map<int, cudaMemPool_t> g_split_pools;   // by device; null where none could be made
+
+cudaMemPool_t split_pool(int dev)
+{
+    std::lock_guard<std::mutex> lk(g_split_pools_mu);
+    auto it = g_split_pools.find(dev);
+    if (it != g_split_pools.end()) return it->second;
+    cudaMemPool_t pool = nullptr;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kSplitPoolKeeps;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        pool = nullptr;
+    } else {
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    return g_split_pools[dev] = pool;
+}
+}  // namespace
+
+cudaError_t split_malloc_async(void** p, size_t bytes, cudaStream_t s)
+{
+    int dev = 0;
+    if (capturing(s) || cudaGetDevice(&dev) != cudaSuccess) return dev_malloc_async(p, bytes, s);
+    cudaMemPool_t pool = split_pool(dev);
+    if (!pool) return dev_malloc_async(p, bytes, s);
+    if (injected_alloc_failure()) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
+}
+
+void release_split_pools()
+{
+    std::lock_guard<std::mutex> lk(g_split_pools_mu);
+    for (auto& it : g_split_pools)
+        if (it.second) cudaMemPoolTrimTo(it.second, 0);
+}
+
 namespace {
 
 thread_local std::string g_err;
@@ -1325,6 +1379,7 @@ int tlibttm_release_buffers(void)
         b->bytes = 0;
     }
     tc_release_buffers();
+    release_split_pools();
     return TLIBTTM_OK;
 }
 

@@ -260,6 +260,14 @@ __host__ __device__ inline uint32_t fast_div(uint32_t n, const FastDiv& f)
 // stream-ordered cudaMallocAsync), so that a test can make the n-th one fail (tlibttm_inject).
 cudaError_t dev_malloc(void** p, size_t bytes);
 cudaError_t dev_malloc_async(void** p, size_t bytes, cudaStream_t s);
+// Memory for the parts of a split l range, freed with cudaFreeAsync: stream-ordered, from a pool of the
+// library's own for the device. The default pool hands its memory back to the driver at every
+// synchronisation (a call after one then took 200 us more), which is the process's to change; this one
+// keeps up to 64 MB, which release_split_pools() gives back. Inside a capture: the default pool's node.
+cudaError_t split_malloc_async(void** p, size_t bytes, cudaStream_t s);
+void release_split_pools();
+// Whether stream s is being captured into a graph.
+bool capturing(cudaStream_t s);
 
 // Bound of the bounded mbarrier waits of the bf16x3 kernel, in ns (4 s unless a test set it).
 unsigned long long wait_limit_ns();

@@ -16,7 +16,6 @@
 //
 // All index arithmetic is 64-bit (a 256^4 tensor has 2^32 elements).
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "common.cuh"
@@ -1565,24 +1564,6 @@ int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
     return (int)ceil_div(v.nq, lper);
 }
 
-// Workspaces come from the stream-ordered pool, which by default hands its memory back to the driver
-// at every synchronisation (a call after one then took 200 us more): up to 64 MB stay cached. The
-// paths with larger scratch keep all of theirs.
-void keep_small_workspaces(cudaStream_t s)
-{
-    static std::atomic<uint64_t> done{0};   // bit per device
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64 || (done.load() >> dev & 1)) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return;
-    cudaMemPool_t pool;
-    uint64_t now = 0, want = uint64_t(64) << 20;
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &now) == cudaSuccess && now < want)
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &want);
-    done.fetch_or(uint64_t(1) << dev);
-}
-
 template <typename T>
 cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool force, bool may_split)
 {
@@ -1595,8 +1576,7 @@ cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool
     if (S <= 1) return simt_gemm_dispatch(v, s, 1, 0, static_cast<T*>(nullptr));
     const int64_t nc = v.outer * v.m * v.inner;
     T* ws = nullptr;
-    keep_small_workspaces(s);
-    if ((e = dev_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess) return e;
+    if ((e = split_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess) return e;
     e = simt_gemm_dispatch(v, s, S, lper, ws);
     if (e == cudaSuccess) {
         split_reduce_kernel<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nc, 256), 4096)), 256, 0, s>>>(

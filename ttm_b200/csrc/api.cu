@@ -286,8 +286,15 @@ int note_launch(cudaError_t e, int kid)
 
 constexpr int64_t kPlanStreamMinBytes = int64_t(4) << 20;
 
-// All operands are device memory: enqueue on stream s.
-int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t stream_min_bytes = kStreamMinBytes)
+// Memory that a plan holds for the parts of a split l range of a small-m problem (p null: none was to
+// be had, or the problem needs none).
+struct SplitSpace {
+    void* p = nullptr;
+};
+
+// All operands are device memory: enqueue on stream s. `space`: the plan's, null for a single call.
+int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t stream_min_bytes = kStreamMinBytes,
+               const SplitSpace* space = nullptr)
 {
     if (!pl.dense) {
         pl.sp.a = x.a;
@@ -306,12 +313,18 @@ int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t s
         // TMA-fed row mode measured 0.87-0.88 of HBM against 0.65-0.72 at m = 8).
         const int64_t a_bytes = v.outer * v.nq * v.inner * (x.dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= stream_min_bytes && stream_supported(v, x.dtype);
-        const SmallGemm gemm = small_m_takes_gemm(v, x.dtype, tma);
+        SmallGemm gemm = small_m_takes_gemm(v, x.dtype, tma, space ? space->p != nullptr : true);
+        // A split l range needs memory for its parts. A graph that a caller captures gets no allocation
+        // of its own for it (only the l-split kernels always had one), and where there is no memory the
+        // kernels that need none run.
+        if (gemm == SmallGemm::Split && !space && (tma || !bvec_small_supported(v)) && capturing(s))
+            gemm = small_m_takes_gemm(v, x.dtype, tma, false);
         if (gemm == SmallGemm::Split) {
             int n = 1;
-            const cudaError_t e = launch_simt_gemm(v, x.dtype, s, &n, true);
+            const cudaError_t e = launch_simt_gemm(v, x.dtype, s, &n, true, true, space ? space->p : nullptr);
             if (e == cudaSuccess && n > 1) g_launches += (unsigned long long)(n - 1);   // the reduction
-            return note_launch(e, K_SIMT_GEMM);
+            if (e != cudaErrorMemoryAllocation) return note_launch(e, K_SIMT_GEMM);
+            gemm = small_m_takes_gemm(v, x.dtype, tma, false);
         }
         if (gemm == SmallGemm::Whole)
             return note_launch(launch_simt_gemm(v, x.dtype, s, nullptr, false, false), K_SIMT_GEMM);
@@ -671,7 +684,35 @@ struct Single {            // one problem launched on its own inside a plan
     const void* b;
     void* c;
     Plan pl;
+    SplitSpace space;
 };
+
+// Whether a plan's problem takes the slice-GEMM with a split l range if it has memory for the parts.
+bool single_splits(const Single& sg, int dtype)
+{
+    const View3& v = sg.pl.v;
+    if (!sg.pl.dense || v.m > kSmallM) return false;
+    const int64_t a_bytes = v.outer * v.nq * v.inner * (dtype == TLIBTTM_F32 ? 4 : 8);
+    const bool tma = a_bytes >= kPlanStreamMinBytes && stream_supported(v, dtype);
+    return small_m_takes_gemm(v, dtype, tma, true) == SmallGemm::Split;
+}
+
+// The views of a plan's single launches, and memory for the parts of those whose l range is split (as
+// much as can be had: a replayed graph then holds no allocation for them).
+void prepare_singles(std::vector<Single>& singles, int dtype)
+{
+    for (Single& sg : singles) {
+        if (!sg.pl.dense) continue;
+        sg.pl.v.a = sg.a;
+        sg.pl.v.b = sg.b;
+        sg.pl.v.c = sg.c;
+        if (!single_splits(sg, dtype)) continue;
+        if (dev_malloc(&sg.space.p, simt_gemm_split_bytes(sg.pl.v, dtype)) != cudaSuccess) {
+            cudaGetLastError();
+            sg.space.p = nullptr;
+        }
+    }
+}
 
 int run_single(Single& sg, int precision, cudaStream_t s)
 {
@@ -681,7 +722,7 @@ int run_single(Single& sg, int precision, cudaStream_t s)
     x.b = sg.b;
     x.c = sg.c;
     // a plan streams many problems through HBM: the TMA-fed small-m kernel pays off from 4 MB
-    return run_device(x, sg.pl, precision, s, kPlanStreamMinBytes);
+    return run_device(x, sg.pl, precision, s, kPlanStreamMinBytes, &sg.space);
 }
 
 // Kernels run_device launches for a plan entry (tensor-core paths launch two).
@@ -692,7 +733,7 @@ int launches_of(const Single& sg, int dtype, int precision)
         const View3& v = sg.pl.v;
         const int64_t a_bytes = v.outer * v.nq * v.inner * (dtype == TLIBTTM_F32 ? 4 : 8);
         const bool tma = a_bytes >= kPlanStreamMinBytes && stream_supported(v, dtype);
-        const SmallGemm gemm = small_m_takes_gemm(v, dtype, tma);
+        const SmallGemm gemm = small_m_takes_gemm(v, dtype, tma, sg.space.p != nullptr);
         if (gemm != SmallGemm::No) return gemm == SmallGemm::Split ? 2 : 1;
         return (!tma && bvec_small_supported(v)) ? 2 : 1;
     }
@@ -822,6 +863,8 @@ void plan_free(tlibttm_plan* P)
     stream_group_destroy(P->sg);
     for (void* b : P->bufs)
         if (b) cudaFree(b);
+    for (const Single& sg : P->singles)
+        if (sg.space.p) cudaFree(sg.space.p);
     if (P->own) cudaStreamDestroy(P->own);
     for (int w = 0; w < kPlanStreams; ++w) {
         if (P->workers[w]) cudaStreamDestroy(P->workers[w]);
@@ -1085,7 +1128,7 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
                     // few rows and a long l range: the l-split launch (a work item would be one block)
                     if (pl.dense && bvec_small_supported(v)) single = true;
                     if (!pl.dense || single) {
-                        P->singles.push_back(Single{dtype, x.a, x.b, x.c, pl});
+                        P->singles.push_back(Single{dtype, x.a, x.b, x.c, pl, {}});
                     } else {
                         GroupDesc d{};
                         d.a = x.a;
@@ -1170,6 +1213,7 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
         return e == cudaErrorMemoryAllocation ? fail(TLIBTTM_ERR_ALLOC, "tlibttm_plan_batched: device allocation failed.")
                                               : cuda_fail(e, "grouped small-m set-up");
     if (!P->singles.empty() && (e = tc_prepare_device()) != cudaSuccess) return cuda_fail(e, "tensor-core state");
+    prepare_singles(P->singles, dtype);
     *plan = P.release();
     return TLIBTTM_OK;
 }
@@ -1239,7 +1283,7 @@ int tlibttm_plan_chain(int dtype, int precision, unsigned p, const void* a, cons
                 } else if (w1 != Where::Device || w2 != Where::Device || w3 != Where::Device) {
                     rc = fail(TLIBTTM_ERR_ARG, "plans take device operands only.");
                 } else {
-                    P->singles.push_back(Single{dtype, in, bs[s], out, pl});
+                    P->singles.push_back(Single{dtype, in, bs[s], out, pl, {}});
                 }
             }
         }
@@ -1248,6 +1292,7 @@ int tlibttm_plan_chain(int dtype, int precision, unsigned p, const void* a, cons
         cur = nc;
     }
     if ((e = tc_prepare_device()) != cudaSuccess) return cuda_fail(e, "tensor-core state");
+    prepare_singles(P->singles, dtype);
     *plan = P.release();
     return TLIBTTM_OK;
 }

@@ -164,12 +164,15 @@ const char* kernel_name(int id);
 // more blocks and the parts are added by a second kernel (*launches = 2, else 1).
 // force_split: split the K loop whenever n_q >= 2048 (a schedule of its own for the tuner);
 // may_split false: never (one launch).
+// `space`: memory for the parts (simt_gemm_split_bytes); none: from a pool, cudaErrorMemoryAllocation
+// if that has none.
 cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr,
-                             bool force_split = false, bool may_split = true);
+                             bool force_split = false, bool may_split = true, void* space = nullptr);
+size_t simt_gemm_split_bytes(const View3& v, int dtype);   // with force_split
 // m <= kSmallM: whether the slice-GEMM is the faster choice against the small-m kernels (`tma`: the
-// TMA-fed one would take the problem), in one launch or with its l range split (two).
+// TMA-fed one would take the problem), in one launch or, if it may, with its l range split (two).
 enum class SmallGemm { No, Whole, Split };
-SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma);
+SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma, bool may_split);
 int simt_gemm_launch_count(const View3& v, int dtype);
 // Few output rows (outer * inner <= 8), 16 < m <= 256, n_q >= 4096: a kernel that streams B with
 // the l range split over the GPU, then a fixed-order reduction (*launches = 2).

@@ -1565,7 +1565,7 @@ int gemm_split_parts(const View3& v, int sms, int64_t& lper, bool force = false)
 }
 
 template <typename T>
-cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool force, bool may_split)
+cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool force, bool may_split, void* space)
 {
     int sms = 0;
     cudaError_t e = sms_of_device(sms);
@@ -1575,24 +1575,35 @@ cudaError_t simt_gemm_launch(const View3& v, cudaStream_t s, int* launches, bool
     if (launches) *launches = S > 1 ? 2 : 1;
     if (S <= 1) return simt_gemm_dispatch(v, s, 1, 0, static_cast<T*>(nullptr));
     const int64_t nc = v.outer * v.m * v.inner;
-    T* ws = nullptr;
-    if ((e = split_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess) return e;
+    T* ws = static_cast<T*>(space);
+    if (!space && (e = split_malloc_async(reinterpret_cast<void**>(&ws), (size_t)S * nc * sizeof(T), s)) != cudaSuccess)
+        return e;
     e = simt_gemm_dispatch(v, s, S, lper, ws);
     if (e == cudaSuccess) {
         split_reduce_kernel<T><<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nc, 256), 4096)), 256, 0, s>>>(
             ws, S, nc, static_cast<T*>(v.c));
         e = cudaGetLastError();
     }
-    cudaFreeAsync(ws, s);
+    if (!space) cudaFreeAsync(ws, s);
     return e;
 }
 
 }  // namespace
 
-cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches, bool force_split, bool may_split)
+cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* launches, bool force_split, bool may_split,
+                             void* space)
 {
-    return dtype == 0 ? simt_gemm_launch<float>(v, s, launches, force_split, may_split)
-                      : simt_gemm_launch<double>(v, s, launches, force_split, may_split);
+    return dtype == 0 ? simt_gemm_launch<float>(v, s, launches, force_split, may_split, space)
+                      : simt_gemm_launch<double>(v, s, launches, force_split, may_split, space);
+}
+
+size_t simt_gemm_split_bytes(const View3& v, int dtype)
+{
+    int sms = 0;
+    if (sms_of_device(sms) != cudaSuccess) return 0;
+    int64_t lper = 0;
+    const int S = dtype == 0 ? gemm_split_parts<float>(v, sms, lper, true) : gemm_split_parts<double>(v, sms, lper, true);
+    return S > 1 ? (size_t)S * (size_t)(v.outer * v.m * v.inner) * (dtype == 0 ? sizeof(float) : sizeof(double)) : 0;
 }
 
 // Measured over A of 2^14 to 2^26 elements, n_q 3 to 2001, inner 1 to 1001, as time of the small-m
@@ -1623,7 +1634,7 @@ cudaError_t launch_simt_gemm(const View3& v, int dtype, cudaStream_t s, int* lau
 // Shorter ranges of few tiles keep to the TMA-fed kernel (m 9..16: 0.5-0.8 at 64 blocks, 1.1 at 128; m
 // 5..8 0.9 at 128, 1.1 at 256), or to the l-split kernels and the column kernel's l split (0.8-0.9
 // below about 16 tiles of 128 rows).
-SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma)
+SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma, bool may_split)
 {
     int sms = 0;
     if (sms_of_device(sms) != cudaSuccess) return SmallGemm::No;
@@ -1633,7 +1644,7 @@ SmallGemm small_m_takes_gemm(const View3& v, int dtype, bool tma)
     const int64_t blocks = ceil_div(rows, f64 && vec ? kGemmRows / 2 : kGemmRows);
     const bool lsplit = !tma && bvec_small_supported(v);   // the l-split kernels would take it
     const bool few = 10 * blocks < 17 * sms;
-    if ((few || (lsplit && !f64)) && v.nq >= 2048 && (f64 || v.nq <= kSplitChainF32 * kMaxSplit) && rows > kBvecMaxR &&
+    if (may_split && (few || (lsplit && !f64)) && v.nq >= 2048 && (f64 || v.nq <= kSplitChainF32 * kMaxSplit) && rows > kBvecMaxR &&
         rows * v.nq >= (int64_t(1) << 21)) {
         bool take = lsplit;
         if (fibres) take = take || v.m > (f64 ? 4 : 8) || rows <= (v.m > 4 ? 4 : 1) * kGemmRows;

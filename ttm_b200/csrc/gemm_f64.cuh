@@ -12,8 +12,9 @@
 // 323 -> 144 us (30 TFLOP/s); (150, 171, 333), m = 100 189 -> 84 us; (200, 180, 160), m = 20
 // 84 -> 19 us; contiguous fibres of 384, 78000 rows, m = 16 (TMA row kernel) 139 -> 50 us. (Running
 // pointers in place of addresses recomputed per copy gave 5-15 % of that.)
-// Rows of 64 for at most 16 columns (five blocks of 128 threads per SM, 16-byte copies): 59 us at
-// 128 rows against 53; with 8-byte copies 128 rows are faster (73 against 119 us).
+// Rows of 64 for at most 16 columns with 16-byte copies (five blocks of 128 threads per SM, four for
+// contiguous fibres): 59 us at 128 rows against 53; with 8-byte copies 128 rows are faster (73 against
+// 119 us).
 #pragma once
 
 #include "common.cuh"

@@ -88,12 +88,19 @@ __device__ __forceinline__ void split_range(View3& v, int64_t lper, T* ws, int64
     }
 }
 
-// Blocks per SM of the FP32 builds: 16 warps of at most 128 registers, or 20 of 100 where the
-// accumulators are small (and not folded).
-constexpr int ffma_blocks(int TX, int TM, int TN) { return TX == 8 ? 2 : TM == 8 || TN <= 4 ? 4 : 5; }
+// Blocks per SM of the FP32 builds: 16 warps of at most 128 registers, or 20 of 100 where the accumulators
+// are small (and not folded); for contiguous fibres, whose rows of A are padded further, as many as
+// their shared memory lets in. The launch bounds and the walking form's grid both follow these.
+constexpr int ffma_blocks(int TX, int TM, int TN, bool AK)
+{
+    return TX == 8 ? 2 : TM == 8 ? (AK ? 3 : 4) : AK || TN <= 4 ? 4 : 5;
+}
+// Shared memory of an SM, of which each block takes 1 KB besides its own.
+constexpr size_t kSmSharedBytes = 228 * 1024;
+constexpr bool blocks_fit(int blocks, size_t smem) { return blocks * (smem + 1024) <= kSmSharedBytes; }
 
 template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
-__global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM, TN)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
+__global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM, TN, AK)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
                                                                                int64_t lper, float* ws)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
@@ -922,13 +929,14 @@ template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
 cudaError_t ffma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, float* ws)
 {
     constexpr int smem = (int)sizeof(f32::Smem<TX, TM, TN, ST, AK>);
+    static_assert(blocks_fit(ffma_blocks(TX, TM, TN, AK), smem), "the walking form's blocks are resident at once");
     const auto kernel = ffma_gemm_kernel<TX, TM, TN, ST, AK, VEC, BCM>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int64_t tiles = ceil_div(v.outer * v.inner, 32 * TM) * gr.cols;
     // as in dmma_launch (m = 64, n_q = 16, A 64 MB: 86 -> 82 us; n_q = 64: 190 us against 197)
     const bool walk = v.nq <= 2 * f32::BK;
-    const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM, TN);
+    const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM, TN, AK);
     const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
     kernel<<<grid, 32 * TX, smem, s>>>(v, gr, tiles, lper, ws);
     return cudaGetLastError();
@@ -1020,6 +1028,7 @@ template <int BM, int NF, int ST, bool AK, bool VEC, bool BCM, int FOLD>
 cudaError_t dmma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws)
 {
     constexpr int smem = (int)sizeof(f64::Smem<BM, NF, ST, AK, BCM>);
+    static_assert(blocks_fit(dmma_blocks(BM, AK, FOLD), smem), "the walking form's blocks are resident at once");
     const auto kernel = dmma_gemm_kernel<BM, NF, ST, AK, VEC, BCM, FOLD>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;

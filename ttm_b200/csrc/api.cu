@@ -1152,21 +1152,21 @@ int tlibttm_plan_batched_ex(int dtype, int precision, size_t count, const tlibtt
                                 // column items: one row per lane (the asynchronous-copy tile takes
                                 // any alignment; a 16-byte build would cost the launch registers)
                                 d.flags = 0;
-                                d.tiles_m = ceil_div(M, 8 * 32);
+                                d.tiles_m = ceil_div(M, kGemvRows);
                             }
                             d.tiles_n = 1;
                         } else {
                             d.kind = 0;
                             d.tiles_m = ceil_div(M, kGemmRows);
                             grouped_columns(v.m, dtype, &d.tiles_n, &d.cols);
+                            // 16-byte copies of A (the tile looks at C's alignment itself)
                             const bool ak = v.inner == 1;
-                            bool vec = (reinterpret_cast<uintptr_t>(v.a) % 16 == 0) && (reinterpret_cast<uintptr_t>(v.c) % 16 == 0);
-                            vec = vec && (ak ? (v.nq % rv == 0 && v.m % rv == 0) : (v.inner % rv == 0));
+                            const bool vec = reinterpret_cast<uintptr_t>(v.a) % 16 == 0 && (ak ? v.nq : v.inner) % rv == 0;
                             d.flags = (ak ? 1 : 0) | (vec ? 2 : 0);
                         }
                         // cost ~ work-item count x work per item, for a largest-first order
                         const double per_item = d.kind == 0 ? (double)v.nq * kGemmRows * d.cols
-                                                            : (double)v.nq * (d.flags & 1 ? kGemvRows : 8 * 32 * (d.flags & 2 ? rv : 1)) * 16;
+                                                            : (double)v.nq * kGemvRows * 16;
                         items.push_back(Item{d, (double)(d.tiles_m * d.tiles_n) * per_item});
                     }
                 }

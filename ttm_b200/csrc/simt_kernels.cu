@@ -1,11 +1,10 @@
 // SIMT kernels of the B200 TTM library: the exact-arithmetic ("plain") paths.
 //
 //  simt_gemm  slice-GEMM over the dense view C[k][j][i] = sum_l A[k][l][i] B(j,l):
-//             FP32 FFMA in 128x128 CTA tiles with register-double-buffered
-//             shared-memory stages; FP64 on the double-precision matrix
-//             instruction (gemm_f64.cuh). Rows of the GEMM are the flattened
-//             (k, i) pairs, so one kernel covers every layout case without
-//             transposing anything.
+//             FP32 on packed FFMA (gemm_f32.cuh), FP64 on the double-precision
+//             matrix instruction (gemm_f64.cuh). Rows of the GEMM are the
+//             flattened (k, i) pairs, so one kernel covers every layout case
+//             without transposing anything.
 //  colvec     bandwidth kernel for small m when A's fibres along mode q are
 //             strided (inner >= 2): each thread owns W consecutive i of one k
 //             and streams 16-byte loads along l; B is staged in shared memory.
@@ -136,7 +135,6 @@ __global__ void __launch_bounds__(2 * BM, dmma_blocks(BM, AK, FOLD)) dmma_gemm_k
 constexpr int kColWarps = 8;
 constexpr int64_t kBvecSmallMaxRows = 65536;   // small m: the l-split kernels' row tiles up to this many rows
 constexpr int64_t kColSplitWarps = 148 * 32;   // fewer warps of rows than this: l split over eight warps
-constexpr int kColUnroll1 = 8;   // l steps unrolled with one scalar row per lane
 
 template <typename T, int MB>
 struct ColvecSmem {
@@ -180,8 +178,7 @@ __device__ __forceinline__ void colvec_tile(const View3& v, int64_t row0, Colvec
         }
         __syncthreads();
         if (valid) {
-            // scalar rows (W = 1) take more l steps at a time, so that more loads are in flight
-#pragma unroll (W == 1 ? kColUnroll1 : 4)
+#pragma unroll 4
             for (int l = part; l < lc; l += LS) {
                 T a[W];
                 load_vec<T, W>(a, ap + (l0 + l) * inner);
@@ -1060,17 +1057,21 @@ cudaError_t dmma_dispatch_form(const View3& v, cudaStream_t s, const ColumnGrid&
                   : dmma_launch<BM, NF, ST, AK, VEC, false, 0>(v, s, gr, sms, split, lper, ws);
 }
 
+// BM 64: 16-byte copies of A only; 128 with one or two groups of columns: 8-byte ones only.
 template <int BM, int NF, int ST>
 cudaError_t dmma_dispatch_nf(const View3& v, cudaStream_t s, const ColumnGrid& gr, int sms, int split, int64_t lper, double* ws,
-                             int fold = 0)
+                             bool vec, int fold = 0)
 {
-    const bool ak = v.inner == 1;
-    const bool vec = aligned16(v.a) && (ak ? v.nq : v.inner) % 2 == 0;
-    if (ak)
-        return vec ? dmma_dispatch_form<BM, NF, ST, true, true>(v, s, gr, sms, split, lper, ws, fold)
-                   : dmma_dispatch_form<BM, NF, ST, true, false>(v, s, gr, sms, split, lper, ws, fold);
-    return vec ? dmma_dispatch_form<BM, NF, ST, false, true>(v, s, gr, sms, split, lper, ws, fold)
-               : dmma_dispatch_form<BM, NF, ST, false, false>(v, s, gr, sms, split, lper, ws, fold);
+    if (vec) {
+        if constexpr (BM == 64 || NF > 2)
+            return v.inner == 1 ? dmma_dispatch_form<BM, NF, ST, true, true>(v, s, gr, sms, split, lper, ws, fold)
+                                : dmma_dispatch_form<BM, NF, ST, false, true>(v, s, gr, sms, split, lper, ws, fold);
+    } else {
+        if constexpr (BM == 128)
+            return v.inner == 1 ? dmma_dispatch_form<BM, NF, ST, true, false>(v, s, gr, sms, split, lper, ws, fold)
+                                : dmma_dispatch_form<BM, NF, ST, false, false>(v, s, gr, sms, split, lper, ws, fold);
+    }
+    return cudaErrorNotSupported;
 }
 
 // The length of the tile's chains (0: one chain of n_q). Chains of 8 take 5-9 % more time than those of 16
@@ -1101,17 +1102,17 @@ cudaError_t simt_gemm_dispatch(const View3& v, cudaStream_t s, int split = 1, in
     const int fold = dmma_chain(v, split);
     switch (gr.nf) {
     case 1:
-        return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws, fold)
-                   : dmma_dispatch_nf<128, 1, 4>(v, s, gr, sms, split, lper, ws, fold);
+        return vec ? dmma_dispatch_nf<64, 1, 4>(v, s, gr, sms, split, lper, ws, true, fold)
+                   : dmma_dispatch_nf<128, 1, 4>(v, s, gr, sms, split, lper, ws, false, fold);
     case 2:
-        return vec ? dmma_dispatch_nf<64, 2, 4>(v, s, gr, sms, split, lper, ws, fold)
-                   : dmma_dispatch_nf<128, 2, 4>(v, s, gr, sms, split, lper, ws, fold);
-    case 3: return dmma_dispatch_nf<128, 3, 4>(v, s, gr, sms, split, lper, ws);
-    case 4: return dmma_dispatch_nf<128, 4, 4>(v, s, gr, sms, split, lper, ws);
-    case 5: return dmma_dispatch_nf<128, 5, 3>(v, s, gr, sms, split, lper, ws);
-    case 6: return dmma_dispatch_nf<128, 6, 3>(v, s, gr, sms, split, lper, ws);
-    case 7: return dmma_dispatch_nf<128, 7, 3>(v, s, gr, sms, split, lper, ws);
-    default: return dmma_dispatch_nf<128, 8, 3>(v, s, gr, sms, split, lper, ws);
+        return vec ? dmma_dispatch_nf<64, 2, 4>(v, s, gr, sms, split, lper, ws, true, fold)
+                   : dmma_dispatch_nf<128, 2, 4>(v, s, gr, sms, split, lper, ws, false, fold);
+    case 3: return dmma_dispatch_nf<128, 3, 4>(v, s, gr, sms, split, lper, ws, vec);
+    case 4: return dmma_dispatch_nf<128, 4, 4>(v, s, gr, sms, split, lper, ws, vec);
+    case 5: return dmma_dispatch_nf<128, 5, 3>(v, s, gr, sms, split, lper, ws, vec);
+    case 6: return dmma_dispatch_nf<128, 6, 3>(v, s, gr, sms, split, lper, ws, vec);
+    case 7: return dmma_dispatch_nf<128, 7, 3>(v, s, gr, sms, split, lper, ws, vec);
+    default: return dmma_dispatch_nf<128, 8, 3>(v, s, gr, sms, split, lper, ws, vec);
     }
 }
 
@@ -1122,7 +1123,7 @@ cudaError_t colvec_dispatch_ls(const View3& v, cudaStream_t s)
     dim3 grid((unsigned)ceil_div(M, (kColWarps / LS) * 32 * W)), block(256);
 #define TLIBTTM_COLVEC(MBv)                                                                \
     do {                                                                                   \
-        if (W == 1) colvec_async_kernel<T, MBv, LS><<<grid, block, 0, s>>>(v); \
+        if constexpr (W == 1) colvec_async_kernel<T, MBv, LS><<<grid, block, 0, s>>>(v);   \
         else colvec_kernel<T, MBv, W, LS><<<grid, block, 0, s>>>(v);                       \
     } while (0)
     if (v.m <= 1) TLIBTTM_COLVEC(1);

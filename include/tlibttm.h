@@ -289,6 +289,8 @@ int tlibttm_get_precision(void);
 
 /* Name of the kernel the last successful call on this thread launched (diagnostics, tests). */
 const char* tlibttm_last_kernel(void);
+/* The same with the kernels of a family told apart: "few_columns" (of colvec), "rowwarp" (of rowdot). */
+const char* tlibttm_last_variant(void);
 
 /* Number of kernels this library launched on the calling thread since the last reset. */
 unsigned long long tlibttm_launch_count(int reset);

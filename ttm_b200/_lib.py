@@ -45,6 +45,7 @@ def _declare(L):
     L.tlibttm_ttm_f32_bf16x3_noalloc.argtypes = sig
     L.tlibttm_last_error.restype = C.c_char_p
     L.tlibttm_last_kernel.restype = C.c_char_p
+    L.tlibttm_last_variant.restype = C.c_char_p
     L.tlibttm_set_precision.restype = C.c_int
     L.tlibttm_set_precision.argtypes = [C.c_int]
     L.tlibttm_get_precision.restype = C.c_int
@@ -115,6 +116,11 @@ def ttm_raw(dtype: int, precision: int, q: int, p: int, a_ptr: int, na, wa, pia,
 
 def last_kernel() -> str:
     return lib().tlibttm_last_kernel().decode()
+
+
+def last_variant() -> str:
+    """As last_kernel, with the kernels of a family told apart."""
+    return lib().tlibttm_last_variant().decode()
 
 
 def launch_count(reset: bool = False) -> int:

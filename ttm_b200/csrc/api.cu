@@ -28,8 +28,10 @@ const char* kernel_name(int id)
 {
     switch (id) {
     case K_SIMT_GEMM: return "simt_gemm";
-    case K_COLVEC: return "colvec";
-    case K_ROWDOT: return "rowdot";
+    case K_COLVEC:
+    case K_FEW_COLUMNS: return "colvec";
+    case K_ROWDOT:
+    case K_ROWWARP: return "rowdot";
     case K_STRIDED: return "strided";
     case K_TC_BF16X3: return "tc_bf16x3";
     case K_TC_FP8: return "tc_fp8";
@@ -42,6 +44,15 @@ const char* kernel_name(int id)
     case K_TC_PAIR: return "tc_bf16x3_pair";
     case K_BVEC: return "bvec";
     default: return "";
+    }
+}
+
+const char* kernel_variant(int id)
+{
+    switch (id) {
+    case K_FEW_COLUMNS: return "few_columns";
+    case K_ROWWARP: return "rowwarp";
+    default: return kernel_name(id);
     }
 }
 
@@ -118,7 +129,7 @@ void release_split_pools()
 namespace {
 
 thread_local std::string g_err;
-thread_local const char* g_last_kernel = "";
+thread_local const char *g_last_kernel = "", *g_last_variant = "";
 thread_local unsigned long long g_launches = 0;
 
 int initial_precision()
@@ -280,6 +291,7 @@ int note_launch(cudaError_t e, int kid)
 {
     if (e != cudaSuccess) return cuda_fail(e, kernel_name(kid));
     g_last_kernel = kernel_name(kid);
+    g_last_variant = kernel_variant(kid);
     ++g_launches;
     return TLIBTTM_OK;
 }
@@ -336,12 +348,15 @@ int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t s
             if (e == cudaSuccess && n > 1) g_launches += (unsigned long long)(n - 1);
             return note_launch(e, K_BVEC);
         }
+        int kid = K_NONE;
         if (v.inner == 1) {
             if (tma && v.nq >= 16) return note_launch(launch_stream(v, x.dtype, s), K_STREAM_ROWS);
-            return note_launch(launch_rowdot(v, x.dtype, s), K_ROWDOT);
+            const cudaError_t e = launch_rowdot(v, x.dtype, s, &kid);
+            return note_launch(e, kid);
         }
         if (tma) return note_launch(launch_stream(v, x.dtype, s), K_STREAM_COLS);
-        return note_launch(launch_colvec(v, x.dtype, s), K_COLVEC);
+        const cudaError_t e = launch_colvec(v, x.dtype, s, &kid);
+        return note_launch(e, kid);
     }
     if (precision == TLIBTTM_PREC_DEFAULT) precision = g_precision.load();
     if (precision == TLIBTTM_PREC_AUTO)
@@ -963,9 +978,14 @@ int tlibttm_ttm_sched(int dtype, int schedule, unsigned q, unsigned p, const voi
         if (e == cudaSuccess && n > 1) g_launches += (unsigned long long)(n - 1);
         return note_launch(e, K_SIMT_GEMM);
     }
-    case TLIBTTM_SCHED_COLS: return note_launch(launch_colvec_ls(v, dtype, 1, s), K_COLVEC);
-    case TLIBTTM_SCHED_COLS_SPLIT: return note_launch(launch_colvec_ls(v, dtype, 8, s), K_COLVEC);
-    case TLIBTTM_SCHED_ROWS: return note_launch(launch_rowdot(v, dtype, s), K_ROWDOT);
+    case TLIBTTM_SCHED_COLS:
+    case TLIBTTM_SCHED_COLS_SPLIT:
+    case TLIBTTM_SCHED_ROWS: {
+        int kid = K_NONE;
+        e = schedule == TLIBTTM_SCHED_ROWS ? launch_rowdot(v, dtype, s, &kid)
+                                           : launch_colvec_ls(v, dtype, schedule == TLIBTTM_SCHED_COLS ? 1 : 8, s, &kid);
+        return note_launch(e, kid);
+    }
     case TLIBTTM_SCHED_COLS_TMA:
         return note_launch(launch_stream(v, dtype, s), v.inner == 1 ? K_STREAM_ROWS : K_STREAM_COLS);
     case TLIBTTM_SCHED_SIMT_SPLIT:
@@ -1393,6 +1413,8 @@ int tlibttm_set_precision(int precision)
 int tlibttm_get_precision(void) { return g_precision.load(); }
 
 const char* tlibttm_last_kernel(void) { return g_last_kernel; }
+
+const char* tlibttm_last_variant(void) { return g_last_variant; }
 
 unsigned long long tlibttm_launch_count(int reset)
 {

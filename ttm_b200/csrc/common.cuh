@@ -153,10 +153,13 @@ enum KernelId : int {
     K_TC_PAIR,
     K_BVEC,
     K_TC_FP8_PAIR,
+    K_FEW_COLUMNS,   // of the colvec family
+    K_ROWWARP,       // of the rowdot family
     K_COUNT
 };
 
-const char* kernel_name(int id);
+const char* kernel_name(int id);      // the family's name
+const char* kernel_variant(int id);   // the kernel's own
 
 // Launchers (simt_kernels.cu). Return cudaSuccess or the launch error.
 // The slice-GEMM; when its tiles cannot fill the GPU and n_q is long, the K loop is split over
@@ -179,10 +182,13 @@ bool bvec_supported(const View3& v);
 // The same split for small m (m <= kSmallM): few rows and n_q >= 4096.
 bool bvec_small_supported(const View3& v);
 cudaError_t launch_bvec(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr);
-cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s);
+// *kid: the kernel launched (K_COLVEC or K_FEW_COLUMNS; K_ROWDOT or K_ROWWARP).
+cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s, int* kid);
 // colvec with an explicit l split over warps (1 or 8).
-cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s);
-cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s);
+cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s, int* kid);
+cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s, int* kid);
+// Whether launch_colvec splits l over eight warps.
+bool colvec_splits(const View3& v, int dtype);
 cudaError_t launch_strided(const StridedProblem& sp, int dtype, cudaStream_t s);
 // Sets n elements at p (float when dtype == 0, else double) to v.
 cudaError_t launch_fill(void* p, int64_t n, int dtype, double v, cudaStream_t s);

@@ -963,7 +963,7 @@ bool one_chain_before(const View3& v, int dtype, int split)
     const bool tma = rows * v.nq * (16 / rv) >= kStreamMinBytes && stream_supported(v, dtype);
     if (v.inner == 1) return tma ? rows >= 148 * 512 && v.nq <= 1024 : rows > kBvecSmallMaxRows || v.nq < 1024;
     if (tma) return v.nq < 160 || (rows >= 2 * 148 * 256 * rv && v.nq <= 1024);
-    const int64_t w = aligned16(v.a) && aligned16(v.c) && v.inner % rv == 0 ? rv : 1;
+    const int64_t w = aligned16(v.a) && aligned16(v.c) && v.inner % rv == 0 ? rv : 1;   // rows per lane
     return rows > kColSplitWarps * 32 * w;
 }
 
@@ -1135,14 +1135,6 @@ cudaError_t colvec_dispatch_ls(const View3& v, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// Few rows (fewer than ~32 warps of rows per SM): split the l loop across warps.
-template <typename T, int W>
-cudaError_t colvec_dispatch_w(const View3& v, cudaStream_t s)
-{
-    const int64_t row_warps = ceil_div(v.outer * v.inner, 32 * W);
-    return row_warps < kColSplitWarps ? colvec_dispatch_ls<T, W, 8>(v, s) : colvec_dispatch_ls<T, W, 1>(v, s);
-}
-
 template <int TN>
 cudaError_t few_columns_launch(const View3& v, cudaStream_t s)
 {
@@ -1169,16 +1161,27 @@ bool few_columns_takes(const View3& v)
            16 * v.inner >= (v.m <= 4 ? 8 : 9) * room;
 }
 
+cudaError_t few_columns_dispatch(const View3& v, cudaStream_t s)
+{
+    return v.m <= 1 ? few_columns_launch<1>(v, s) : v.m <= 2 ? few_columns_launch<2>(v, s)
+         : v.m <= 4 ? few_columns_launch<4>(v, s) : few_columns_launch<8>(v, s);
+}
+
+// Rows per lane of the column kernel: 16 bytes of them, or one.
 template <typename T>
-cudaError_t colvec_dispatch(const View3& v, cudaStream_t s)
+int colvec_rows_per_lane(const View3& v)
 {
     constexpr int RV = 16 / sizeof(T);
-    const bool vec = aligned16(v.a) && aligned16(v.c) && (v.inner % RV == 0);
-    if constexpr (sizeof(T) == 4)
-        if (few_columns_takes(v))
-            return v.m <= 1 ? few_columns_launch<1>(v, s) : v.m <= 2 ? few_columns_launch<2>(v, s)
-                 : v.m <= 4 ? few_columns_launch<4>(v, s) : few_columns_launch<8>(v, s);
-    return vec ? colvec_dispatch_w<T, RV>(v, s) : colvec_dispatch_w<T, 1>(v, s);
+    return aligned16(v.a) && aligned16(v.c) && v.inner % RV == 0 ? RV : 1;
+}
+
+template <typename T>
+cudaError_t colvec_dispatch(const View3& v, int ls, cudaStream_t s)
+{
+    constexpr int RV = 16 / sizeof(T);
+    if (colvec_rows_per_lane<T>(v) == RV)
+        return ls == 8 ? colvec_dispatch_ls<T, RV, 8>(v, s) : colvec_dispatch_ls<T, RV, 1>(v, s);
+    return ls == 8 ? colvec_dispatch_ls<T, 1, 8>(v, s) : colvec_dispatch_ls<T, 1, 1>(v, s);
 }
 
 template <typename T, bool VEC>
@@ -1262,7 +1265,7 @@ bool rowwarp_takes(const View3& v)
 }
 
 template <typename T>
-cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s)
+cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s, int* kid)
 {
     const int64_t span = 64 / (int64_t)sizeof(T);
     const int64_t mb = v.m <= 1 ? 1 : v.m <= 2 ? 2 : v.m <= 4 ? 4 : v.m <= 8 ? 8 : 16;
@@ -1286,9 +1289,11 @@ cudaError_t rowdot_dispatch(const View3& v, cudaStream_t s)
     constexpr int RV = 16 / sizeof(T);
     const bool vec = aligned16(v.a) && (v.nq % RV == 0);
     if constexpr (sizeof(T) == 4)
-        if (!vec && rowwarp_takes(v))
+        if (!vec && rowwarp_takes(v)) {
+            *kid = K_ROWWARP;
             return v.m <= 1 ? rowwarp_launch<1>(v, s) : v.m <= 2 ? rowwarp_launch<2>(v, s)
                  : v.m <= 4 ? rowwarp_launch<4>(v, s) : rowwarp_launch<8>(v, s);
+        }
     return vec ? rowdot_dispatch_v<T, true>(v, s) : rowdot_dispatch_v<T, false>(v, s);
 }
 
@@ -1713,27 +1718,33 @@ cudaError_t launch_bvec(const View3& v, int dtype, cudaStream_t s, int* launches
     return dtype == 0 ? bvec_dispatch<float>(v, sms, s, launches) : bvec_dispatch<double>(v, sms, s, launches);
 }
 
-cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s)
+// Few rows (fewer than ~32 warps of rows per SM): the l loop is split across warps.
+bool colvec_splits(const View3& v, int dtype)
 {
-    return dtype == 0 ? colvec_dispatch<float>(v, s) : colvec_dispatch<double>(v, s);
+    if (dtype == 0 && few_columns_takes(v)) return false;
+    const int64_t w = dtype == 0 ? colvec_rows_per_lane<float>(v) : colvec_rows_per_lane<double>(v);
+    return ceil_div(v.outer * v.inner, 32 * w) < kColSplitWarps;
 }
 
-cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s)
+cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s, int* kid)
 {
-    constexpr int RF = 4, RD = 2;
-    if (dtype == 0) {
-        const bool vec = aligned16(v.a) && aligned16(v.c) && (v.inner % RF == 0);
-        if (vec) return ls == 8 ? colvec_dispatch_ls<float, RF, 8>(v, s) : colvec_dispatch_ls<float, RF, 1>(v, s);
-        return ls == 8 ? colvec_dispatch_ls<float, 1, 8>(v, s) : colvec_dispatch_ls<float, 1, 1>(v, s);
+    if (dtype == 0 && few_columns_takes(v)) {
+        *kid = K_FEW_COLUMNS;
+        return few_columns_dispatch(v, s);
     }
-    const bool vec = aligned16(v.a) && aligned16(v.c) && (v.inner % RD == 0);
-    if (vec) return ls == 8 ? colvec_dispatch_ls<double, RD, 8>(v, s) : colvec_dispatch_ls<double, RD, 1>(v, s);
-    return ls == 8 ? colvec_dispatch_ls<double, 1, 8>(v, s) : colvec_dispatch_ls<double, 1, 1>(v, s);
+    return launch_colvec_ls(v, dtype, colvec_splits(v, dtype) ? 8 : 1, s, kid);
 }
 
-cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s)
+cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s, int* kid)
 {
-    return dtype == 0 ? rowdot_dispatch<float>(v, s) : rowdot_dispatch<double>(v, s);
+    *kid = K_COLVEC;
+    return dtype == 0 ? colvec_dispatch<float>(v, ls, s) : colvec_dispatch<double>(v, ls, s);
+}
+
+cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s, int* kid)
+{
+    *kid = K_ROWDOT;
+    return dtype == 0 ? rowdot_dispatch<float>(v, s, kid) : rowdot_dispatch<double>(v, s, kid);
 }
 
 void grouped_columns(int64_t m, int dtype, int64_t* tiles, int* cols)

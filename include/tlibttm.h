@@ -143,7 +143,9 @@ int tlibttm_ttm_f32_bf16x3_noalloc(unsigned q, unsigned p,
 enum tlibttm_schedule {
     TLIBTTM_SCHED_HEURISTIC = 0,   /* the planner's built-in choice (as tlibttm_ttm_ex, PLAIN) */
     TLIBTTM_SCHED_SIMT_GEMM = 1,   /* slice-GEMM on FFMA / FP64 mma, any m */
-    TLIBTTM_SCHED_COLS = 2,        /* small-m kernel for strided fibres, rows spread over warps (m <= 16, inner >= 2) */
+    TLIBTTM_SCHED_COLS = 2,        /* small-m kernel for strided fibres, rows spread over warps (m <= 16, inner >= 2);
+                                      float, m <= 8, rows off 16-byte boundaries: the few-column kernel where its
+                                      tiles are filled */
     TLIBTTM_SCHED_COLS_SPLIT = 3,  /* small-m kernel for strided fibres, l split over 8 warps (m <= 16, inner >= 2) */
     TLIBTTM_SCHED_ROWS = 4,        /* small-m kernel for contiguous fibres (m <= 16, q == pia[0]) */
     TLIBTTM_SCHED_TC_BF16X3 = 5,   /* tensor-core bf16x3 on single SMs, float only (FP32-accurate, not exact; m > 16) */

@@ -1,5 +1,5 @@
 """The few-column and warp-per-rows kernels run on their side of each edge of their rules, and the kernels
-they belong with on the other."""
+they belong with on the other, for the default call; the tuner's schedules reach them too."""
 import ctypes as C
 
 import pytest
@@ -42,6 +42,9 @@ def _call(cuda, outer, nq, inner, m, sched=None, shift=0, dtype="float32"):
 def test_few_columns_rule(cuda, outer, nq, inner, m, shift, variant):
     got, err = _call(cuda, outer, nq, inner, m, shift=shift)
     assert got == variant and err <= 2e-6
+    # the tuner's schedule with rows spread over warps takes it by the same rule, the l-split one never
+    assert _call(cuda, outer, nq, inner, m, sched=2, shift=shift)[0] == variant
+    assert _call(cuda, outer, nq, inner, m, sched=3, shift=shift)[0] == "colvec"
 
 
 # its rule: float, m <= 8, fibres off 16-byte boundaries of 32 / 96 / 256 (m <= 2 / 4 / 8) to 1024

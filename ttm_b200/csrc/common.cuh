@@ -184,7 +184,7 @@ bool bvec_small_supported(const View3& v);
 cudaError_t launch_bvec(const View3& v, int dtype, cudaStream_t s, int* launches = nullptr);
 // *kid: the kernel launched (K_COLVEC or K_FEW_COLUMNS; K_ROWDOT or K_ROWWARP).
 cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s, int* kid);
-// colvec with an explicit l split over warps (1 or 8).
+// colvec with an explicit l split over warps (1 or 8); 1: the few-column kernel where it takes the problem.
 cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s, int* kid);
 cudaError_t launch_rowdot(const View3& v, int dtype, cudaStream_t s, int* kid);
 // Whether launch_colvec splits l over eight warps.

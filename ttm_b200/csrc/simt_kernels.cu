@@ -1728,15 +1728,15 @@ bool colvec_splits(const View3& v, int dtype)
 
 cudaError_t launch_colvec(const View3& v, int dtype, cudaStream_t s, int* kid)
 {
-    if (dtype == 0 && few_columns_takes(v)) {
-        *kid = K_FEW_COLUMNS;
-        return few_columns_dispatch(v, s);
-    }
     return launch_colvec_ls(v, dtype, colvec_splits(v, dtype) ? 8 : 1, s, kid);
 }
 
 cudaError_t launch_colvec_ls(const View3& v, int dtype, int ls, cudaStream_t s, int* kid)
 {
+    if (dtype == 0 && ls == 1 && few_columns_takes(v)) {
+        *kid = K_FEW_COLUMNS;
+        return few_columns_dispatch(v, s);
+    }
     *kid = K_COLVEC;
     return dtype == 0 ? colvec_dispatch<float>(v, ls, s) : colvec_dispatch<double>(v, ls, s);
 }

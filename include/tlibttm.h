@@ -171,6 +171,12 @@ int tlibttm_ttm_sched(int dtype, int schedule, unsigned q, unsigned p,
 int tlibttm_schedule_valid(int dtype, int schedule, unsigned q, unsigned p, const size_t* na, const size_t* pia,
                            size_t m);
 
+/* The schedule that a call of tlibttm_ttm_ex with this precision (PLAIN or AUTO) takes for a dense TTM whose
+ * operands lie on 16-byte boundaries; HEURISTIC where what it takes has no schedule of its own; -1 for
+ * invalid arguments. */
+int tlibttm_default_schedule(int dtype, int precision, unsigned q, unsigned p, const size_t* na, const size_t* pia,
+                             size_t m);
+
 /*
  * Kernels of the learned schedule selector (no counterpart in the reference):
  * a multilayer perceptron over float32 device buffers, activations

@@ -304,6 +304,15 @@ struct SplitSpace {
     void* p = nullptr;
 };
 
+// The single-SM tensor-core kernel has no K split: when its tiles fill less than half the GPU and the l
+// range is long, the split-K SIMT GEMM (exact) is the faster choice.
+bool tc_leaves_sms_idle(const View3& v)
+{
+    int sms = 0;
+    return !tc_pair_supported(v) && v.nq >= 2048 &&
+           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0) == cudaSuccess && tc_single_tiles(v) * 2 < sms;
+}
+
 // All operands are device memory: enqueue on stream s. `space`: the plan's, null for a single call.
 int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t stream_min_bytes = kStreamMinBytes,
                const SplitSpace* space = nullptr)
@@ -397,13 +406,7 @@ int run_device(const Args& x, Plan& pl, int precision, cudaStream_t s, int64_t s
         return note_launch(e, K_BVEC);
     }
     if (precision != TLIBTTM_PREC_PLAIN && tc_supported(v, precision)) {
-        // The single-SM tensor-core kernel has no K split: when its tiles fill less than half the
-        // GPU and the l range is long, the split-K SIMT GEMM (exact) is the faster choice.
-        int sms = 0;
-        const bool few = !tc_pair_supported(v) && v.nq >= 2048 &&
-                         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0) == cudaSuccess &&
-                         tc_single_tiles(v) * 2 < sms;
-        if (!few) {
+        if (!tc_leaves_sms_idle(v)) {
             int kid = K_NONE;
             cudaError_t e = launch_tc(v, precision, s, &kid);
             if (e == cudaSuccess && kid == K_TC_BF16X3) ++g_launches;   // the operand-split kernel that precedes it
@@ -759,11 +762,7 @@ int launches_of(const Single& sg, int dtype, int precision)
     if (pr == TLIBTTM_PREC_FP8 || pr == TLIBTTM_PREC_OZAKI) return tc8_launches(sg.pl.v, pr);
     if (bvec_supported(sg.pl.v)) return 2;
     if (pr != TLIBTTM_PREC_PLAIN && tc_supported(sg.pl.v, pr)) {
-        int sms = 0;
-        const bool few = !tc_pair_supported(sg.pl.v) && sg.pl.v.nq >= 2048 &&
-                         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0) == cudaSuccess &&
-                         tc_single_tiles(sg.pl.v) * 2 < sms;
-        if (!few) return tc_pair_supported(sg.pl.v) ? 1 : 2;
+        if (!tc_leaves_sms_idle(sg.pl.v)) return tc_pair_supported(sg.pl.v) ? 1 : 2;
     }
     return simt_gemm_launch_count(sg.pl.v, dtype);
 }
@@ -1009,15 +1008,14 @@ int tlibttm_ttm_sched(int dtype, int schedule, unsigned q, unsigned p, const voi
     }
 }
 
-int tlibttm_schedule_valid(int dtype, int schedule, unsigned q, unsigned p, const size_t* na, const size_t* pia,
-                           size_t m)
+// The dense view of a problem given by its metadata, operands on 16-byte boundaries; false if invalid.
+static bool metadata_view(unsigned q, unsigned p, const size_t* na, const size_t* pia, size_t m, View3& v)
 {
-    if (!na || !pia || p == 0 || q == 0 || q > p) return 0;
+    if (!na || !pia || p == 0 || q == 0 || q > p) return false;
     if (!tlib::ttm::detail::is_valid_shape(na, na + p) || !tlib::ttm::detail::is_valid_layout(pia, pia + p) || m == 0)
-        return 0;
+        return false;
     unsigned qh = 0;
     while (pia[qh] != q) ++qh;
-    View3 v{};
     v.inner = 1;
     v.outer = 1;
     for (unsigned r = 0; r < qh; ++r) v.inner *= (int64_t)na[pia[r] - 1];
@@ -1026,7 +1024,38 @@ int tlibttm_schedule_valid(int dtype, int schedule, unsigned q, unsigned p, cons
     v.m = (int64_t)m;
     alignas(16) static const float aligned_probe[4] = {0, 0, 0, 0};
     v.a = aligned_probe;   // alignment of the real operands is checked again when the schedule runs
-    return sched_valid_view(dtype, schedule, v) ? 1 : 0;
+    return true;
+}
+
+int tlibttm_schedule_valid(int dtype, int schedule, unsigned q, unsigned p, const size_t* na, const size_t* pia,
+                           size_t m)
+{
+    View3 v{};
+    return metadata_view(q, p, na, pia, m, v) && sched_valid_view(dtype, schedule, v) ? 1 : 0;
+}
+
+int tlibttm_default_schedule(int dtype, int precision, unsigned q, unsigned p, const size_t* na, const size_t* pia,
+                             size_t m)
+{
+    View3 v{};
+    if ((dtype != TLIBTTM_F32 && dtype != TLIBTTM_F64) ||
+        (precision != TLIBTTM_PREC_PLAIN && precision != TLIBTTM_PREC_AUTO) || !metadata_view(q, p, na, pia, m, v))
+        return -1;
+    if (v.m <= kSmallM) {
+        const int64_t a_bytes = v.outer * v.nq * v.inner * (dtype == TLIBTTM_F32 ? 4 : 8);
+        const bool tma = a_bytes >= kStreamMinBytes && stream_supported(v, dtype);
+        const SmallGemm gemm = small_m_takes_gemm(v, dtype, tma, true);
+        if (gemm != SmallGemm::No) return gemm == SmallGemm::Split ? TLIBTTM_SCHED_SIMT_SPLIT : TLIBTTM_SCHED_SIMT_GEMM;
+        if (!tma && bvec_small_supported(v)) return TLIBTTM_SCHED_HEURISTIC;   // no schedule of its own
+        if (v.inner == 1) return tma && v.nq >= 16 ? TLIBTTM_SCHED_COLS_TMA : TLIBTTM_SCHED_ROWS;
+        if (tma) return TLIBTTM_SCHED_COLS_TMA;
+        return colvec_splits(v, dtype) ? TLIBTTM_SCHED_COLS_SPLIT : TLIBTTM_SCHED_COLS;
+    }
+    if (bvec_supported(v)) return TLIBTTM_SCHED_BVEC;
+    if (precision == TLIBTTM_PREC_AUTO && dtype == TLIBTTM_F32 && tc_supported(v, TLIBTTM_PREC_BF16X3) &&
+        !tc_leaves_sms_idle(v))
+        return tc_pair_supported(v) ? TLIBTTM_SCHED_TC_BF16X3_PAIR : TLIBTTM_SCHED_TC_BF16X3;
+    return TLIBTTM_SCHED_SIMT_GEMM;
 }
 
 // No counterpart in the reference: the bf16x3 contraction without any device

@@ -56,6 +56,9 @@ def _declare(L):
     L.tlibttm_schedule_valid.restype = C.c_int
     L.tlibttm_schedule_valid.argtypes = [C.c_int, C.c_int, C.c_uint, C.c_uint, C.POINTER(C.c_size_t),
                                          C.POINTER(C.c_size_t), C.c_size_t]
+    L.tlibttm_default_schedule.restype = C.c_int
+    L.tlibttm_default_schedule.argtypes = [C.c_int, C.c_int, C.c_uint, C.c_uint, C.POINTER(C.c_size_t),
+                                           C.POINTER(C.c_size_t), C.c_size_t]
     vp, i, f = C.c_void_p, C.c_int, C.c_float
     L.tlibttm_mlp_forward.restype = i
     L.tlibttm_mlp_forward.argtypes = [vp, vp, vp, vp, i, i, i, i, vp]
@@ -392,26 +395,13 @@ def evaluate(model, tuner, test, margin=0.15):
 
 
 def _heuristic_in(pr, allowed):
-    """The planner's default choice for a problem (plain for 'exact', auto for 'fp32_accurate')."""
-    inner, nq, outer = geometry(pr["na"], pr["pia"], pr["q"])
-    es = 4 if dtype_of(pr) == _lib.F32 else 8
-    if pr["m"] <= 16:
-        if inner == 1:
-            big = math.prod(pr["na"]) * es >= 64 << 20
-            return 6 if (6 in allowed and big and nq >= 16 and valid_mask(pr)[5]) else 4
-        if 6 in allowed and math.prod(pr["na"]) * es >= 64 << 20 and valid_mask(pr)[5]:
-            return 6
-        rv = 16 // es
-        w = rv if inner % rv == 0 else 1
-        return 3 if math.ceil(inner * outer / (32 * w)) < 148 * 32 else 2
-    ok = valid_mask(pr)
-    if 9 in allowed and ok[8]:
-        return 9
-    if 7 in allowed and ok[6]:
-        return 7
-    if 5 in allowed and ok[4]:
-        return 5
-    return 1
+    """The planner's default choice for a problem (plain for 'exact', auto for 'fp32_accurate'), asked of
+    the library itself."""
+    s = lib().tlibttm_default_schedule(dtype_of(pr), _lib.PREC_AUTO if 5 in allowed else _lib.PREC_PLAIN, pr["q"], pr["p"],
+                                       _lib.sz(pr["na"]), _lib.sz(pr["pia"]), pr["m"])
+    if s in allowed and valid_mask(pr)[s - 1]:
+        return s
+    raise ValueError(f"the planner's choice for {pr['na']} q={pr['q']} m={pr['m']} is not among the schedules")
 
 
 _default = {}

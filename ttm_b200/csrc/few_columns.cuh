@@ -46,9 +46,9 @@ __device__ __forceinline__ void copy4(void* dst, const void* src, bool ok)
                  : "memory");
 }
 
-// Tile `t` of outer * ceil(inner / 256). A warp's chains are `chain` + 1 stages (a power of two) of four l
-// of its own.
-template <int TN, bool BCM>
+// Tile `t` of outer * ceil(inner / 256). CHAINS: a warp's chains are `chain` + 1 stages (a power of two) of
+// four l of its own; else it has one.
+template <int TN, bool BCM, bool CHAINS>
 __device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<TN>& sm)
 {
     const float* __restrict__ A = static_cast<const float*>(v.a);
@@ -89,11 +89,14 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<
     // this warp's l (warp, warp + 4, ...) all have one residue mod 4, and so one shift: BK inner and
     // BM are multiples of four
     const int sh = (int)((((uint32_t)k * (uint32_t)nq + (uint32_t)warp) * (uint32_t)inner) & 3u);
-    unsigned long long acc[RPL / 2][TN], sum[RPL / 2][TN];   // rows 64 p + lane and 64 p + 32 + lane
+    unsigned long long acc[RPL / 2][TN], sum[CHAINS ? RPL / 2 : 1][TN];   // rows 64 p + lane and 64 p + 32 + lane
 #pragma unroll
     for (int p = 0; p < RPL / 2; ++p)
 #pragma unroll
-        for (int q = 0; q < TN; ++q) acc[p][q] = sum[p][q] = 0ull;
+        for (int q = 0; q < TN; ++q) {
+            acc[p][q] = 0ull;
+            if (CHAINS) sum[p][q] = 0ull;
+        }
     int rd = 0, wr = ST - 1;
     const int nk = (int)ceil_div(nq, BK);
     for (int kt = 0; kt < nk; ++kt) {
@@ -117,7 +120,7 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<
                 for (int p = 0; p < RPL / 2; ++p) ffma2(acc[p][q], a[p], bq);
             }
         }
-        if ((kt & chain) == chain || kt + 1 == nk) {   // a chain ends
+        if (CHAINS && (kt & chain) == chain) {   // a chain ends
 #pragma unroll
             for (int p = 0; p < RPL / 2; ++p)
 #pragma unroll
@@ -128,6 +131,12 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<
         }
         rd = rd + 1 == ST ? 0 : rd + 1;
         wr = wr + 1 == ST ? 0 : wr + 1;
+    }
+    if (CHAINS) {
+#pragma unroll
+        for (int p = 0; p < RPL / 2; ++p)
+#pragma unroll
+            for (int q = 0; q < TN; ++q) acc[p][q] = add2(sum[p][q], acc[p][q]);
     }
     // the warps' sums, up to four columns at a time: thread t adds rows t and t + 128
     float* __restrict__ C = static_cast<float*>(v.c) + k * m * inner + i0;
@@ -140,8 +149,8 @@ __device__ __forceinline__ void tile(const View3& v, int64_t t, int chain, Smem<
         for (int q = 0; q < QC; ++q)
 #pragma unroll
             for (int p = 0; p < RPL / 2; ++p) {
-                sm.red[warp][q][64 * p + lane] = pair_lo(sum[p][q0 + q]);
-                sm.red[warp][q][64 * p + 32 + lane] = pair_hi(sum[p][q0 + q]);
+                sm.red[warp][q][64 * p + lane] = pair_lo(acc[p][q0 + q]);
+                sm.red[warp][q][64 * p + 32 + lane] = pair_hi(acc[p][q0 + q]);
             }
         __syncthreads();
 #pragma unroll

@@ -382,11 +382,11 @@ __global__ void __launch_bounds__(256) colvec_async_kernel(View3 v)
 }
 
 // few_columns.cuh: rows of i off 16-byte boundaries, m <= 8, long l ranges.
-template <int TN, bool BCM>
+template <int TN, bool BCM, bool CHAINS>
 __global__ void __launch_bounds__(few::NT, 3) few_columns_kernel(View3 v, int chain)
 {
     extern __shared__ __align__(16) unsigned char few_smem[];
-    few::tile<TN, BCM>(v, blockIdx.x, chain, *reinterpret_cast<few::Smem<TN>*>(few_smem));
+    few::tile<TN, BCM, CHAINS>(v, blockIdx.x, chain, *reinterpret_cast<few::Smem<TN>*>(few_smem));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1139,12 +1139,13 @@ template <int TN>
 cudaError_t few_columns_launch(const View3& v, cudaStream_t s)
 {
     constexpr int smem = (int)sizeof(few::Smem<TN>);
-    const auto kernel = v.b_cm ? few_columns_kernel<TN, true> : few_columns_kernel<TN, false>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     // the column kernel would split l over eight warps below this many rows
     const bool chains = v.outer * v.inner <= kColSplitWarps * 32;
-    const int chain = !chains ? 0x7fffffff : v.nq < 128 ? 1 : 3;
+    const auto kernel = v.b_cm ? (chains ? few_columns_kernel<TN, true, true> : few_columns_kernel<TN, true, false>)
+                               : (chains ? few_columns_kernel<TN, false, true> : few_columns_kernel<TN, false, false>);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int chain = v.nq < 128 ? 1 : 3;
     kernel<<<(unsigned)(v.outer * ceil_div(v.inner, few::BM)), few::NT, smem, s>>>(v, chain);
     return cudaGetLastError();
 }

@@ -188,75 +188,32 @@ struct Digits {
     }
 };
 
-// Exponents and digits of A in one launch (ozaki): a block takes 32 rows, finds their maxima, then
+// Exponents and digits of A in one launch (ozaki): a block takes some rows, finds their maxima, then
 // reads them again (from L2: 148 SMs x a few blocks x 32 rows) and writes the image as slice_kernel
 // does. Bound by reading A and writing 7/8 of its bytes; on A 256^3 the two kernels took 39 and 125
 // us, the second on 64-bit digit arithmetic, this one 70 us (contiguous fibres 93).
+// A block takes 32 rows, four chunks of 32 l of each at a time. KC = 1, 2 or 4: rows of at most so many
+// chunks, 128 / KC of them per block, whose 16 l of a thread stay in registers between the maximum and the
+// digits, so that A is read once (KC = 0: longer rows). With 32 rows throughout, threads had no digits to
+// cut below four chunks: rows of i, n_q = 19, 1.76M of them 734 us against 424 of the two kernels; now 159.
+template <int KC>
 __global__ void __launch_bounds__(256, 2) exponent_slice_kernel(RowView v, int64_t r0, int64_t nrows, int* __restrict__ ex,
                                                                int kchunks, uint8_t* __restrict__ img)
 {
+    constexpr int RB = KC ? 128 / KC : 32;
     __shared__ double red[8][32];
-    __shared__ int es[32];
+    __shared__ int es[RB];
     const double* a = static_cast<const double*>(v.base);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t b0 = (int64_t)blockIdx.x * 32;   // first row of the block within the chunk
-    if (v.ls == 1) {
-        // contiguous fibres: a warp reads four rows, lanes along l
-        double mx[4] = {0.0, 0.0, 0.0, 0.0};
-        const double* p[4];
-        bool ok[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int64_t rr = b0 + warp * 4 + r;
-            ok[r] = rr < nrows;
-            p[r] = a + (ok[r] ? row_off(v, r0 + rr) : 0);
-        }
-#pragma unroll 4
-        for (int64_t l = lane; l < v.nq; l += 32) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) mx[r] = fmax(mx[r], ok[r] ? fabs(__ldg(p[r] + l)) : 0.0);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx[r] = fmax(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
-            if (lane == 0) {
-                int e = 0;
-                if (mx[r] > 0.0) frexp(mx[r], &e);
-                es[warp * 4 + r] = e;
-            }
-        }
-    } else {
-        // a lane reads one row; the warps split l
-        double mx = 0.0;
-        if (b0 + lane < nrows) {
-            const double* p = a + row_off(v, r0 + b0 + lane);
-#pragma unroll 8
-            for (int64_t l = warp; l < v.nq; l += 8) mx = fmax(mx, fabs(__ldg(p + l * v.ls)));
-        }
-        red[warp][lane] = mx;
-        __syncthreads();
-        if (warp == 0) {
-#pragma unroll
-            for (int w = 1; w < 8; ++w) mx = fmax(mx, red[w][lane]);
-            int e = 0;
-            if (mx > 0.0) frexp(mx, &e);
-            es[lane] = e;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < 32 && b0 + threadIdx.x < nrows) ex[b0 + threadIdx.x] = es[threadIdx.x];
+    const int64_t b0 = (int64_t)blockIdx.x * RB;   // first row of the block within the chunk
     // thread: half c of a 32-l chunk of one row; neighbouring lanes the two halves of a row
-    const int c = threadIdx.x & 1, row = (threadIdx.x >> 1) & 31;
+    const int c = threadIdx.x & 1, row = (threadIdx.x >> 1) & (RB - 1), kc0 = threadIdx.x / (2 * RB);
     const int64_t rr = b0 + row, tile = b0 / kRows;
     const bool rv = rr < nrows;
     const double* p = a + (rv ? row_off(v, r0 + rr) : 0);
-    const int sh = 7 * kOzakiSlices - es[row];
     const bool vec = v.ls == 1 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0;   // the thread's 16 l contiguous
     const uint32_t off = kmaj_sw32_off((uint32_t)(rr - tile * kRows), (uint32_t)c);
-    for (int kc = threadIdx.x >> 6; kc < kchunks; kc += 4) {
+    auto load = [&](int kc, double (&x)[16]) {
         const int64_t l0 = (int64_t)kc * kLChunk + c * 16;
-        double x[16];
         if (vec && rv && l0 + 16 <= v.nq) {
 #pragma unroll
             for (int t = 0; t < 16; t += 2) {
@@ -268,9 +225,80 @@ __global__ void __launch_bounds__(256, 2) exponent_slice_kernel(RowView v, int64
 #pragma unroll
             for (int t = 0; t < 16; ++t) x[t] = rv && l0 + t < v.nq ? __ldg(p + (l0 + t) * v.ls) : 0.0;
         }
+    };
+    auto exponent = [](double mx) {
+        int e = 0;
+        if (mx > 0.0) frexp(mx, &e);
+        return e;
+    };
+    auto digits = [&](int kc, const double (&x)[16], int e) {
         Digits d;
-        d.set(x, sh);
+        d.set(x, 7 * kOzakiSlices - e);
         d.store(img + (size_t)((tile * kchunks + kc) * kOzakiSlices) * kBlock + off, kBlock);
+    };
+    if constexpr (KC != 0) {
+        double x[16], mx = 0.0;
+        load(kc0, x);   // zeros past the row
+#pragma unroll
+        for (int t = 0; t < 16; ++t) mx = fmax(mx, fabs(x[t]));
+        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        if constexpr (KC > 1) {
+            double* most = &red[0][0];   // [KC][RB]
+            if (c == 0) most[kc0 * RB + row] = mx;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < KC; ++k) mx = fmax(mx, most[k * RB + row]);
+        }
+        const int e = exponent(mx);
+        if (c == 0 && kc0 == 0 && rv) ex[rr] = e;
+        if (kc0 < kchunks) digits(kc0, x, e);
+    } else {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (v.ls == 1) {
+            // contiguous fibres: a warp reads four rows, lanes along l
+            double mx[4] = {0.0, 0.0, 0.0, 0.0};
+            const double* q[4];
+            bool ok[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                ok[r] = b0 + warp * 4 + r < nrows;
+                q[r] = a + (ok[r] ? row_off(v, r0 + b0 + warp * 4 + r) : 0);
+            }
+#pragma unroll 4
+            for (int64_t l = lane; l < v.nq; l += 32) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) mx[r] = fmax(mx[r], ok[r] ? fabs(__ldg(q[r] + l)) : 0.0);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) mx[r] = fmax(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], o));
+                if (lane == 0) es[warp * 4 + r] = exponent(mx[r]);
+            }
+        } else {
+            // a lane reads one row; the warps split l
+            double mx = 0.0;
+            if (b0 + lane < nrows) {
+                const double* q = a + row_off(v, r0 + b0 + lane);
+#pragma unroll 8
+                for (int64_t l = warp; l < v.nq; l += 8) mx = fmax(mx, fabs(__ldg(q + l * v.ls)));
+            }
+            red[warp][lane] = mx;
+            __syncthreads();
+            if (warp == 0) {
+#pragma unroll
+                for (int w = 1; w < 8; ++w) mx = fmax(mx, red[w][lane]);
+                es[lane] = exponent(mx);
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 32 && b0 + threadIdx.x < nrows) ex[b0 + threadIdx.x] = es[threadIdx.x];
+        const int e = es[row];
+        for (int kc = kc0; kc < kchunks; kc += 4) {
+            double x[16];
+            load(kc, x);
+            digits(kc, x, e);
+        }
     }
 }
 
@@ -710,7 +738,12 @@ cudaError_t launch_tc8(const View3& v, int precision, int dtype, cudaStream_t s,
             if (e == cudaSuccess) e = launch_slices<float, MODE_FP8>(av, r0, nr, aexp, p.S, kRows, p.kchunks, aimg, s);
         } else {
             const int64_t tiles = (nr + kRows - 1) / kRows;
-            exponent_slice_kernel<<<(unsigned)(tiles * (kRows / 32)), 256, 0, s>>>(av, r0, nr, aexp, p.kchunks, aimg);
+            const auto kernel = p.kchunks == 1   ? exponent_slice_kernel<1>
+                                : p.kchunks == 2 ? exponent_slice_kernel<2>
+                                : p.kchunks <= 4 ? exponent_slice_kernel<4>
+                                                 : exponent_slice_kernel<0>;
+            const int rb = p.kchunks == 1 ? 128 : p.kchunks == 2 ? 64 : 32;   // rows per block
+            kernel<<<(unsigned)(tiles * (kRows / rb)), 256, 0, s>>>(av, r0, nr, aexp, p.kchunks, aimg);
             e = cudaGetLastError();
         }
         if (e != cudaSuccess) break;

@@ -6,8 +6,8 @@
 // TM x TN outputs. Accumulators pair neighbouring rows, which come from shared memory as 64-bit
 // halves of a 16-byte load; each column value is duplicated once for TM / 2 pairs. Widths are whole
 // builds in groups of eight columns, so that padding of m is not multiplied (m = 100: two tiles of
-// 56). A warp is 8 x 4 threads: its 16-byte loads of A and B cover at most 128 distinct bytes (one
-// wavefront each), its stores of C 128 contiguous bytes.
+// 56). A warp is 8 x 4 threads (4 x 8 for wide tiles of contiguous fibres): its 16-byte loads of A and B cover
+// at most 128 distinct bytes (one wavefront each), its stores of C 128 contiguous bytes.
 // A and B tiles of 16 l go through a ring of ST shared-memory stages filled with cp.async, B as
 // [l][j], A as [l][row] for rows of i and as [row][l] for contiguous fibres (whose accumulators pair
 // neighbouring columns instead).
@@ -93,7 +93,7 @@ constexpr int kFoldChain = 8, kFoldStages = 8;
 
 // A thread's outputs where rows of i are contiguous: acc[p][q] holds rows 2 p and 2 p + 1 of its TM
 // (chunks of four rows 128 apart), column q.
-template <int TX, int TM, int NA, bool FOLD>
+template <int TX, int TM, int NA, bool FOLD, bool HALF>
 struct AccRows {
     unsigned long long acc[TM / 2][NA];
     static constexpr int FP = FOLD ? TM / 2 : 1, FQ = FOLD ? NA : 1;
@@ -133,12 +133,13 @@ struct AccRows {
             }
     }
 
-    // one stage (16 l)
+    // one stage: 16 l, with HALF only its first 8 where n, those left of the range, are no more
     template <int TN, int AP, int BP>
-    __device__ __forceinline__ void stage(const float (&sa)[BK][AP], const float (&sb)[BK][BP], int ty, int tx)
+    __device__ __forceinline__ void stage(const float (&sa)[BK][AP], const float (&sb)[BK][BP], int ty, int tx, int n)
     {
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
+            if (HALF && kk == BK / 2 && n <= BK / 2) break;   // the rest is padding
             unsigned long long a[TM / 2], bq[TN];
 #pragma unroll
             for (int h = 0; h < TM / 4; ++h) {
@@ -209,7 +210,7 @@ struct AccRows {
 
 // A thread's outputs where fibres are contiguous: rows 32 apart, acc[r][p] holds columns 2 p and
 // 2 p + 1 of row r, last[r] the column left over. A's rows come four l at a time.
-template <int TX, int TM, int NA, bool FOLD>
+template <int TX, int TM, int NA, bool FOLD, bool HALF>
 struct AccFibres {
     static constexpr int NP = NA / 2;   // column pairs
     unsigned long long acc[TM][NP > 0 ? NP : 1];
@@ -261,10 +262,11 @@ struct AccFibres {
     }
 
     template <int TN, int AR, int AP, int BP>
-    __device__ __forceinline__ void stage(const float (&sa)[AR][AP], const float (&sb)[BK][BP], int ty, int tx)
+    __device__ __forceinline__ void stage(const float (&sa)[AR][AP], const float (&sb)[BK][BP], int ty, int tx, int n)
     {
 #pragma unroll
         for (int k2 = 0; k2 < BK; k2 += 2) {
+            if (HALF && k2 == BK / 2 && n <= BK / 2) break;
             float2 a[TM];
 #pragma unroll
             for (int r = 0; r < TM; ++r) a[r] = *reinterpret_cast<const float2*>(&sa[r * 32 + ty][k2]);
@@ -327,9 +329,10 @@ struct AccFibres {
 
 // Tiles first, first + step, ... below `last`, l in [l_begin, l_end) of each; the stages of
 // consecutive tiles follow one another through the ring. VEC: 16-byte copies of A (alignment
-// checked by the host). EXACT: every tile has TN groups of columns, else gr.nf <= TN.
+// checked by the host). EXACT: every tile has TN groups of columns, else gr.nf <= TN. HALF: a last
+// stage of at most 8 l multiplies 8 (a branch in every stage, which costs long ranges up to 9 %).
 // The caller synchronises the block between two calls that share `sm`.
-template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM, bool EXACT>
+template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM, bool EXACT, bool HALF = false>
 __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t step, int64_t last, const ColumnGrid& gr,
                                       Smem<TX, TM, TN, ST, AK>& sm, int64_t l_begin, int64_t l_end)
 {
@@ -341,7 +344,11 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     const int64_t inner = v.inner, m = v.m, nq = v.nq;
     const int64_t M = v.outer * inner;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ty = warp / (TX / 4) * 8 + (lane & 7), tx = warp % (TX / 4) * 4 + (lane >> 3);
+    // rows of i: 8 x 4 threads a warp; contiguous fibres 4 x 8 where there are eight along the columns, so
+    // that a store of C covers whole lines
+    constexpr bool LINES = AK && TX == 8;
+    const int ty = LINES ? warp * 4 + (lane >> 3) : warp / (TX / 4) * 8 + (lane & 7);
+    const int tx = LINES ? lane & 7 : warp % (TX / 4) * 4 + (lane >> 3);
 
     // A copies of WA elements: AX along the contiguous extent (l or the rows), AY of the other per pass
     // (an extent longer than the block takes RP parts of NT copies each)
@@ -424,20 +431,20 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
     const int nk = (int)ceil_div(l_end - l_begin, BK);
 
     for (int64_t t = first; t < last; t += step) {
-        typename std::conditional<AK, AccFibres<TX, TM, TN, FOLD>, AccRows<TX, TM, TN, FOLD>>::type out;
+        typename std::conditional<AK, AccFibres<TX, TM, TN, FOLD, HALF>, AccRows<TX, TM, TN, FOLD, HALF>>::type out;
         out.clear();
         for (int kt = 0; kt < nk; ++kt) {
             asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
             __syncthreads();   // stage rd has landed for all, and all have read stage wr's last contents
             load_next(wr);
             if constexpr (EXACT) {
-                out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx);
+                out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx, (int)(l_end - l_begin) - kt * BK);
                 if constexpr (FOLD)
                     if (kt % kFoldStages == kFoldStages - 1) out.fold();
             } else {
-                if (gr.nf > 6) out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx);
-                else if (gr.nf > 4) out.template stage<6>(sm.a[rd], sm.b[rd], ty, tx);
-                else out.template stage<4>(sm.a[rd], sm.b[rd], ty, tx);
+                if (gr.nf > 6) out.template stage<TN>(sm.a[rd], sm.b[rd], ty, tx, (int)(l_end - l_begin) - kt * BK);
+                else if (gr.nf > 4) out.template stage<6>(sm.a[rd], sm.b[rd], ty, tx, (int)(l_end - l_begin) - kt * BK);
+                else out.template stage<4>(sm.a[rd], sm.b[rd], ty, tx, (int)(l_end - l_begin) - kt * BK);
             }
             rd = rd + 1 == ST ? 0 : rd + 1;
             wr = wr + 1 == ST ? 0 : wr + 1;

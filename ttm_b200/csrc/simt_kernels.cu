@@ -98,14 +98,14 @@ constexpr int ffma_blocks(int TX, int TM, int TN, bool AK)
 constexpr size_t kSmSharedBytes = 228 * 1024;
 constexpr bool blocks_fit(int blocks, size_t smem) { return blocks * (smem + 1024) <= kSmSharedBytes; }
 
-template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM>
+template <int TX, int TM, int TN, int ST, bool AK, bool VEC, bool BCM, bool HALF>
 __global__ void __launch_bounds__(32 * TX, ffma_blocks(TX, TM, TN, AK)) ffma_gemm_kernel(View3 v, ColumnGrid gr, int64_t tiles,
                                                                                int64_t lper, float* ws)
 {
     extern __shared__ __align__(16) unsigned char gemm_smem[];
     int64_t l0, l1;
     split_range(v, lper, ws, l0, l1);
-    f32::tiles<TX, TM, TN, ST, AK, VEC, BCM, true>(v, blockIdx.x, gridDim.x, tiles, gr,
+    f32::tiles<TX, TM, TN, ST, AK, VEC, BCM, true, HALF>(v, blockIdx.x, gridDim.x, tiles, gr,
                                                    *reinterpret_cast<f32::Smem<TX, TM, TN, ST, AK>*>(gemm_smem), l0, l1);
 }
 
@@ -927,12 +927,17 @@ cudaError_t ffma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, in
 {
     constexpr int smem = (int)sizeof(f32::Smem<TX, TM, TN, ST, AK>);
     static_assert(blocks_fit(ffma_blocks(TX, TM, TN, AK), smem), "the walking form's blocks are resident at once");
-    const auto kernel = ffma_gemm_kernel<TX, TM, TN, ST, AK, VEC, BCM>;
+    // wide tiles of contiguous fibres, short ranges: half stages (128000 fibres, m = 512: n_q = 20 125 ->
+    // 99 us, n_q = 8 85 -> 69)
+    auto kernel = ffma_gemm_kernel<TX, TM, TN, ST, AK, VEC, BCM, false>;
+    if constexpr (AK && TX == 8)
+        if (v.nq <= 4 * f32::BK) kernel = ffma_gemm_kernel<TX, TM, TN, ST, AK, VEC, BCM, true>;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int64_t tiles = ceil_div(v.outer * v.inner, 32 * TM) * gr.cols;
-    // as in dmma_launch (m = 64, n_q = 16, A 64 MB: 86 -> 82 us; n_q = 64: 190 us against 197)
-    const bool walk = v.nq <= 2 * f32::BK;
+    // as in dmma_launch (m = 64, n_q = 16, A 64 MB: 86 -> 82 us; n_q = 64: 190 us against 197); several
+    // column tiles are balanced better one by one (128000 fibres of 20, m = 99: 35 us against 45)
+    const bool walk = gr.cols == 1 && v.nq <= 2 * f32::BK;
     const int64_t slots = (int64_t)sms * ffma_blocks(TX, TM, TN, AK);
     const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
     kernel<<<grid, 32 * TX, smem, s>>>(v, gr, tiles, lper, ws);
@@ -1033,7 +1038,9 @@ cudaError_t dmma_launch(const View3& v, cudaStream_t s, const ColumnGrid& gr, in
     // Short l ranges: a fixed set of blocks walks the tiles, so that the ring stays full across
     // them (n_q = 16, A 256 MB: m = 64 147 -> 114 us, m = 8 94 -> 67 us). Longer ones: a block per
     // tile, which the scheduler balances better (m = 64, n_q = 48: 97 us against 113).
-    const bool walk = v.nq <= (NF <= 2 ? 8 : 2) * f64::BK;
+    // So are several column tiles of fibres whose outputs leave one by one (128000 fibres of 8, m = 355 161
+    // us against 205; m = 130, in pairs, 45 against 36).
+    const bool walk = v.nq <= (NF <= 2 ? 8 : 2) * f64::BK && (gr.cols == 1 || !AK || v.m % 2 == 0);
     const int64_t slots = (int64_t)sms * dmma_blocks(BM, AK, FOLD);
     const dim3 grid((unsigned)(walk ? std::min(tiles, slots) : tiles), 1, (unsigned)split);
     kernel<<<grid, 2 * BM, smem, s>>>(v, gr, tiles, lper, ws);

@@ -239,10 +239,12 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
 #pragma unroll
             for (int e = 0; e < 2; ++e) mid[r][f][e] = sum[r][f][e] = err[r][f][e] = 0.0;
 
+    const bool mine = m0 + warp * 16 < M;   // a warp past the last row only copies
     for (int kt = 0; kt < nk; ++kt) {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
         __syncthreads();   // stage rd has landed for all, and all have read stage wr's last contents
         load_next(wr);
+        if (mine) {
         if constexpr (EXACT) {
             if constexpr (FOLD != 0) {
                 if (kt > 0) close_chains();
@@ -261,6 +263,7 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
             case 7: stage<7, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
             default: stage<NF, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
             }
+        }
         }
         rd = rd + 1 == ST ? 0 : rd + 1;
         wr = wr + 1 == ST ? 0 : wr + 1;

@@ -815,8 +815,8 @@ constexpr size_t grouped_smem_bytes()
         else     { if (g.b_cm) TLIBTTM_TILE(false, false, true); else TLIBTTM_TILE(false, false, false); } \
     }
 
-// Two CTAs per SM (at most 128 registers; a few spill): measured faster on the batched workload
-// than one CTA of 255 registers.
+// Two CTAs per SM (at most 128 registers; the FP64 build spills some 300 bytes a thread): measured faster
+// on the batched workload than one CTA of 255 registers.
 template <typename T>
 __global__ void __launch_bounds__(256, 2) grouped_kernel(const GroupDesc* __restrict__ desc, int count, int64_t total,
                                                       unsigned long long* queue)
@@ -1652,8 +1652,8 @@ size_t simt_gemm_split_bytes(const View3& v, int dtype)
 //             1.3 at 512 rows)
 //   column kernel: double m 5..8 3.4-6, float m 9..16 2.1-5.4; m below that, to 8192 rows 1.7-4
 // Float keeps to ranges whose parts are at most kSplitChainF32 l long, and splits whatever the block
-// count in place of the l-split kernels: a chain of 1024 FMAs is 5.7e-7 off (relative, N(0,1)
-// entries), the chains of the kernels it replaces 1e-7 to 6e-7.
+// count in place of the l-split kernels. (The parts' sums are folded: no further off than those kernels',
+// gemm_f32.cuh.)
 // Shorter ranges of few tiles keep to the TMA-fed kernel (m 9..16: 0.5-0.8 at 64 blocks, 1.1 at 128; m
 // 5..8 0.9 at 128, 1.1 at 256), or to the l-split kernels and the column kernel's l split (0.8-0.9
 // below about 16 tiles of 128 rows).

@@ -17,14 +17,15 @@
 //       FP64 arithmetic on the GPU is limited to the exponent extraction, the digit
 //       extraction and this recombination.
 //
-// Both run in three steps per chunk of rows of the slice GEMM: an exponent kernel, a slicer
-// that writes the 8-bit operand image in the K-major 32-byte-swizzled layout the MMA reads
-// (128 rows x 32 l per 4 KB block, S blocks per (row tile, l chunk)), and the MMA kernel.
+// Both make the exponents and the 8-bit operand image, in the K-major 32-byte-swizzled layout
+// the MMA reads (128 rows x 32 l per 4 KB block, S blocks per (row tile, l chunk)), per chunk
+// of rows of the slice GEMM and then run the MMA kernel on it: fp8 with an exponent kernel and
+// a slicer, ozaki with one kernel for both (its B, and all of fp8's operands, with two).
 // Rows enumerate (k, i) with i fastest, R = k * inner + i, so one code path serves every
 // layout; B's rows are j. The operand images are scratch from the stream-ordered pool, at
 // most about 1 GB per chunk of rows.
 //
-// MMA kernel warp roles (320 threads, one CTA per SM, persistent over tiles):
+// MMA kernel warp roles (576 threads, one CTA per SM, persistent over tiles):
 //   warp 0     bulk-copy producer: the A and B image blocks of one l chunk per stage
 //   warp 1     TMEM allocator and MMA issuer (the whole warp, one elected lane per MMA)
 //   warps 2-17 epilogue: TMEM -> registers -> scaled C, direct stores; four warps per TMEM lane

@@ -17,7 +17,7 @@
 //
 // Warp roles (736 threads, one CTA per SM, persistent over tiles):
 //   warp 0     TMA producer of the FP32 A tile (tensor map).
-//   warp 1     TMEM allocator and MMA issuer (one elected lane).
+//   warp 1     TMEM allocator and MMA issuer (the whole warp, one elected lane per MMA).
 //   warp 2     bulk copies of the pre-split B_hi/B_lo image of this stage.
 //   warps 3-18 converters: FP32 tile -> bf16 hi/lo in the swizzled UMMA layout.
 //   warps 19-22 epilogue: TMEM -> registers -> global C (double-buffered accumulator).

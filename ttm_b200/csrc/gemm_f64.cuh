@@ -9,7 +9,7 @@
 // DFMA) once m passes about 24; below that, reading A. A k-step of four l costs a warp 1 or 2 A and
 // NF B shared loads for 2 NF mma of 256 multiply-adds each; the DFMA tile of 64 x 64 it replaced
 // needed 8 loads for 16 DFMA of 32. Measured, before -> now: A 256^3, m = 128, middle mode
-// 323 -> 144 us (30 TFLOP/s); (150, 171, 333), m = 100 189 -> 84 us; (200, 180, 160), m = 20
+// 323 -> 139 us (31 TFLOP/s); (150, 171, 333), m = 100 189 -> 82 us; (200, 180, 160), m = 20
 // 84 -> 19 us; contiguous fibres of 384, 78000 rows, m = 16 (TMA row kernel) 139 -> 50 us. (Running
 // pointers in place of addresses recomputed per copy gave 5-15 % of that.)
 // Rows of 64 for at most 16 columns with 16-byte copies (five blocks of 128 threads per SM, four for
@@ -239,12 +239,24 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
 #pragma unroll
             for (int e = 0; e < 2; ++e) mid[r][f][e] = sum[r][f][e] = err[r][f][e] = 0.0;
 
-    const bool mine = m0 + warp * 16 < M;   // a warp past the last row only copies
-    for (int kt = 0; kt < nk; ++kt) {
+    // stage rd has landed for all, and all have read stage wr's last contents (a warp at a time reaches
+    // this barrier from one of the two loops below)
+    auto turn = [&]() {
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-        __syncthreads();   // stage rd has landed for all, and all have read stage wr's last contents
+        asm volatile("bar.sync 0;" ::: "memory");
         load_next(wr);
-        if (mine) {
+    };
+    auto advance = [&]() {
+        rd = rd + 1 == ST ? 0 : rd + 1;
+        wr = wr + 1 == ST ? 0 : wr + 1;
+    };
+    const int mine = m0 + warp * 16 < M ? nk : 0;   // a warp past the last row only copies
+    for (int kt = mine; kt < nk; ++kt) {
+        turn();
+        advance();
+    }
+    for (int kt = 0; kt < mine; ++kt) {
+        turn();
         if constexpr (EXACT) {
             if constexpr (FOLD != 0) {
                 if (kt > 0) close_chains();
@@ -264,9 +276,7 @@ __device__ __forceinline__ void tiles(const View3& v, int64_t first, int64_t ste
             default: stage<NF, AK, BCM, 0>(sm.a[rd], sm.b[rd], warp, g, c, acc); break;
             }
         }
-        }
-        rd = rd + 1 == ST ? 0 : rd + 1;
-        wr = wr + 1 == ST ? 0 : wr + 1;
+        advance();
     }
 
     if constexpr (FOLD != 0) {
